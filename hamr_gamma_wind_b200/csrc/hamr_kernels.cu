@@ -1025,7 +1025,8 @@ __global__ void k_face_update_polar(const Dims d, const Geom m, const double *ps
     face_update_eval(d, m, psi, psf, E, st.sub(), i, j, z, c, gix(d, i, j), 7);
 }
 
-// geometric source gdet T^k_l Gamma^l_{jk} (source, GPU_phys_mhd.h:34-175)
+// geometric source gdet T^k_l Gamma^l_{jk} (source, GPU_phys_mhd.h:34-175),
+// components UU .. U3 (the others are zero and not written)
 // conn(s, k): the connection coefficient of symmetric pair s and index k at
 // the zone's (i, j) column (from the tables, or staged in shared memory)
 template <class Conn>
@@ -1043,8 +1044,7 @@ __device__ __forceinline__ void source_c(double gam, const double *ph, const Geo
 #pragma unroll
         for (int b = 0; b < 4; b++)
             mhd[a][b] = eta * q.ucon[a] * q.ucov[b] + ptot * (a == b ? 1. : 0.) - q.bcon[a] * q.bcov[b];
-#pragma unroll
-    for (int k = 0; k < NPR; k++) dU[k] = 0.;
+    dU[UU] = dU[U1] = dU[U2] = dU[U3] = 0.;
 #define CONN(s, k) conn((s), (k))
 #pragma unroll
     for (int k = 0; k < 4; k++) {
@@ -1065,7 +1065,6 @@ __device__ __forceinline__ void source_c(double gam, const double *ph, const Geo
     dU[U1] *= gm.g;
     dU[U2] *= gm.g;
     dU[U3] *= gm.g;
-    dU[KTOT] *= gm.g;
 }
 
 // connection accessors: from the tables (one (i, j) column: base pointer and
@@ -1099,8 +1098,7 @@ __device__ __forceinline__ void source(double gam, const double *ph, const Geo<d
 #pragma unroll
         for (int b = 0; b < 4; b++)
             mhd[a][b] = eta * q.ucon[a] * q.ucov[b] + ptot * (a == b ? 1. : 0.) - q.bcon[a] * q.bcov[b];
-#pragma unroll
-    for (int k = 0; k < NPR; k++) dU[k] = 0.;
+    dU[UU] = dU[U1] = dU[U2] = dU[U3] = 0.;
 #define CONN(s, k) __ldg(&m.conn[(long)((s) * 4 + (k)) * gs + gi])
 #pragma unroll
     for (int k = 0; k < 4; k++) {
@@ -1121,8 +1119,15 @@ __device__ __forceinline__ void source(double gam, const double *ph, const Geo<d
     dU[U1] *= gm.g;
     dU[U2] *= gm.g;
     dU[U3] *= gm.g;
-    dU[KTOT] *= gm.g;
 }
+
+// The components of U that the conserved update advances: the magnetic ones
+// are left out wherever U[B] is set from the updated faces before anything
+// reads it (face_average_b: B1 and B2 always, B3 on 3-D blocks), so their
+// flux divergences, their planes of the U(p^n) cache and their staged fluxes
+// need not exist. U[B] returned by the update is zero there.
+constexpr int N_ADV = 6;   // RHO, UU, U1, U2, U3, KTOT (and B3 on 2-D blocks)
+__host__ __device__ constexpr int adv_comp(int q) { return q < 5 ? q : KTOT; }
 
 // Conserved update of one active zone (fixup, GPU_fixup.h:5-424, up to the
 // inversion): U(p^n) computed and cached by the half sub-step or read back by
@@ -1139,6 +1144,8 @@ __device__ __forceinline__ void cons_update_fx(const Dims &d, const Geom &m, con
     const long ks = d.ks;
     State<double> q;
     double dU[NPR];
+    const bool two_d = d.ng3 == 0;
+    auto advanced = [&](int k) { return k < B1 || k == KTOT || (k == B3 && two_d); };
     if (!full) {
 #pragma unroll
         for (int k = 0; k < NPR; k++) { pf[k] = 0.0; pf[k] += (1.0 / ((double)1)) * pin[k * ks + c]; }
@@ -1146,17 +1153,22 @@ __device__ __forceinline__ void cons_update_fx(const Dims &d, const Geom &m, con
         double vd;
         primtoflux(d.gam, pf, q, 0, gm, entropy(d.gam, pf), U, &vd, &vd);
 #pragma unroll
-        for (int k = 0; k < NPR; k++) Ucache[k * ks + c] = U[k];
+        for (int k = 0; k < NPR; k++)
+            if (advanced(k)) Ucache[k * ks + c] = U[k];
     } else {
 #pragma unroll
-        for (int k = 0; k < NPR; k++) U[k] = Ucache[k * ks + c];
+        for (int k = 0; k < NPR; k++)
+            if (advanced(k)) U[k] = Ucache[k * ks + c];
 #pragma unroll
         for (int k = 0; k < NPR; k++) { pf[k] = 0.0; pf[k] += (1.0 / ((double)1)) * pb[k * ks + c]; }
         get_state(pf, gm, q);
     }
+    U[B1] = U[B2] = 0.0;
+    if (!two_d) U[B3] = 0.0;
     if constexpr (sizeof(T) == sizeof(double)) {
 #pragma unroll
         for (int k = 0; k < NPR; k++) {
+            if (!advanced(k)) continue;
             if (d.ng1 > 0) U[k] -= div_rcp(Dt * (FX_(1, k, 1) - FX_(1, k, 0)), d.dx1, d.rdx1);
             if (d.ng2 > 0) U[k] -= div_rcp(Dt * (FX_(2, k, 1) - FX_(2, k, 0)), d.dx2, d.rdx2);
             if (d.ng3 > 0) U[k] -= div_rcp(Dt * (FX_(3, k, 1) - FX_(3, k, 0)), d.dx3, d.rdx3);
@@ -1164,7 +1176,7 @@ __device__ __forceinline__ void cons_update_fx(const Dims &d, const Geom &m, con
         if constexpr (std::is_same<Conn, ConnTable>::value) source(d.gam, pf, gm, d, m, gi, dU, q);
         else source_c(d.gam, pf, gm, conn, dU, q);
 #pragma unroll
-        for (int k = 0; k < NPR; k++) U[k] += Dt * (dU[k]);
+        for (int k = UU; k <= U3; k++) U[k] += Dt * (dU[k]);   // the source has no other component
     } else {
         // float fluxes: differences taken in double (exact for two floats of
         // similar size) and the four increments added to U^n with Neumaier
@@ -1173,6 +1185,7 @@ __device__ __forceinline__ void cons_update_fx(const Dims &d, const Geom &m, con
         else source_c(d.gam, pf, gm, conn, dU, q);
 #pragma unroll
         for (int k = 0; k < NPR; k++) {
+            if (!advanced(k)) continue;
             double sum = U[k], comp = 0.;
             auto add = [&](double x) {
                 const double tt = sum + x;
@@ -1182,7 +1195,7 @@ __device__ __forceinline__ void cons_update_fx(const Dims &d, const Geom &m, con
             if (d.ng1 > 0) add(div_rcp(-Dt * ((double)FX_(1, k, 1) - (double)FX_(1, k, 0)), d.dx1, d.rdx1));
             if (d.ng2 > 0) add(div_rcp(-Dt * ((double)FX_(2, k, 1) - (double)FX_(2, k, 0)), d.dx2, d.rdx2));
             if (d.ng3 > 0) add(div_rcp(-Dt * ((double)FX_(3, k, 1) - (double)FX_(3, k, 0)), d.dx3, d.rdx3));
-            add(Dt * dU[k]);
+            if (k >= UU && k <= U3) add(Dt * dU[k]);
             U[k] = sum + comp;
         }
     }
@@ -1366,7 +1379,7 @@ __device__ __forceinline__ void k_cons_at(const Dims &d, const Geom &m, const do
     W[3 * d.ks + c] = U[U2];
     W[4 * d.ks + c] = U[U3];
     W[5 * d.ks + c] = U[KTOT];
-    W[6 * d.ks + c] = U[B3];   // kept in 2-D, where the faces do not set it
+    if (d.ng3 == 0) W[6 * d.ks + c] = U[B3];   // in 3-D the faces set it
 }
 
 template <typename T>
@@ -1432,7 +1445,7 @@ __global__ void __launch_bounds__(BLK, HAMR_CONS_MINB) k_cons_cols(const Dims d,
     W[3 * d.ks + c] = U[U2];
     W[4 * d.ks + c] = U[U3];
     W[5 * d.ks + c] = U[KTOT];
-    W[6 * d.ks + c] = U[B3];
+    if (d.ng3 == 0) W[6 * d.ks + c] = U[B3];
 }
 
 // the inversion's inputs of one zone: the stage's primitives as the initial
@@ -1448,16 +1461,16 @@ __device__ __forceinline__ void invert_inputs(const Dims &d, const Geom &m, cons
     U[U2] = W[3 * d.ks + c];
     U[U3] = W[4 * d.ks + c];
     U[KTOT] = W[5 * d.ks + c];
-    U[B3] = W[6 * d.ks + c];
+    if (d.ng3 == 0) U[B3] = W[6 * d.ks + c];
     face_average_b(d, m, psf, i, j, c, gi, U);
 }
 
 // ------------------------------------------- TMA-staged conserved update
 // The conserved update of one (i, j) row of zones (or an equal piece of it)
-// per CTA, with the 45 flux operands of every zone -- the x1 fluxes on both
-// faces, the x2 fluxes on both faces, the x3 fluxes of the row and one more
+// per CTA, with the 30 flux operands of every zone -- six components' x1 fluxes
+// on both faces, x2 fluxes on both faces, x3 fluxes of the row and one more
 // -- brought into shared memory by bulk asynchronous copies (TMA,
-// cp.async.bulk) before any arithmetic: 45 copies per row, completion
+// cp.async.bulk) before any arithmetic: 30 copies per row, completion
 // counted on one mbarrier, all in flight at once, where a thread of the
 // one-zone-per-thread kernel can only keep as many loads in flight as its
 // registers hold. A bulk copy must start and end on 16-byte boundaries: each
@@ -1516,7 +1529,7 @@ __host__ __device__ __forceinline__ ConsTmaLayout cons_tma_layout(int lpiece) {
     L.cap = ((lpiece + 1 + 2 * (A - 1)) + A - 1) / A * A;
     L.seg_bytes = L.cap * (int)sizeof(T);
     L.f_off = 16 + ((COL_VALS * 8 + 15) / 16) * 16;
-    L.total = L.f_off + 5 * NPR * L.seg_bytes;
+    L.total = L.f_off + 5 * N_ADV * L.seg_bytes;
     return L;
 }
 
@@ -1580,12 +1593,13 @@ __device__ __forceinline__ void cons_tma_row(const Dims &d, const Geom &m, const
         for (int q = 0; q < 5; q++) {
             const long s0 = seg_start(q), sa = s0 & ~(long)(A - 1);
             const long se = (s0 + seg_len(q) + A - 1) & ~(long)(A - 1);
-            total += (unsigned)((se - sa) * (long)sizeof(T)) * NPR;
+            total += (unsigned)((se - sa) * (long)sizeof(T)) * N_ADV;
         }
         if (threadIdx.x == 0) mbar_expect_tx(bar_a, total);
         __syncwarp();
-        for (int e = threadIdx.x; e < 5 * NPR; e += 32) {
-            const int q = e / NPR, k = e % NPR;
+        if (threadIdx.x < 5 * N_ADV) {
+            const int e = threadIdx.x;
+            const int q = e / N_ADV, k = adv_comp(e % N_ADV);
             const long s0 = seg_start(q), sa = s0 & ~(long)(A - 1);
             const long se = (s0 + seg_len(q) + A - 1) & ~(long)(A - 1);
             bulk_g2s(smem_addr(sf + (long)e * lay.cap), seg_src(q) + (long)k * ks + sa,
@@ -1618,7 +1632,7 @@ __device__ __forceinline__ void cons_tma_row(const Dims &d, const Geom &m, const
     }
     auto fx = [&](int dir, int k, int up) -> T {
         const int q = dir == 1 ? up : (dir == 2 ? 2 + up : 4);
-        return sf[(long)(q * NPR + k) * lay.cap + off[q] + (dir == 3 ? up : 0)];
+        return sf[(q * N_ADV + (k < B1 ? k : 5)) * lay.cap + off[q] + (dir == 3 ? up : 0)];
     };
     Geo<double> gm;
 #pragma unroll
@@ -1627,20 +1641,15 @@ __device__ __forceinline__ void cons_tma_row(const Dims &d, const Geom &m, const
     geo_lapse(gm);
     double pf[NPR], U[NPR];
     cons_update_fx<T>(d, m, pin, pb, Ucache, fx, full, st.sub(), i, j, c, gi, gm, ConnStaged{sg + 21}, pf, U);
-    auto write_w = [&]() {
-        W[0 * d.ks + c] = U[RHO];
-        W[1 * d.ks + c] = U[UU];
-        W[2 * d.ks + c] = U[U1];
-        W[3 * d.ks + c] = U[U2];
-        W[4 * d.ks + c] = U[U3];
-        W[5 * d.ks + c] = U[KTOT];
-        W[6 * d.ks + c] = U[B3];
+    auto write_w = [&](const double *w) {   // 3-D: the faces set U[B]
+#pragma unroll
+        for (int q = 0; q < N_ADV; q++) W[q * ks + c] = w[q];
     };
+    const double Uw[N_ADV] = {U[RHO], U[UU], U[U1], U[U2], U[U3], U[KTOT]};
     if constexpr (FUSE == 0) {
-        write_w();
+        write_w(Uw);
     } else {
         constexpr int INV = FUSE - 1;
-        const double Uw[7] = {U[RHO], U[UU], U[U1], U[U2], U[U3], U[KTOT], U[B3]};
         // the inversion's inputs as k_invert_primary reads them: the guess
         // straight from pb, U[B] from the updated faces
 #pragma unroll
@@ -1648,9 +1657,7 @@ __device__ __forceinline__ void cons_tma_row(const Dims &d, const Geom &m, const
         face_average_b(d, m, psf, i, j, c, gi, U);
         const int flag = invert_primary<INV>(d, inv_k(d, m, gi, gm), gm, U, pf);
         if (flag) {
-            U[RHO] = Uw[0]; U[UU] = Uw[1]; U[U1] = Uw[2]; U[U2] = Uw[3]; U[U3] = Uw[4]; U[KTOT] = Uw[5];
-            U[B3] = Uw[6];
-            write_w();
+            write_w(Uw);
             const long t = ((long)(i - d.ng1) * d.n2 + (j - d.ng2)) * d.n3 + (za - d.ng3 + l);
             flist[atomicAdd(nfail, 1)] = (int)t;
             return;
