@@ -184,6 +184,7 @@ __device__ __forceinline__ double flux_face(const Dims &d, const Geom &m, const 
     T pl[NPR], pr[NPR];
 #pragma unroll
     for (int k = 0; k < NPR; k++) {
+        if (k == B1 + DIR - 1) continue;   // the normal field comes from the face
         const double *pk = pv + (long)k * d.ks + c;
         if constexpr ((REC & 1) == HAMR_RECON_MC) {
             // linear MC: the zones' face values y -+ slope/2 (fluxcalcprep, PPM = 0)
@@ -198,11 +199,7 @@ __device__ __forceinline__ double flux_face(const Dims &d, const Geom &m, const 
             T x[6];
 #pragma unroll
             for (int s = 0; s < 6; s++) x[s] = (T)__ldg(pk + (s - 3) * stride);
-            T lo, hi;
-            para(x, lo, hi);       // zone c-1: upper edge is the left state
-            pl[k] = hi;
-            para(x + 1, lo, hi);   // zone c: lower edge is the right state
-            pr[k] = lo;
+            para_face(x, pl[k], pr[k]);   // upper edge of zone c-1, lower edge of zone c
         }
     }
     return flux_eval<DIR, T, REC>(d, gm, ps, pl, pr, F, c, j);
@@ -210,7 +207,8 @@ __device__ __forceinline__ double flux_face(const Dims &d, const Geom &m, const 
 
 // The face flux from the reconstructed states pl, pr (the normal field and
 // the polar B1 fix applied here): two states, four flux evaluations, HLL (or
-// HLLC), the flux written at cell index c; returns the face's signal-speed
+// HLLC), the flux written at cell index c, all but the normal field's, which
+// is zero and which nothing reads; returns the face's signal-speed
 // contribution to the CFL limit (ctop_term).
 template <int DIR, typename T, int REC>
 __device__ __forceinline__ double flux_eval(const Dims &d, const Geo<T> &gm, const double *__restrict__ ps, T *pl,
@@ -230,7 +228,8 @@ __device__ __forceinline__ double flux_eval(const Dims &d, const Geo<T> &gm, con
         T Fo[NPR];
         const T ctop = hllc_face<DIR, T, (REC & 4) != 0>(gam, pl, pr, gm, Fo);
 #pragma unroll
-        for (int k = 0; k < NPR; k++) F[(long)k * d.ks + c] = Fo[k];
+        for (int k = 0; k < NPR; k++)
+            if (k != B1 + DIR - 1) F[(long)k * d.ks + c] = Fo[k];
         (void)dxd;
         (void)dtf;
         return ctop_term(d, DIR, (double)ctop);
@@ -252,7 +251,8 @@ __device__ __forceinline__ double flux_eval(const Dims &d, const Geo<T> &gm, con
     const Divisor<T> dh(cmax + cmin + T(SMALL_D));   // the nine HLL quotients share it
 #pragma unroll
     for (int k = 0; k < NPR; k++)
-        F[(long)k * d.ks + c] = dh.div(cmax * t1[k] + cmin * t3[k] - cmax * cmin * (t4[k] - t2[k]));
+        if (k != B1 + DIR - 1)
+            F[(long)k * d.ks + c] = dh.div(cmax * t1[k] + cmin * t3[k] - cmax * cmin * (t4[k] - t2[k]));
     (void)dxd;
     (void)dtf;
     return ctop_term(d, DIR, (double)ctop);
@@ -332,25 +332,36 @@ __device__ __forceinline__ void zone_edges(const Dims &d, const double *__restri
 }
 
 // x3 faces (phi, the contiguous direction) with each zone reconstructed once.
-// The zones a row of x3 faces touches, z = ng3 - 1 .. ng3 + n3 (n3 + 2 of
-// them for n3 + 1 faces), are numbered row after row as "slots"; CTA b takes
-// slots b (BLK - 1) .. b (BLK - 1) + BLK - 1, one per thread, so consecutive
-// CTAs share one slot. Phase 1: every thread reconstructs its slot's zone and
-// leaves both edges in shared memory. Phase 2: thread l evaluates the face
-// between slots l and l + 1 when both lie in the same row (left state: the
-// upper edge of slot l, right state: the lower edge of slot l + 1). Every
-// thread does the same work in each phase, so the barrier between them costs
-// little. Same values as k_flux<3> face by face: the same para on the same
-// five zones.
+// A row's zones z = ng3 - 1 .. ng3 + n3, those its x3 faces touch (n3 + 2 of
+// them for n3 + 1 faces), and for PPM one more either side, whose limited
+// slopes the outer zones need, are numbered row after row as "slots"; a CTA
+// takes BLK consecutive slots, one per thread, and the CTAs overlap by the
+// slots whose neighbours they lack. PPM, in three phases with a barrier after
+// each: every slot's limited slope; the interpolated value between slots l and
+// l + 1, from both slots' values and slopes; the monotonised edges of slot l
+// from the values on its two faces, the lower edge into shared memory. So each
+// slope and each face value is evaluated once per zone, where the five-zone
+// stencil by itself takes three and two, and a thread loads three zones
+// instead of five (per step of the 384 x 192 x 192 torus, centre EMFs included:
+// FP64 5.60 -> 4.17 ms, mixed 2.34 -> 1.99). MC: the edges straight from the slot's slope, in one phase.
+// Last, thread l evaluates the face between slots l and l + 1 (left state: its
+// own upper edge, right state: the lower edge of slot l + 1). Same values as
+// k_flux<3> face by face.
+template <int REC>
+struct X3Slots {
+    static constexpr int H = (REC & 1) == HAMR_RECON_MC ? 0 : 1;   // extra slots at either end of a row
+    static constexpr int STEP = BLK - 1 - 2 * H;                   // faces per CTA: threads H .. H + STEP - 1
+};
+__host__ __device__ __forceinline__ int x3_halo(const Dims &d) { return d.recon == HAMR_RECON_MC ? 0 : 1; }
 __host__ __device__ __forceinline__ long n_x3_slots(const Dims &d) {
-    return (long)(d.n1 + 2 * d.d1) * (d.n2 + 2 * d.d2) * (d.n3 + 2 * d.d3);
+    return (long)(d.n1 + 2 * d.d1) * (d.n2 + 2 * d.d2) * (d.n3 + 2 * d.d3 + 2 * x3_halo(d));
 }
 
 // build options: resident blocks per SM for the double and float x3 slot
-// kernels. Measured per 384 x 192 x 192 step: float 10 blocks (48 registers)
-// 2.04 ms, 12: 2.09, 8: 2.14, 6 (80 registers, no spills): 2.54; double (with
-// the shared-divisor quotients and the centre EMFs) 5 blocks 5.48 ms, 4:
-// 5.52, 6: 5.62.
+// kernels. Measured per 384 x 192 x 192 step, before the slopes and face
+// values were shared: float 10 blocks (48 registers) 2.04 ms, 12: 2.09, 8:
+// 2.14, 6 (80 registers, no spills): 2.54; double 5 blocks 5.48 ms, 4: 5.52,
+// 6: 5.62.
 // The face-frame solvers (HLLC, HLLD) in the x3 slot kernel, which hold both
 // frame states, their fluxes and (HLLD) the wave fan in thread-local arrays:
 // on the 384 x 192 x 192 torus, FP64, per step, 4 blocks per SM (128
@@ -383,55 +394,84 @@ template <typename T, int REC>
 __device__ __forceinline__ double flux_x3_slots(const Dims &d, const Geom &m, const double *__restrict__ pv,
                                                 const double *__restrict__ ps, T *__restrict__ F,
                                                 T *__restrict__ Ec, long blk) {
-    __shared__ T slo[NPR - 1][BLK], shi[NPR - 1][BLK];   // zone edges per slot (B3 skipped)
+    constexpr int H = X3Slots<REC>::H, STEP = X3Slots<REC>::STEP;
+    constexpr int NK = NPR - 1;            // B3 is not reconstructed
+    __shared__ T sa[NK][BLK], sb[NK][BLK]; // PPM: slopes, then lower edges | face values; MC: lower edges
     const int l = threadIdx.x;
     const long nslot = n_x3_slots(d);
-    const int rz = d.n3 + 2 * d.d3;   // slots per row
+    const int rz = d.n3 + 2 * d.d3 + 2 * H;   // slots per row
     const int nj = d.n2 + 2 * d.d2;
-    const long sl = blk * (BLK - 1) + l;
+    const long sl = blk * STEP + l;
     const int zl = (int)(sl % rz);
     const long row = sl / rz;
     const int j = (d.ng2 - 1) * d.d2 + (int)(row % nj);
     const int i = (d.ng1 - 1) * d.d1 + (int)(row / nj);
-    const long c = cix(d, i, j, d.ng3 - 1 + zl);   // the slot's zone
-    if (sl < nslot) {
-        T lo[NPR], hi[NPR];
-        zone_edges<3, T, REC>(d, pv, c, 1, lo, hi);
+    const long c = cix(d, i, j, d.ng3 - 1 - H + zl);   // the slot's zone
+    T hi[NPR];
+    if constexpr (H == 0) {
+        if (sl < nslot) {
+            T lo[NPR];
+            zone_edges<3, T, REC>(d, pv, c, 1, lo, hi);
 #pragma unroll
-        for (int k = 0, q = 0; k < NPR; k++)
-            if (k != B3) {
-                slo[q][l] = lo[k];
-                shi[q++][l] = hi[k];
-            }
-        if (Ec && (l < BLK - 1 || sl == nslot - 1)) {
-            T e[3];
-            emf_centre_eval(d, m, pv, i, j, c, e);
-            Ec[1 * d.ks + c] = e[0];
-            Ec[2 * d.ks + c] = e[1];
-            Ec[3 * d.ks + c] = e[2];
+            for (int k = 0, q = 0; k < NPR; k++)
+                if (k != B3) sa[q++][l] = lo[k];
         }
+    } else {
+        T y0[NK], y1[NK];
+        if (sl < nslot) {
+#pragma unroll
+            for (int k = 0, q = 0; k < NPR; k++) {
+                if (k == B3) continue;
+                const double *pk = pv + (long)k * d.ks + c;
+                const T ym = (T)__ldg(pk - 1);
+                y0[q] = (T)__ldg(pk);
+                y1[q] = (T)__ldg(pk + 1);
+                sa[q][l] = ppm_slope(ym, y0[q], y1[q]);
+                q++;
+            }
+        }
+        __syncthreads();
+        if (l < BLK - 1 && sl + 1 < nslot)
+#pragma unroll
+            for (int q = 0; q < NK; q++) sb[q][l] = ppm_face(y0[q], y1[q], sa[q][l], sa[q][l + 1]);
+        __syncthreads();
+        if (l > 0 && l < BLK - 1 && sl + 1 < nslot)
+#pragma unroll
+            for (int k = 0, q = 0; k < NPR; k++) {
+                if (k == B3) continue;
+                T lo;
+                ppm_limit(y0[q], sb[q][l - 1], sb[q][l], lo, hi[k]);
+                sa[q++][l] = lo;
+            }
+    }
+    // the CTA's own slots: the last CTA also takes the last zone's
+    const bool mine = l >= H && (l < H + STEP || sl + 1 + H == nslot);
+    if (Ec && mine && zl >= H && zl < rz - H && sl < nslot) {
+        T e[3];
+        emf_centre_eval(d, m, pv, i, j, c, e);
+        Ec[1 * d.ks + c] = e[0];
+        Ec[2 * d.ks + c] = e[1];
+        Ec[3 * d.ks + c] = e[2];
     }
     __syncthreads();
     double cmx = 0.0;
     // the face above this slot's zone: zone c + 1 is the next slot of the row
-    if (l < BLK - 1 && sl + 1 < nslot && zl + 1 < rz) {
-        T pl[NPR], pr[NPR];
+    if (l >= H && l < H + STEP && sl + 1 + H < nslot && zl >= H && zl + 1 + H < rz) {
+        T pr[NPR];
 #pragma unroll
         for (int k = 0, q = 0; k < NPR; k++)
-            if (k != B3) {
-                pl[k] = shi[q][l];
-                pr[k] = slo[q++][l + 1];
-            }
+            if (k != B3) pr[k] = sa[q++][l + 1];
         Geo<T> gm;
         load_geo_t(d, m, i, j, FACE3, gm);
-        cmx = flux_eval<3, T, REC>(d, gm, ps, pl, pr, F, c + 1, j);
+        cmx = flux_eval<3, T, REC>(d, gm, ps, hi, pr, F, c + 1, j);
     }
     return cmx;
 }
 
-// CTAs of the slot range: CTA b takes slots b (BLK - 1) .. b (BLK - 1) + BLK - 1
+// CTAs of the slot range: each takes the faces above STEP consecutive slots
 __host__ __device__ __forceinline__ long n_x3_slot_ctas(const Dims &d) {
-    return (n_x3_slots(d) - 1 + BLK - 2) / (BLK - 1);
+    const int h = x3_halo(d), step = BLK - 1 - 2 * h;
+    return (n_x3_slots(d) - 1 - 2 * h + step - 1) / step;
 }
 
 template <typename T, int REC>
@@ -453,8 +493,7 @@ __global__ void __launch_bounds__(BLK, sizeof(T) == 8 ? ((REC & 2) != 0 ? HAMR_F
 // per SM for the row kernels (FP64, float). Measured on the 384 x 192 x 192
 // torus: rows of 12 beat 6, 8, 24 and 48 (shorter rows: more threads in
 // flight, longer: fewer extra reconstructions); 7 float blocks beat 6 and 8,
-// 5 double blocks beat 4. The stencil window (RowWindow) took the float x1 +
-// x2 fluxes from 4.48 to 3.77 ms per step (FP64 13.49 -> 13.36).
+// 5 double blocks beat 4.
 #ifndef HAMR_FLUX_ROW
 #define HAMR_FLUX_ROW 12
 #endif
@@ -473,48 +512,73 @@ __host__ __device__ __forceinline__ long n_flux_rows(const Dims &d) {
     return ((nf + FLUX_ROW - 1) / FLUX_ROW) * nt * (d.n3 + 2 * d.d3);
 }
 
-// A thread's stencil window along its row, in shared memory: the NW zones
-// (5 for PPM, 3 for MC) around the zone being reconstructed, each as its
-// NPR - 1 reconstructed primitives (the normal field component is not
-// reconstructed), converted to T once when loaded. Slot of zone index q along
-// the row: q mod NW. Each thread touches only its own column (threadIdx.x), so
-// no barrier is needed, and consecutive threads hit consecutive banks. Moving
-// to the next face loads one new zone (NPR - 1 values) instead of the whole
-// stencil (NW (NPR - 1) values); the reconstruction sees the same values as
-// zone_edges.
+// A thread's reconstruction state along its row, in shared memory: NV values
+// for each of the NPR - 1 reconstructed primitives (the normal field component
+// is not reconstructed). Each thread touches only its own column
+// (threadIdx.x), so no barrier is needed, and consecutive threads hit
+// consecutive banks. Moving to the next face loads one new zone. PPM keeps
+// what the next zone shares with the ones behind it -- its value and the one
+// above, its limited slope and the interpolated value on its lower face -- and
+// evaluates one new slope and one new face value per zone, where the five-zone
+// stencil by itself takes three and two (x1 + x2 fluxes of the 384 x 192 x 192
+// torus, per step: FP64 8.92 -> 6.83 ms, mixed 3.61 -> 2.55, bound by the
+// instructions issued and the FP64 pipe). MC keeps the zone and the one below
+// it. Same values as zone_edges, which evaluates the same functions of the
+// same zones.
 template <int DIR, typename T, int REC>
 struct RowWindow {
-    static constexpr int NW = (REC & 1) == HAMR_RECON_MC ? 3 : 5;
-    static constexpr int H = NW / 2;
+    static constexpr bool MC = (REC & 1) == HAMR_RECON_MC;
+    static constexpr int NV = MC ? 2 : 4;
+    static constexpr int H = MC ? 1 : 2;   // zones the stencil reaches on either side
     static constexpr int NK = NPR - 1;
     T *w;
-    __device__ __forceinline__ T &at(int slot, int kk) const { return w[(slot * NK + kk) * BLK]; }
-    __device__ __forceinline__ void load(const Dims &d, const double *__restrict__ pv, long cz, int slot) const {
+    __device__ __forceinline__ T &at(int v, int kk) const { return w[(v * NK + kk) * BLK]; }
+    // state for the zone at cell cz, from the zones below it
+    __device__ __forceinline__ void start(const Dims &d, const double *__restrict__ pv, long cz, long stride) const {
         int kk = 0;
 #pragma unroll
         for (int k = 0; k < NPR; k++) {
             if (k == B1 + DIR - 1) continue;
-            at(slot, kk++) = (T)__ldg(pv + (long)k * d.ks + cz);
+            const double *pk = pv + (long)k * d.ks + cz;
+            const T ym = (T)__ldg(pk - stride), y0 = (T)__ldg(pk);
+            if constexpr (MC) {
+                at(0, kk) = ym;
+                at(1, kk) = y0;
+            } else {
+                const T yl = (T)__ldg(pk - 2 * stride), yp = (T)__ldg(pk + stride);
+                const T dq = ppm_slope(ym, y0, yp);
+                at(0, kk) = y0;
+                at(1, kk) = yp;
+                at(2, kk) = dq;
+                at(3, kk) = ppm_face(ym, y0, ppm_slope(yl, ym, y0), dq);
+            }
+            kk++;
         }
     }
-    // edges of the zone whose stencil starts in slot s0 (the zone q - H)
-    __device__ __forceinline__ void edges(int s0, T *lo, T *hi) const {
+    // edges of the zone at cell cz, whose state this is, and the state of the
+    // next zone; par: parity of the zones passed since start (the two values
+    // of PPM's state swap places)
+    __device__ __forceinline__ void edges(const Dims &d, const double *__restrict__ pv, long cz, long stride, int par,
+                                          T *lo, T *hi) const {
         int kk = 0;
 #pragma unroll
         for (int k = 0; k < NPR; k++) {
             if (k == B1 + DIR - 1) continue;
-            T x[NW];
-#pragma unroll
-            for (int s = 0; s < NW; s++) {
-                const int sl = s0 + s;
-                x[s] = at(sl >= NW ? sl - NW : sl, kk);
-            }
-            if constexpr (NW == 3) {
-                const T temp = T(0.5) * slope_lim(x[0], x[1], x[2]);
-                lo[k] = x[1] - temp;
-                hi[k] = x[1] + temp;
+            const T yn = (T)__ldg(pv + (long)k * d.ks + cz + H * stride);
+            if constexpr (MC) {
+                const T ym = at(par, kk), y0 = at(1 - par, kk);
+                const T temp = T(0.5) * slope_lim(ym, y0, yn);
+                lo[k] = y0 - temp;
+                hi[k] = y0 + temp;
+                at(par, kk) = yn;
             } else {
-                para(x, lo[k], hi[k]);
+                const T y0 = at(par, kk), yp = at(1 - par, kk);
+                const T dq = ppm_slope(y0, yp, yn);
+                const T f = ppm_face(y0, yp, at(2, kk), dq);
+                ppm_limit(y0, at(3, kk), f, lo[k], hi[k]);
+                at(par, kk) = yn;
+                at(2, kk) = dq;
+                at(3, kk) = f;
             }
             kk++;
         }
@@ -522,9 +586,9 @@ struct RowWindow {
 };
 
 // One row of FLUX_ROW faces along DIR (row t < n_flux_rows), reconstructed
-// through the thread's stencil window in `wbuf` (a CTA's NW * NK * BLK
-// values; column threadIdx.x); returns the row's largest signal-speed
-// contribution (ctop_term)
+// through the thread's state in `wbuf` (a CTA's NV * NK * BLK values; column
+// threadIdx.x); returns the row's largest signal-speed contribution
+// (ctop_term)
 template <int DIR, typename T, int REC>
 __device__ __forceinline__ double flux_row(const Dims &d, const Geom &m, const double *__restrict__ pv,
                                            const double *__restrict__ ps, T *__restrict__ F, T *wbuf, const long t) {
@@ -542,32 +606,23 @@ __device__ __forceinline__ double flux_row(const Dims &d, const Geom &m, const d
     const long stride = DIR == 1 ? (long)d.G2 * d.G3 : (long)d.G3;
     const int face = DIR == 1 ? FACE1 : FACE2;
     const Win win{wbuf + threadIdx.x};
-    constexpr int NW = Win::NW, H = Win::H;
     T pl[NPR], lo[NPR], hi[NPR];
-    // the stencil of the zone below the first face, zones f0 - 1 - H ..
-    // f0 - 1 + H (f0 >= ng > H), then its upper edge: the first left state
-    const long cf0 = DIR == 1 ? cix(d, f0, a, z) : cix(d, a, f0, z);
-#pragma unroll
-    for (int s = 0; s < NW; s++) win.load(d, pv, cf0 + (s - 1 - H) * stride, (f0 - 1 - H + s) % NW);
-    win.edges((f0 - 1 - H) % NW, lo, hi);
-#pragma unroll
-    for (int k = 0; k < NPR; k++) pl[k] = hi[k];
-    int s0 = (f0 - H) % NW;   // slot of zone f - H
+    // the zone below the first face (f0 - 1, whose stencil starts at
+    // f0 - 1 - H >= 0): its upper edge is the first left state
+    long c = DIR == 1 ? cix(d, f0, a, z) : cix(d, a, f0, z);
+    win.start(d, pv, c - stride, stride);
+    win.edges(d, pv, c - stride, stride, 0, lo, pl);
+    int par = 1;
     for (int f = f0; f < f1; f++) {
         const int i = DIR == 1 ? f : a, j = DIR == 1 ? a : f;
-        const long c = cix(d, i, j, z);
-        // zone f + H replaces zone f - H - 1 (slot s0 + 2H, mod NW)
-        win.load(d, pv, c + H * stride, s0 == 0 ? NW - 1 : s0 - 1);
-        win.edges(s0, lo, hi);
-        s0 = s0 == NW - 1 ? 0 : s0 + 1;
+        win.edges(d, pv, c, stride, par, lo, hi);
+        par ^= 1;
         Geo<T> gm;
         load_geo_t(d, m, i, j, face, gm);
-        T l[NPR];
-#pragma unroll
-        for (int k = 0; k < NPR; k++) l[k] = pl[k];
-        cmx = d_max(cmx, flux_eval<DIR, T, REC>(d, gm, ps, l, lo, F, c, j));
+        cmx = d_max(cmx, flux_eval<DIR, T, REC>(d, gm, ps, pl, lo, F, c, j));
 #pragma unroll
         for (int k = 0; k < NPR; k++) pl[k] = hi[k];
+        c += stride;
     }
     return cmx;
 }
@@ -578,7 +633,7 @@ __global__ void __launch_bounds__(BLK, sizeof(T) == 8 ? ((REC & 2) != 0 ? HAMR_F
     k_flux_rows(const Dims d, const Geom m, const double *__restrict__ pv, const double *__restrict__ ps,
                 T *__restrict__ F, unsigned long long *__restrict__ dtbits, int calc_dt) {
     using Win = RowWindow<DIR, T, REC>;
-    __shared__ T wbuf[Win::NW * Win::NK * BLK];
+    __shared__ T wbuf[Win::NV * Win::NK * BLK];
     const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
     const double cmx = t < n_flux_rows<DIR>(d) ? flux_row<DIR, T, REC>(d, m, pv, ps, F, wbuf, t) : 0.0;
     if (calc_dt) cta_max_ctop(d, DIR, cmx, &dtbits[DIR]);
@@ -1125,7 +1180,10 @@ __device__ __forceinline__ void source(double gam, const double *ph, const Geo<d
 // are left out wherever U[B] is set from the updated faces before anything
 // reads it (face_average_b: B1 and B2 always, B3 on 3-D blocks), so their
 // flux divergences, their planes of the U(p^n) cache and their staged fluxes
-// need not exist. U[B] returned by the update is zero there.
+// need not exist. U[B] returned by the update is zero there. Update with the
+// primary inversion on the 384 x 192 x 192 torus, per step: FP64 5.20 -> 3.76
+// ms (the smaller staging also lets a third CTA of 192-zone rows onto an SM),
+// mixed 4.23 -> 3.92.
 constexpr int N_ADV = 6;   // RHO, UU, U1, U2, U3, KTOT (and B3 on 2-D blocks)
 __host__ __device__ constexpr int adv_comp(int q) { return q < 5 ? q : KTOT; }
 

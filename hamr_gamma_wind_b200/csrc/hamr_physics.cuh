@@ -62,6 +62,8 @@ template <> __device__ __forceinline__ double d_pow<double>(double x, double y) 
 // per step, L1 of every field against FP64 after 1000 steps unchanged
 template <> __device__ __forceinline__ float d_pow<float>(float x, float y) { return __powf(x, y); }
 template <typename T> __device__ __forceinline__ T d_fabs(T x) { return x < T(0) ? -x : x; }
+__device__ __forceinline__ double d_fabs(double x) { return fabs(x); }   // an operand modifier, not a comparison
+__device__ __forceinline__ float d_fabs(float x) { return fabsf(x); }
 // x^(-1/2), correctly rounded in all but vanishingly rare near-midpoint cases,
 // so that it agrees with a correctly rounded host pow(x, -0.5): the IEEE
 // quotient 1/sqrt(x) (within about one ulp) takes one Newton step
@@ -290,36 +292,71 @@ __device__ __forceinline__ T div6(T a) {
     }
 }
 
+// x < 0 and x > 0 of a double from the bits of its upper word, so that the
+// test runs on the integer pipe and not on the FP64 one, where PPM's dozen
+// comparisons per value would queue with its arithmetic. Same answers as the
+// comparison, infinities, zeros of either sign and NaNs (false) included,
+// save that a magnitude below 2^-1042 counts as zero.
+__device__ __forceinline__ bool is_neg(double x) { return (unsigned)__double2hiint(x) - 0x80000001u < 0x7ff00000u; }
+__device__ __forceinline__ bool is_pos(double x) { return (unsigned)__double2hiint(x) - 1u < 0x7ff00000u; }
+__device__ __forceinline__ bool is_neg(float x) { return x < 0.f; }
+__device__ __forceinline__ bool is_pos(float x) { return x > 0.f; }
+
+// PPM in three parts, each a value that neighbouring zones share, so that a
+// kernel that walks or shares a row evaluates it once:
+//   ppm_slope   the limited slope of a zone (its five-zone stencils overlap
+//               three times), min(2|a|, 2|b|, |a + b|/2) with the sign of the
+//               centred difference, zero at an extremum. The doublings of the
+//               reference's form are folded into one exact scaling at the end
+//               (powers of two), which gives the same value bit for bit;
+//   ppm_face    the interpolated value between two zones, the upper edge of
+//               one and the lower edge of the next;
+//   ppm_limit   the monotonised edges of a zone from its value and the two.
+template <typename T>
+__device__ __forceinline__ T ppm_slope(T y0, T y1, T y2) {
+    const T a = y1 - y0, b = y2 - y1, c = y2 - y0;
+    const T m = T(4.) * d_min(d_fabs(a), d_fabs(b));
+    const T v = T(0.5) * d_min(d_fabs(c), m);
+    // the product's sign; in float scaled as the reference's, so that it
+    // underflows no earlier
+    const T s = sizeof(T) == 4 ? (T(4.) * a) * b : a * b;
+    return is_pos(s) ? (is_pos(c) ? v : -v) : T(0.);
+}
+template <typename T>
+__device__ __forceinline__ T ppm_face(T y1, T y2, T dq1, T dq2) {
+    return T(0.5) * (y2 + y1) - div6(dq2 - dq1);
+}
+template <typename T>
+__device__ __forceinline__ void ppm_limit(T y, T l, T r, T &lout, T &rout) {
+    const T qa = (r - y) * (y - l);
+    const T qd = (r - l);
+    const T qe = T(6.0) * (y - T(0.5) * (l + r));
+    if (qa <= T(0.)) { l = y; r = y; }
+    if (is_neg(qd * (qd - qe))) l = T(3.0) * y - T(2.0) * r;
+    else if (is_neg(qd * (qd + qe))) r = T(3.0) * y - T(2.0) * l;
+    lout = l;
+    rout = r;
+}
+
 // PPM face values of the middle of five zones: l = lower edge, r = upper edge
 template <typename T>
 __device__ __forceinline__ void para(const T *y, T &lout, T &rout) {
-    T dq[5];
+    const T d1 = ppm_slope(y[0], y[1], y[2]), d2 = ppm_slope(y[1], y[2], y[3]), d3 = ppm_slope(y[2], y[3], y[4]);
+    ppm_limit(y[2], ppm_face(y[1], y[2], d1, d2), ppm_face(y[2], y[3], d2, d3), lout, rout);
+}
+
+// the two states at the face between the third and fourth of six zones: the
+// upper edge of the third (hi2) and the lower edge of the fourth (lo3)
+template <typename T>
+__device__ __forceinline__ void para_face(const T *y, T &hi2, T &lo3) {
+    T dq[4];
 #pragma unroll
-    for (int i = 1; i < 4; i++) {
-        T Dqm = T(2.) * (y[i] - y[i - 1]);
-        T Dqp = T(2.) * (y[i + 1] - y[i]);
-        T Dqc = T(0.5) * (y[i + 1] - y[i - 1]);
-        T aDqm = d_fabs(Dqm), aDqp = d_fabs(Dqp), aDqc = d_fabs(Dqc);
-        T s = Dqm * Dqp;
-        Dqm = d_min(aDqm, aDqp);
-        if (aDqc < Dqm) {
-            if (Dqc > T(0.)) dq[i] = (aDqc) * (T)(s > T(0.));
-            else dq[i] = (-aDqc) * (T)(s > T(0.));
-        } else {
-            if (Dqc > T(0.)) dq[i] = (Dqm) * (T)(s > T(0.));
-            else dq[i] = (-Dqm) * (T)(s > T(0.));
-        }
-    }
-    T l = T(0.5) * (y[2] + y[1]) - div6(dq[2] - dq[1]);
-    T r = T(0.5) * (y[3] + y[2]) - div6(dq[3] - dq[2]);
-    T qa = (r - y[2]) * (y[2] - l);
-    T qd = (r - l);
-    T qe = T(6.0) * (y[2] - T(0.5) * (l + r));
-    if (qa <= T(0.)) { l = y[2]; r = y[2]; }
-    if (qd * (qd - qe) < T(0.0)) l = T(3.0) * y[2] - T(2.0) * r;
-    else if (qd * (qd + qe) < T(0.0)) r = T(3.0) * y[2] - T(2.0) * l;
-    lout = l;
-    rout = r;
+    for (int k = 0; k < 4; k++) dq[k] = ppm_slope(y[k], y[k + 1], y[k + 2]);
+    const T f1 = ppm_face(y[1], y[2], dq[0], dq[1]), f2 = ppm_face(y[2], y[3], dq[1], dq[2]),
+            f3 = ppm_face(y[3], y[4], dq[2], dq[3]);
+    T drop;
+    ppm_limit(y[2], f1, f2, drop, hi2);
+    ppm_limit(y[3], f2, f3, lo3, drop);
 }
 
 // ---------------------------------------------------------------- inversion
