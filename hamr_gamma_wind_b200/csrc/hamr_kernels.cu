@@ -65,13 +65,73 @@ struct Geom {
     // reciprocal (11-15), with geo_lapse's operations (k_inv_tab). Brace
     // initialisation with the four metric tables leaves it null.
     const double *itab;
+    // the same metric point by point (GeoTab), in the arithmetic type of the
+    // step; null where a warp's lanes would read many points (geo_tab_wanted)
+    const double *gtab;
+    const float *gtabf;
 };
+
+// One point's metric as one block of GT values: the whole of what the HLL
+// fluxes and the EMFs read first, in 16 values, then the rest. The lanes of a
+// warp share a column wherever phi runs long, so a block is four or eight
+// 16-byte loads, each one transaction for the warp, where the planes above
+// take an address and a load per component (and in the mixed step a
+// conversion). Block (loc, column) at (loc * gs + column) * GT.
+constexpr int GT = 32;
+enum { GT_COV = 0, GT_G = 10, GT_RLAPSE = 11, GT_CON0 = 12, GT_CON = 13, GT_LAPSE = 22 };   // g^tt, then the other nine
+
+// Blocks pay where the lanes of a warp read few columns: n3 of half a warp.
+// On 2-D blocks, where every lane has a column of its own, the planes'
+// neighbouring columns coalesce and blocks would not.
+constexpr int GEO_TAB_MIN_N3 = 16;
+__host__ __device__ __forceinline__ bool geo_tab_wanted(int n3) { return n3 >= GEO_TAB_MIN_N3; }
+
+__device__ __forceinline__ void load16(const double *p, double *o) {
+    const double2 *q = reinterpret_cast<const double2 *>(p);
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+        const double2 v = __ldg(q + k);
+        o[2 * k] = v.x;
+        o[2 * k + 1] = v.y;
+    }
+}
+__device__ __forceinline__ void load16(const float *p, float *o) {
+    const float4 *q = reinterpret_cast<const float4 *>(p);
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const float4 v = __ldg(q + k);
+        o[4 * k] = v.x;
+        o[4 * k + 1] = v.y;
+        o[4 * k + 2] = v.z;
+        o[4 * k + 3] = v.w;
+    }
+}
+
+// metric of a block of the point-by-point table
+template <typename T>
+__device__ __forceinline__ void load_geo_block(const T *q, Geo<T> &o) {
+    T v[GT];
+    load16(q, v);
+    load16(q + 16, v + 16);   // what of it is not used is not loaded
+#pragma unroll
+    for (int s = 0; s < 10; s++) o.gcov[s] = v[GT_COV + s];
+    o.g = v[GT_G];
+    o.rlapse = v[GT_RLAPSE];
+    o.gcon[0] = v[GT_CON0];
+#pragma unroll
+    for (int s = 1; s < 10; s++) o.gcon[s] = v[GT_CON + s - 1];
+    o.lapse = v[GT_LAPSE];
+}
 
 __device__ __forceinline__ long cix(const Dims &d, int i, int j, int z) { return ((long)i * d.G2 + j) * d.G3 + z; }
 __device__ __forceinline__ long gix(const Dims &d, int i, int j) { return (long)i * d.G2 + j; }
 
 __device__ __forceinline__ void load_geo(const Dims &d, const Geom &m, int i, int j, int loc, Geo<double> &o) {
     long idx = gix(d, i, j);
+    if (m.gtab) {
+        load_geo_block(m.gtab + ((long)loc * d.gs + idx) * GT, o);
+        return;
+    }
 #pragma unroll
     for (int s = 0; s < 10; s++) {
         o.gcon[s] = __ldg(&m.gcon[(long)(s * 5 + loc) * d.gs + idx]);
@@ -96,6 +156,13 @@ __device__ __forceinline__ double div_face_volume(const Dims &d, const Geom &m, 
 template <typename T>
 __device__ __forceinline__ void load_geo_t(const Dims &d, const Geom &m, int i, int j, int loc, Geo<T> &o) {
     long idx = gix(d, i, j);
+    const T *tab;
+    if constexpr (sizeof(T) == sizeof(double)) tab = m.gtab;
+    else tab = m.gtabf;
+    if (tab) {
+        load_geo_block(tab + ((long)loc * d.gs + idx) * GT, o);
+        return;
+    }
 #pragma unroll
     for (int s = 0; s < 10; s++) {
         o.gcon[s] = (T)__ldg(&m.gcon[(long)(s * 5 + loc) * d.gs + idx]);
@@ -1376,6 +1443,37 @@ __global__ void k_inv_tab(const Dims d, const double *__restrict__ gcon, const d
     }
 }
 
+// the point-by-point table from the planes and the column table: one thread
+// per column and location; every value is the one load_geo_t would form from
+// the planes (in float the converted component, and the lapse of the converted
+// metric)
+template <typename T>
+__global__ void k_geo_tab(const Dims d, const Geom m, T *__restrict__ tab) {
+    const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= 5 * d.gs) return;
+    const int loc = (int)(t / d.gs);
+    const long idx = t % d.gs;
+    Geo<T> o;
+#pragma unroll
+    for (int s = 0; s < 10; s++) {
+        o.gcon[s] = (T)m.gcon[(long)(s * 5 + loc) * d.gs + idx];
+        o.gcov[s] = (T)m.gcov[(long)(s * 5 + loc) * d.gs + idx];
+    }
+    o.g = (T)m.gdet[(long)loc * d.gs + idx];
+    if constexpr (sizeof(T) == sizeof(double)) {
+        o.lapse = m.itab[(long)(6 + loc) * d.gs + idx];
+        o.rlapse = m.itab[(long)(11 + loc) * d.gs + idx];
+    } else {
+        geo_lapse(o);
+    }
+    T *q = tab + t * GT;
+    for (int s = 0; s < 10; s++) q[GT_COV + s] = o.gcov[s];
+    q[GT_G] = o.g;
+    q[GT_RLAPSE] = o.rlapse;
+    q[GT_CON0] = o.gcon[0];
+    for (int s = 1; s < 10; s++) q[GT_CON + s - 1] = o.gcon[s];
+    q[GT_LAPSE] = o.lapse;
+}
 
 // primary solver: Noble 2D, or Newman-Hamlin in its place (NEWMAN builds)
 template <int INV>
@@ -1454,9 +1552,18 @@ __global__ void __launch_bounds__(BLK, HAMR_CONS_MINB) k_cons(const Dims d, cons
 
 // The same update with the zones' metric and connection staged in shared
 // memory: the zones of a CTA lie in at most three (i, j) columns when
-// n3 >= 64 (z runs fastest), whose 61 metric and connection values each are
+// n3 >= 64 (z runs fastest), whose metric and connection values each are
 // loaded once per CTA instead of once per zone.
-constexpr int COL_VALS = 61;   // gcov 10, gcon 10, gdet 1 (centre), conn 40
+constexpr int COL_VALS = 63;   // gcov 10, gcon 10, gdet 1, lapse and its reciprocal (centre), conn 40
+constexpr int COL_CONN = 23;
+// staged values 21 .. of a column: the lapse and its reciprocal (in place
+// where there is no column table), then the connection
+__device__ __forceinline__ double column_value(const Geom &m, long gs, long gi, int v) {
+    if (v >= COL_CONN) return m.conn[(long)(v - COL_CONN) * gs + gi];
+    if (m.itab) return m.itab[(long)(v == 21 ? 6 + CENT : 11 + CENT) * gs + gi];
+    const double a = 1. / sqrt(-m.gcon[(long)CENT * gs + gi]);
+    return v == 21 ? a : 1. / a;
+}
 template <typename T>
 __global__ void __launch_bounds__(BLK, HAMR_CONS_MINB) k_cons_cols(const Dims d, const Geom m,
                                                const double *__restrict__ pin, const double *__restrict__ pb,
@@ -1479,7 +1586,7 @@ __global__ void __launch_bounds__(BLK, HAMR_CONS_MINB) k_cons_cols(const Dims d,
         if (v < 10) x = m.gcov[(long)(v * 5 + CENT) * gs + gi];
         else if (v < 20) x = m.gcon[(long)((v - 10) * 5 + CENT) * gs + gi];
         else if (v == 20) x = m.gdet[(long)CENT * gs + gi];
-        else x = m.conn[(long)(v - 21) * gs + gi];
+        else x = column_value(m, gs, gi, v);
         sg[e / COL_VALS][v] = x;
     }
     __syncthreads();
@@ -1494,9 +1601,10 @@ __global__ void __launch_bounds__(BLK, HAMR_CONS_MINB) k_cons_cols(const Dims d,
 #pragma unroll
     for (int q = 0; q < 10; q++) { gm.gcov[q] = g[q]; gm.gcon[q] = g[10 + q]; }
     gm.g = g[20];
-    geo_lapse(gm);
+    gm.lapse = g[21];
+    gm.rlapse = g[22];
     double pf[NPR], U[NPR];
-    cons_update<T>(d, m, pin, pb, Ucache, F1, F2, F3, full, st.sub(), i, j, c, gi, gm, ConnStaged{g + 21}, pf, U);
+    cons_update<T>(d, m, pin, pb, Ucache, F1, F2, F3, full, st.sub(), i, j, c, gi, gm, ConnStaged{g + COL_CONN}, pf, U);
     W[0 * d.ks + c] = U[RHO];
     W[1 * d.ks + c] = U[UU];
     W[2 * d.ks + c] = U[U1];
@@ -1670,7 +1778,7 @@ __device__ __forceinline__ void cons_tma_row(const Dims &d, const Geom &m, const
         if (v < 10) x = m.gcov[(long)(v * 5 + CENT) * d.gs + gi];
         else if (v < 20) x = m.gcon[(long)((v - 10) * 5 + CENT) * d.gs + gi];
         else if (v == 20) x = m.gdet[(long)CENT * d.gs + gi];
-        else x = m.conn[(long)(v - 21) * d.gs + gi];
+        else x = column_value(m, d.gs, gi, v);
         sg[v] = x;
     }
     __syncthreads();
@@ -1696,9 +1804,10 @@ __device__ __forceinline__ void cons_tma_row(const Dims &d, const Geom &m, const
 #pragma unroll
     for (int q = 0; q < 10; q++) { gm.gcov[q] = sg[q]; gm.gcon[q] = sg[10 + q]; }
     gm.g = sg[20];
-    geo_lapse(gm);
+    gm.lapse = sg[21];
+    gm.rlapse = sg[22];
     double pf[NPR], U[NPR];
-    cons_update_fx<T>(d, m, pin, pb, Ucache, fx, full, st.sub(), i, j, c, gi, gm, ConnStaged{sg + 21}, pf, U);
+    cons_update_fx<T>(d, m, pin, pb, Ucache, fx, full, st.sub(), i, j, c, gi, gm, ConnStaged{sg + COL_CONN}, pf, U);
     auto write_w = [&](const double *w) {   // 3-D: the faces set U[B]
 #pragma unroll
         for (int q = 0; q < N_ADV; q++) W[q * ks + c] = w[q];
@@ -2268,6 +2377,8 @@ struct hamr_ctx {
     int *pflag = nullptr, *failimage = nullptr;
     double *gcov = nullptr, *gcon = nullptr, *gdet = nullptr, *conn = nullptr;
     double *itab = nullptr;   // the column table of reciprocals (k_inv_tab), 16 planes of gs
+    double *gtab = nullptr;   // the metric point by point (k_geo_tab), FP64 step, or
+    float *gtabf = nullptr;   // mixed step; neither on blocks with short phi rows
     unsigned long long *dtbits = nullptr;
     double *ndt = nullptr, *dt_state = nullptr;
     int *counter = nullptr;
@@ -2292,7 +2403,7 @@ int fail_cuda(hamr_ctx *c, cudaError_t e, const char *what) {
         if (e_ != cudaSuccess) return fail_cuda(ctx, e_, #call); \
     } while (0)
 
-Geom geom_of(const hamr_ctx *c) { return Geom{c->gcov, c->gcon, c->gdet, c->conn, c->itab}; }
+Geom geom_of(const hamr_ctx *c) { return Geom{c->gcov, c->gcon, c->gdet, c->conn, c->itab, c->gtab, c->gtabf}; }
 
 // the error word kernels set when a bounded wait gave up (read after a
 // synchronisation the caller already makes; cleared once reported)
@@ -2663,6 +2774,8 @@ int hamr_ctx_create(const hamr_params *prm, hamr_ctx **out) {
         {(void **)&ctx->gcov, 50 * sizeof(double) * d.gs}, {(void **)&ctx->gcon, 50 * sizeof(double) * d.gs},
         {(void **)&ctx->gdet, 5 * sizeof(double) * d.gs}, {(void **)&ctx->conn, 40 * sizeof(double) * d.gs},
         {(void **)&ctx->itab, 16 * sizeof(double) * d.gs},
+        {(void **)&ctx->gtab, geo_tab_wanted(d.n3) && prm->precision == HAMR_FP64 ? 5 * GT * sizeof(double) * d.gs : 0},
+        {(void **)&ctx->gtabf, geo_tab_wanted(d.n3) && prm->precision == HAMR_MIXED ? 5 * GT * sizeof(float) * d.gs : 0},
         {(void **)&ctx->dtbits, 4 * sizeof(unsigned long long)}, {(void **)&ctx->ndt, sizeof(double)},
         {(void **)&ctx->dt_state, sizeof(double)}, {(void **)&ctx->counter, sizeof(int)},
         {(void **)&ctx->divb, sizeof(unsigned long long)},
@@ -2707,7 +2820,7 @@ int hamr_ctx_destroy(hamr_ctx *ctx) {
     if (ctx->graph) cudaGraphExecDestroy(ctx->graph);
     void *bufs[] = {ctx->p, ctx->ph, ctx->ps, ctx->psh, ctx->U, ctx->F1, ctx->F2, ctx->F3, ctx->Ec, ctx->emf,
                     ctx->W, ctx->pflag, ctx->failimage, ctx->gcov, ctx->gcon, ctx->gdet, ctx->conn, ctx->itab,
-                    ctx->dtbits,
+                    ctx->gtab, ctx->gtabf, ctx->dtbits,
                     ctx->ndt, ctx->dt_state, ctx->counter, ctx->divb, ctx->rlist, ctx->rcount,
                     ctx->flist, ctx->nfail, ctx->kerr};
     for (void *b : bufs)
@@ -2738,6 +2851,8 @@ int hamr_set_geometry(hamr_ctx *ctx, const double *gcov, const double *gcon, con
     CK(cudaMemcpyAsync(ctx->gdet, gdet, 5 * g, cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemcpyAsync(ctx->conn, conn, 40 * g, cudaMemcpyHostToDevice, ctx->stream));
     k_inv_tab<<<nblk(ctx->d.gs), BLK, 0, ctx->stream>>>(ctx->d, ctx->gcon, ctx->gdet, ctx->itab);
+    if (ctx->gtab) k_geo_tab<double><<<nblk(5 * ctx->d.gs), BLK, 0, ctx->stream>>>(ctx->d, geom_of(ctx), ctx->gtab);
+    if (ctx->gtabf) k_geo_tab<float><<<nblk(5 * ctx->d.gs), BLK, 0, ctx->stream>>>(ctx->d, geom_of(ctx), ctx->gtabf);
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(ctx->stream));
     ctx->have_geom = true;
