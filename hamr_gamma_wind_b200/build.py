@@ -2,8 +2,9 @@
 
 Two shared objects come out of the same sources:
   libhamr_b200.so         production build (fused multiply-add contraction on)
-  libhamr_b200_strict.so  --fmad=false: reproduces the reference's operation
-                          order, used by the bit-level parity tests
+  libhamr_b200_strict.so  --fmad=false and HAMR_STRICT: reproduces the
+                          reference's operation order, used by the bit-level
+                          parity tests
 """
 import os
 import subprocess
@@ -21,7 +22,7 @@ NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 
 TARGETS = {
     "libhamr_b200.so": [],
-    "libhamr_b200_strict.so": ["--fmad=false"],
+    "libhamr_b200_strict.so": ["--fmad=false", "-DHAMR_STRICT"],
 }
 
 

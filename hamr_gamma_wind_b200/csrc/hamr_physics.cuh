@@ -35,6 +35,16 @@ constexpr double W_TOO_BIG = 1.e20;
 constexpr double UTSQ_TOO_BIG = 1.e20;
 constexpr double FAIL_VAL = 1.e30;
 
+// The strict build (HAMR_STRICT, compiled without contraction) keeps the
+// reference's operation order and roundings, which pins the arithmetic to the
+// reference bit for bit; the production build may use any form of the same
+// formulas that is as accurate. Code that differs says so with this flag.
+#ifdef HAMR_STRICT
+constexpr bool STRICT = true;
+#else
+constexpr bool STRICT = false;
+#endif
+
 template <typename T>
 struct Geo {
     T gcov[10], gcon[10], g;
@@ -116,23 +126,36 @@ __device__ __forceinline__ void geo_lapse(Geo<T> &o) {
     o.rlapse = T(1.) / o.lapse;   // read by the double-precision quotients only
 }
 
-// Quotients a_k / b that share one divisor. In double precision: one IEEE
-// reciprocal of b, then the exact form per quotient (div_rcp_inf: the IEEE
-// quotient bit for bit for 2^-900 <= |a| <= 2^900, zeros and infinities),
-// which replaces all but one full division by three operations. Other types
-// (float, whose division is already the approximate one in the mixed step,
-// and the adjoint's dual numbers) divide as written.
+// Quotients a_k / b that share one divisor: one reciprocal of b, then per
+// quotient a product (within 1.5 ulp, as accurate as the sums these quotients
+// enter), or in the strict build's double precision the exact form
+// (div_rcp_inf: the IEEE quotient bit for bit for 2^-900 <= |a| <= 2^900,
+// zeros and infinities). The adjoint's dual numbers divide as written.
 template <typename T>
 struct Divisor {
     T b, rb;
     __device__ __forceinline__ explicit Divisor(T b_) : b(b_), rb(b_) {
-        if constexpr (std::is_same<T, double>::value) rb = 1.0 / b_;
+        if constexpr (std::is_floating_point<T>::value) rb = T(1.0) / b_;
     }
     // with the divisor's reciprocal already at hand (rounded once, 1/b)
     __device__ __forceinline__ Divisor(T b_, T rb_) : b(b_), rb(rb_) {}
     __device__ __forceinline__ T div(T a) const {
-        if constexpr (std::is_same<T, double>::value) return div_rcp_inf(a, b, rb);
+        if constexpr (std::is_same<T, double>::value && STRICT) return div_rcp_inf(a, b, rb);
+        else if constexpr (std::is_floating_point<T>::value) return a * rb;
         else return a / b;
+    }
+};
+
+// the same with IEEE quotients in both builds: HLLD's pressure solve differences
+// a residual over a relative step of 1e-10, so the last bits of its quotients
+// are what its root is good to
+template <typename T>
+struct ExactDivisor {
+    T b, rb;
+    __device__ __forceinline__ explicit ExactDivisor(T b_) : b(b_), rb(T(1.0) / b_) {}
+    __device__ __forceinline__ T div(T a) const {
+        if constexpr (std::is_same<T, double>::value) return div_rcp_inf(a, b, rb);
+        else return a * rb;
     }
 };
 
@@ -173,9 +196,16 @@ __device__ __forceinline__ void ucon_calc(const T *pr, const Geo<G> &gm, T *ucon
     const G alpha = gm.lapse;   // 1/sqrt(-g^tt), from the Geo (tabulated or geo_lapse)
     G beta[4];
     T gamma;
+    gamma_calc(pr, gm, &gamma);
+    if constexpr (std::is_same<T, G>::value && !STRICT) {
+        // beta^j / alpha = alpha g^tj: no division is left
+        ucon[0] = gamma * gm.rlapse;
+#pragma unroll
+        for (int j = 1; j < 4; j++) ucon[j] = pr[U1 + j - 1] - gamma * (gm.gcon[j] * alpha);
+        return;
+    }
 #pragma unroll
     for (int j = 1; j < 4; j++) beta[j] = gm.gcon[j] * alpha * alpha;
-    gamma_calc(pr, gm, &gamma);
     if constexpr (std::is_same<T, G>::value) {
         const Divisor<T> da(alpha, gm.rlapse);   // four quotients by the lapse
         ucon[0] = da.div(gamma);
@@ -265,6 +295,62 @@ __device__ __forceinline__ void primtoflux(T gam, const T *pr, const State<T> &q
     }
 }
 
+// One side of an HLL face in the production build: fluxes along DIR and
+// conserved variables, both without sqrt(-g) (the caller's HLL weights carry
+// it), and the fast speeds along DIR. get_state and primtoflux in both
+// directions in one, sharing what they share, and with
+//   b^i u^t - b^t u^i = B^i                 (the conserved field)
+//   c_s^2 + v_A^2 - c_s^2 v_A^2 = (gamma P + b^2) / (w + b^2)
+// and the halved quadratic for the speeds. The normal field's flux is zero and
+// left out.
+template <int DIR, typename T>
+__device__ __forceinline__ void hll_side(T gam, const T *pr, const Geo<T> &gm, T *F, T *U, T &vmax, T &vmin) {
+    T u[4], ul[4], b[4], bl[4];
+    ucon_calc(pr, gm, u);
+    lower4(u, gm.gcov, ul);
+    bcon_calc(pr, u, ul, b);
+    lower4(b, gm.gcov, bl);
+    const T P = (gam - T(1.)) * pr[UU], gP = gam * P;
+    const T bsq = dot4(b, bl);
+    const T eta = pr[RHO] + gam * pr[UU] + bsq;
+    const T ptot = P + T(0.5) * bsq;
+    const T ent = P * d_pow(pr[RHO], -gam);
+    F[RHO] = pr[RHO] * u[DIR];
+    U[RHO] = pr[RHO] * u[0];
+    F[KTOT] = F[RHO] * ent;
+    U[KTOT] = U[RHO] * ent;
+    const T ed = eta * u[DIR], e0 = eta * u[0];
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        F[UU + j] = ed * ul[j] - b[DIR] * bl[j];
+        U[UU + j] = e0 * ul[j] - b[0] * bl[j];
+    }
+    F[UU + DIR] += ptot;
+    F[UU] += F[RHO];
+    U[UU] += ptot + U[RHO];
+#pragma unroll
+    for (int j = 1; j < 4; j++)
+        if (j != DIR) {
+            F[B1 + j - 1] = b[j] * u[DIR] - b[DIR] * u[j];
+            U[B1 + j - 1] = pr[B1 + j - 1];
+        }
+    T c2 = (gP + bsq) / eta;
+    if (c2 < T(0.)) c2 = T(SMALL_D);
+    if (c2 > T(1.)) c2 = T(1.);
+    constexpr int sdd = DIR == 1 ? 4 : (DIR == 2 ? 7 : 9);
+    const T u02 = u[0] * u[0], u0d = u[0] * u[DIR], ud2 = u[DIR] * u[DIR];
+    const T A = u02 - (gm.gcon[0] + u02) * c2;
+    const T B = u0d - (gm.gcon[DIR] + u0d) * c2;
+    const T C = ud2 - (gm.gcon[sdd] + ud2) * c2;
+    T disc = B * B - A * C;
+    if (disc < T(0.)) disc = T(0.);
+    disc = d_sqrt(disc);
+    const T rA = T(1.) / A;
+    const T vp = (B - disc) * rA, vm = (B + disc) * rA;
+    vmax = d_max(vp, vm);
+    vmin = d_min(vp, vm);
+}
+
 // monotonized-central slope with the GPU's steepening factor 2 (slope_lim,
 // GPU_interp.h:2-38); a zone's face values are y -+ slope/2
 template <typename T>
@@ -279,17 +365,14 @@ __device__ __forceinline__ T slope_lim(T y1, T y2, T y3) {
     return Dqc;
 }
 
-// a / 6 for PPM's edge correction: in double precision by the exact
-// reciprocal form (div_rcp; the IEEE quotient bit for bit for
+// a / 6 for PPM's edge correction: in the strict build's double precision by
+// the exact reciprocal form (div_rcp; the IEEE quotient bit for bit for
 // 2^-900 <= |a| <= 2^900 and zeros, the range of differences of limited
-// slopes of the state), else the type's own division
+// slopes of the state), else a product
 template <typename T>
 __device__ __forceinline__ T div6(T a) {
-    if constexpr (std::is_same<T, double>::value) {
-        return div_rcp(a, 6.0, 1.0 / 6.0);
-    } else {
-        return a / T(6.0);
-    }
+    if constexpr (std::is_same<T, double>::value && STRICT) return div_rcp(a, 6.0, 1.0 / 6.0);
+    else return a * T(1.0 / 6.0);
 }
 
 // x < 0 and x > 0 of a double from the bits of its upper word, so that the
@@ -1045,17 +1128,17 @@ __device__ __forceinline__ void hlld_side(int dir, T ptot, T S, T sgn, T BX, con
     const T C = R[U_2] * R[B_2] + R[U_3] * R[B_3];
     const T Q = -A - G + (BX * BX) * (T(1.) - S * S);
     const T X = BX * (A * S * BX + C) - (A + G) * (S * ptot - R[UU]);
-    const Divisor<T> dX(X);   // quotients sharing a divisor (exact form in FP64)
+    const ExactDivisor<T> dX(X);   // quotients sharing a divisor (exact form in FP64)
     v[G_1] = dX.div(BX * (A * BX + S * C) - (A + G) * (ptot + R[U_1]));
     v[G_2] = dX.div(Q * R[U_2] + R[B_2] * (C + BX * (S * R[U_1] + R[UU])));
     v[G_3] = dX.div(Q * R[U_3] + R[B_3] * (C + BX * (S * R[U_1] + R[UU])));
     w = ptot + (-R[UU] - (v[G_1] * R[U_1] + v[G_2] * R[U_2] + v[G_3] * R[U_3])) / (S - v[G_1] + T(SMALL_D));
     Bs[G_1] = BX;
-    const Divisor<T> dS(S - v[G_1]);
+    const ExactDivisor<T> dS(S - v[G_1]);
     Bs[G_2] = dS.div(R[B_2] - Bs[G_1] * v[G_2]);
     Bs[G_3] = dS.div(R[B_3] - Bs[G_1] * v[G_3]);
     eta = sgn * ((T)(BX > T(0.0)) - (T)(BX <= T(0.0))) * d_sqrt(d_fabs(w));
-    const Divisor<T> dden(S * ptot - R[UU] + BX * eta);
+    const ExactDivisor<T> dden(S * ptot - R[UU] + BX * eta);
     K[G_1] = dden.div(R[U_1] + ptot + R[B_1] * eta);
     K[G_2] = dden.div(R[U_2] + R[B_2] * eta);
     K[G_3] = dden.div(R[U_3] + R[B_3] * eta);
@@ -1069,7 +1152,7 @@ __device__ __forceinline__ T hlld_error(int dir, T ptot, T cmin, T cmax, T BX, c
     hlld_side(dir, ptot, cmin, T(-1.), BX, R_l, f.v_al, f.B_al, f.K_al, f.w_al, f.eta_l);
     hlld_side(dir, ptot, cmax, T(1.), BX, R_r, f.v_ar, f.B_ar, f.K_ar, f.w_ar, f.eta_r);
     f.B_c[G_1] = BX;
-    const Divisor<T> dK(f.K_ar[dir] - f.K_al[dir] + T(1e-12));
+    const ExactDivisor<T> dK(f.K_ar[dir] - f.K_al[dir] + T(1e-12));
 #pragma unroll
     for (int t = 0; t < 2; t++) {
         const int Gt = t ? G_3 : G_2;
@@ -1088,7 +1171,7 @@ __device__ __forceinline__ T hlld_error(int dir, T ptot, T cmin, T cmax, T BX, c
     const T error = delta_Kx * (T(1.) - f.B_ar[dir] * (Y_r - Y_l));
     const T kbl = f.eta_l - (f.K_al[1] * f.B_c[1] + f.K_al[2] * f.B_c[2] + f.K_al[3] * f.B_c[3]);
     const T kbr = f.eta_r - (f.K_ar[1] * f.B_c[1] + f.K_ar[2] * f.B_c[2] + f.K_ar[3] * f.B_c[3]);
-    const Divisor<T> dkl(kbl), dkr(kbr);
+    const ExactDivisor<T> dkl(kbl), dkr(kbr);
 #pragma unroll
     for (int q = 1; q < 4; q++) {
         f.v_cl[q] = (f.K_al[q] - dkl.div(f.B_c[q] * (T(1.) - kl2)));
@@ -1188,7 +1271,7 @@ template <typename T>
 __device__ __forceinline__ void hlld_outer(int dir, T S, const T *R, T ptot, const T *v, const T *Bs, T BX, T *X) {
     const int G_1 = dir, G_2 = dir % 3 + 1, G_3 = (dir + 1) % 3 + 1;
     const T v_dot_B = v[1] * Bs[1] + v[2] * Bs[2] + v[3] * Bs[3];
-    const Divisor<T> dS(S - v[G_1]);
+    const ExactDivisor<T> dS(S - v[G_1]);
     X[RHO] = dS.div(R[RHO]);
     X[UU] = (R[UU] - ptot * v[G_1] + v_dot_B * Bs[G_1]) / (S - v[G_1] + T(SMALL_D));
     X[UU + G_1] = (-X[UU] + ptot) * v[G_1] - v_dot_B * Bs[G_1];
@@ -1206,7 +1289,7 @@ __device__ __forceinline__ void hlld_inner(int dir, const T *Xa, T Ka, const T *
                                            T BX, T *X) {
     const int G_1 = dir, G_2 = dir % 3 + 1, G_3 = (dir + 1) % 3 + 1;
     const T v_dot_B = vc[1] * Bc[1] + vc[2] * Bc[2] + vc[3] * Bc[3];
-    const Divisor<T> dK(Ka - vc[G_1]);
+    const ExactDivisor<T> dK(Ka - vc[G_1]);
     X[RHO] = dK.div(Xa[RHO] * (Ka - va[G_1]));
     X[UU] = dK.div(-(-Ka * Xa[UU] - Xa[UU + G_1] + ptot * vc[G_1] - v_dot_B * Xa[B1 + G_1 - 1]));
     X[UU + G_1] = (-Xa[UU] + ptot) * vc[G_1] - v_dot_B * Bc[G_1];
