@@ -312,7 +312,7 @@ __device__ __forceinline__ double flux_eval(const Dims &d, const Geo<T> &gm, con
         const T cmax = d_max(d_max(T(0.), xl), xr);
         const T cmin = d_max(d_max(T(0.), -nl), -nr);
         // the HLL weights with sqrt(-g)
-        const T rg = gm.g / (cmax + cmin + T(SMALL_D));
+        const T rg = gm.g * d_rcp(cmax + cmin + T(SMALL_D));
         const T wl = cmax * rg, wr = cmin * rg, wu = cmax * wr;
 #pragma unroll
         for (int k = 0; k < NPR; k++)

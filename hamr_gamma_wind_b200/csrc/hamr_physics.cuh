@@ -21,6 +21,8 @@
 
 #include <type_traits>
 
+#include "hamr_pow.cuh"
+
 namespace hamr {
 
 enum { RHO = 0, UU = 1, U1 = 2, U2 = 3, U3 = 4, B1 = 5, B2 = 6, B3 = 7, KTOT = 8, NPR = 9 };
@@ -61,16 +63,59 @@ struct State {
 };
 
 template <typename T> __device__ __forceinline__ T d_sqrt(T x);
-template <> __device__ __forceinline__ double d_sqrt<double>(double x) { return sqrt(x); }
+template <> __device__ __forceinline__ double d_sqrt<double>(double x);   // below, with the reciprocal
 template <> __device__ __forceinline__ float d_sqrt<float>(float x) { return sqrtf(x); }
 template <typename T> __device__ __forceinline__ T d_pow(T x, T y);
-template <> __device__ __forceinline__ double d_pow<double>(double x, double y) { return pow(x, y); }
+template <> __device__ __forceinline__ double d_pow<double>(double x, double y) { return STRICT ? pow(x, y) : pow_tab(x, y); }
 // float (the mixed step's entropy K = P rho^-gam of the face states, which
 // only the entropy flux carries): the fast exp2(y log2 x) intrinsic, relative
 // error a few 1e-6 at the atmosphere's densities against powf's ulp; measured
 // on the 384 x 192 x 192 torus: the three float flux kernels 6.05 -> 5.59 ms
 // per step, L1 of every field against FP64 after 1000 steps unchanged
 template <> __device__ __forceinline__ float d_pow<float>(float x, float y) { return __powf(x, y); }
+
+// Reciprocal and square root of the production build, by Newton's iteration
+// (Goldschmidt's form for the root) from the hardware's approximations, which
+// are good to about 2^-20: the reciprocal's one third-order step,
+// r (1 + e + e^2) with e = 1 - b r, leaves e^3; the root's second-order step and
+// final residual leave 2^-80; each then rounds within 0.6 ulp
+// (tests/test_gpu_reciprocal.py). A zero, infinite or NaN operand, where the
+// residuals are NaN, keeps the approximation's own exact answer. Three and
+// seven FP64 operations without a branch: the step takes eleven of them per
+// face and four per Newton iteration of the inversion, in dependent chains.
+__device__ __forceinline__ bool not_finite(double x) { return (__double2hiint(x) & 0x7ff00000) == 0x7ff00000; }
+__device__ __forceinline__ double rcp_nr(double b) {
+    double r0;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r0) : "d"(b));
+    const double e = fma(-b, r0, 1.0);
+    const double r = fma(r0, fma(e, e, e), r0);
+    return not_finite(r) ? r0 : r;
+}
+// sqrt(x) and 1/sqrt(x) of a positive normal x
+__device__ __forceinline__ double sqrt_nr_pos(double x, double &rs) {
+    double r0;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(r0) : "d"(x));
+    const double g = x * r0, h = 0.5 * r0;
+    const double e = fma(-g, h, 0.5);
+    const double g1 = fma(g, e, g), h1 = fma(h, e, h);
+    const double s = fma(fma(-g1, g1, x), h1, g1);
+    const double r1 = 2.0 * h1;
+    rs = fma(r1, fma(-s, r1, 1.0), r1);   // not evaluated where it is not used
+    return s;
+}
+__device__ __noinline__ double sqrt_rest(double x) { return sqrt(x); }
+__device__ __forceinline__ bool pos_normal(double x) { return (unsigned)__double2hiint(x) - 0x00100000u < 0x7fe00000u; }
+__device__ __forceinline__ double sqrt_nr(double x) {
+    double rs;
+    return pos_normal(x) ? sqrt_nr_pos(x, rs) : sqrt_rest(x);
+}
+template <> __device__ __forceinline__ double d_sqrt<double>(double x) { return STRICT ? sqrt(x) : sqrt_nr(x); }
+// 1 / x in the arithmetic of the build
+template <typename T> __device__ __forceinline__ T d_rcp(T x) {
+    if constexpr (std::is_same<T, double>::value && !STRICT) return rcp_nr(x);
+    else return T(1.0) / x;
+}
+
 template <typename T> __device__ __forceinline__ T d_fabs(T x) { return x < T(0) ? -x : x; }
 __device__ __forceinline__ double d_fabs(double x) { return fabs(x); }   // an operand modifier, not a comparison
 __device__ __forceinline__ float d_fabs(float x) { return fabsf(x); }
@@ -108,6 +153,7 @@ template <> __device__ __forceinline__ float d_rsqrt<float>(float x) { return po
 __device__ __forceinline__ double div_rcp(double a, double b, double rb) {
     const double q0 = a * rb;
     const double r = fma(-q0, b, a);
+    if constexpr (!STRICT) return fma(r, rb, q0);   // but for the sign of a zero the same
     return r == 0.0 ? q0 : fma(r, rb, q0);
 }
 
@@ -117,6 +163,7 @@ __device__ __forceinline__ double div_rcp(double a, double b, double rb) {
 __device__ __forceinline__ double div_rcp_inf(double a, double b, double rb) {
     const double q0 = a * rb;
     const double r = fma(-q0, b, a);
+    if constexpr (!STRICT) return not_finite(r) ? q0 : fma(r, rb, q0);
     return (r == 0.0 || !(fabs(r) <= 1.7976931348623157e308)) ? q0 : fma(r, rb, q0);
 }
 
@@ -135,7 +182,7 @@ template <typename T>
 struct Divisor {
     T b, rb;
     __device__ __forceinline__ explicit Divisor(T b_) : b(b_), rb(b_) {
-        if constexpr (std::is_floating_point<T>::value) rb = T(1.0) / b_;
+        if constexpr (std::is_floating_point<T>::value) rb = d_rcp(b_);
     }
     // with the divisor's reciprocal already at hand (rounded once, 1/b)
     __device__ __forceinline__ Divisor(T b_, T rb_) : b(b_), rb(rb_) {}
@@ -334,7 +381,7 @@ __device__ __forceinline__ void hll_side(T gam, const T *pr, const Geo<T> &gm, T
             F[B1 + j - 1] = b[j] * u[DIR] - b[DIR] * u[j];
             U[B1 + j - 1] = pr[B1 + j - 1];
         }
-    T c2 = (gP + bsq) / eta;
+    T c2 = (gP + bsq) * d_rcp(eta);
     if (c2 < T(0.)) c2 = T(SMALL_D);
     if (c2 > T(1.)) c2 = T(1.);
     constexpr int sdd = DIR == 1 ? 4 : (DIR == 2 ? 7 : 9);
@@ -345,7 +392,7 @@ __device__ __forceinline__ void hll_side(T gam, const T *pr, const Geo<T> &gm, T
     T disc = B * B - A * C;
     if (disc < T(0.)) disc = T(0.);
     disc = d_sqrt(disc);
-    const T rA = T(1.) / A;
+    const T rA = d_rcp(A);
     const T vp = (B - disc) * rA, vm = (B + disc) * rA;
     vmax = d_max(vp, vm);
     vmin = d_min(vp, vm);
@@ -502,9 +549,10 @@ __device__ __forceinline__ int guess_utsq(const double *gcov, const double *prim
 
 __device__ __forceinline__ void set_velocity(const InvQ &s, double gamma, double W, double *prim) {
     const Divisor<double> dw(W);   // the three quotients by W
+    const double gw = STRICT ? gamma / (W + s.Bsq) : gamma * d_rcp(W + s.Bsq);
     for (int i = 1; i < 4; i++) {
         double Qtcon = s.Qcon[i] + s.ncon[i] * s.Qdotn;
-        prim[U1 + i - 1] = gamma / (W + s.Bsq) * (Qtcon + dw.div(s.QdotB * s.Bcon[i]));
+        prim[U1 + i - 1] = gw * (Qtcon + dw.div(s.QdotB * s.Bcon[i]));
     }
 }
 
@@ -533,7 +581,8 @@ __device__ __forceinline__ int inv_prologue(const double *U, double gdet, const 
 __device__ __forceinline__ double vsq_of_W(double W, double Bsq, double Qtsq, double QdotBsq) {
     double Wsq = W * W;
     double Xsq = (Bsq + W) * (Bsq + W);
-    return (Wsq * Qtsq + QdotBsq * (Bsq + 2. * W)) / (Wsq * Xsq);
+    const double num = Wsq * Qtsq + QdotBsq * (Bsq + 2. * W);
+    return STRICT ? num / (Wsq * Xsq) : num * d_rcp(Wsq * Xsq);
 }
 
 // Noble et al. 2006, 2D Newton-Raphson on (W, v^2). The divisions by gamma
@@ -553,8 +602,8 @@ __device__ __forceinline__ int utoprim_2d_k(const InvK &k, const double *U, cons
     double utsq;
     if (guess_utsq(gcov, pt, &utsq)) return 2;
     double gammasq = 1. + utsq;
-    double gamma = sqrt(gammasq);
-    double rho0 = s.D / gamma;
+    double gamma = d_sqrt(gammasq);
+    double rho0 = STRICT ? s.D / gamma : s.D * d_rcp(gamma);
     double u = pt[UU];
     double p = (gam - 1.) * u;
     double w = rho0 + u + p;
@@ -573,29 +622,55 @@ __device__ __forceinline__ int utoprim_2d_k(const InvK &k, const double *U, cons
     const double Bsq = s.Bsq, Qtsq = s.Qtsq, QdotBsq = s.QdotBsq, Qdotn = s.Qdotn, D = s.D;
     // 1/x0 of the current iterate: t23 of this iteration, and the divisor of
     // the previous iteration's errx (the same x0), one reciprocal for both
-    double rx0 = 1. / x0;
+    double rx0 = d_rcp(x0);
     while (keep) {
-        double Wsq = x0 * x0;
-        double gtmp = 1. - x1;
-        double p_tmp = div_rcp_inf((gam - 1.) * (fma(x0, gtmp, -D * sqrt(gtmp))), gam, rgam);
-        double dPdW = div_rcp_inf((gam - 1.) * (1. - x1), gam, rgam);
-        double dPdvsq = div_rcp_inf((gam - 1.) * (fma(0.5, D / sqrt(1. - x1), -x0)), gam, rgam);
-        double t2 = -0.5 * Bsq + dPdvsq;
-        double t3 = Bsq + x0;
-        double t4 = t3 * t3;
-        double t9 = 1. / Wsq;
-        double t11 = Qtsq - x1 * t4 + QdotBsq * (Bsq + 2.0 * x0) * t9;
-        double t16 = QdotBsq * t9;
-        double t18 = -Qdotn - 0.5 * Bsq * (1.0 + x1) + 0.5 * t16 - x0 + p_tmp;
-        double t21 = 1. / t3;
-        double t23 = rx0;
-        double t24 = t16 * t23;
-        double t25 = -1.0 + dPdW - t24;
-        double t35 = t25 * t3 + (Bsq - 2.0 * dPdvsq) * (QdotBsq + x1 * Wsq * x0) * t9 * t23;
-        double t36 = 1. / t35;
-        double dx0 = -(t2 * t11 + t4 * t18) * t21 * t36;
-        double t40 = (x1 + t24) * t3;
-        double dx1 = -(-t25 * t11 - 2.0 * t40 * t18) * t21 * t36;
+        double t11, t18, dx0, dx1;
+        if constexpr (STRICT) {
+            double Wsq = x0 * x0;
+            double gtmp = 1. - x1;
+            double p_tmp = div_rcp_inf((gam - 1.) * (fma(x0, gtmp, -D * sqrt(gtmp))), gam, rgam);
+            double dPdW = div_rcp_inf((gam - 1.) * (1. - x1), gam, rgam);
+            double dPdvsq = div_rcp_inf((gam - 1.) * (fma(0.5, D / sqrt(1. - x1), -x0)), gam, rgam);
+            double t2 = -0.5 * Bsq + dPdvsq;
+            double t3 = Bsq + x0;
+            double t4 = t3 * t3;
+            double t9 = 1. / Wsq;
+            t11 = Qtsq - x1 * t4 + QdotBsq * (Bsq + 2.0 * x0) * t9;
+            double t16 = QdotBsq * t9;
+            t18 = -Qdotn - 0.5 * Bsq * (1.0 + x1) + 0.5 * t16 - x0 + p_tmp;
+            double t21 = 1. / t3;
+            double t23 = rx0;
+            double t24 = t16 * t23;
+            double t25 = -1.0 + dPdW - t24;
+            double t35 = t25 * t3 + (Bsq - 2.0 * dPdvsq) * (QdotBsq + x1 * Wsq * x0) * t9 * t23;
+            double t36 = 1. / t35;
+            dx0 = -(t2 * t11 + t4 * t18) * t21 * t36;
+            double t40 = (x1 + t24) * t3;
+            dx1 = -(-t25 * t11 - 2.0 * t40 * t18) * t21 * t36;
+        } else {
+            // the same residuals and Jacobian with x0^-2 = (1/x0)^2,
+            // (QdotBsq + x1 x0^3) / x0^3 = t24 + x1, the two divisions of each
+            // increment as one, and the root of 1 - x1 with its reciprocal
+            const double gtmp = 1. - x1;
+            double rs;
+            const double sg = sqrt_nr_pos(gtmp, rs);   // 1e-15 <= gtmp <= 1
+            const double kg = (gam - 1.) * rgam;
+            const double p_tmp = kg * fma(x0, gtmp, -D * sg);
+            const double dPdvsq = kg * fma(0.5 * D, rs, -x0);
+            const double t2 = fma(-0.5, Bsq, dPdvsq);
+            const double t3 = Bsq + x0;
+            const double t4 = t3 * t3;
+            const double t16 = QdotBsq * (rx0 * rx0);
+            const double t24 = t16 * rx0;
+            const double t40 = x1 + t24;
+            t11 = fma(t16, fma(2.0, x0, Bsq), fma(-x1, t4, Qtsq));
+            t18 = -Qdotn - 0.5 * Bsq * (1.0 + x1) + 0.5 * t16 - x0 + p_tmp;
+            const double t25 = fma(kg, gtmp, -1.0) - t24;
+            const double t35 = fma(t25, t3, fma(-2.0, dPdvsq, Bsq) * t40);
+            const double r = d_rcp(t3 * t35);
+            dx0 = -fma(t2, t11, t4 * t18) * r;
+            dx1 = fma(t25, t11, 2.0 * (t40 * t3) * t18) * r;
+        }
         df = -t11 * t11 - t18 * t18;
         f = -0.5 * df;
         double xo0 = x0;
@@ -605,7 +680,7 @@ __device__ __forceinline__ int utoprim_2d_k(const InvK &k, const double *U, cons
         x0 = (x0 > W_TOO_BIG) ? xo0 : x0;
         x1 = (x1 < 0.) ? 0. : x1;
         x1 = (x1 > 1.) ? (1. - 1.e-15) : x1;
-        rx0 = 1. / x0;
+        rx0 = d_rcp(x0);
         errx = (x0 == 0.) ? fabs(x0 - xo0) : fabs(div_rcp_inf(x0 - xo0, x0, rx0));
         if ((fabs(errx) <= NEWT_TOL) && (doing_extra == 0) && (EXTRA_NEWT_ITER > 0)) doing_extra = 1;
         if (doing_extra == 1) i_extra++;
@@ -620,8 +695,8 @@ __device__ __forceinline__ int utoprim_2d_k(const InvK &k, const double *U, cons
     if ((retval != 0) || (W == FAIL_VAL)) return retval * 100 + 1;
     if (W <= 0. || W > W_TOO_BIG) return 3;
     if (vsq >= 1.) return 4;
-    double gtmp = sqrt(1. - vsq);
-    gamma = 1. / gtmp;
+    double gtmp = d_sqrt(1. - vsq);
+    gamma = d_rcp(gtmp);
     rho0 = s.D * gtmp;
     w = W * (1. - vsq);
     p = div_rcp_inf((gam - 1.) * (w - rho0), gam, rgam);
@@ -643,7 +718,7 @@ __device__ __forceinline__ int utoprim_2d(double gam, const double *U, const dou
 __device__ __forceinline__ double W_of_vsq2(double gam, double vsq, double *p, double *rho, double *u, double D, double K) {
     double gtmp = (1. - vsq);
     *rho = D * sqrt(gtmp);
-    *p = K * pow(*rho, gam);
+    *p = K * d_pow(*rho, gam);
     *u = *p / (gam - 1.);
     return (*rho + *u + *p) / gtmp;
 }
