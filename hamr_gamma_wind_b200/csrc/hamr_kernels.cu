@@ -814,69 +814,52 @@ __global__ void __launch_bounds__(BLK) k_emf_centre(const Dims d, const Geom m, 
     k_emf_centre_at(d, m, pv, Ec, t);
 }
 
-template <typename T> __device__ __forceinline__ T up(T f) { return (T)(f <= T(0.0)); }
-template <typename T> __device__ __forceinline__ T dn(T f) { return (T)(f > T(0.0)); }
-
 // edge EMFs: average of the four face EMFs plus, when ct_upwind, the
 // centre-minus-face corrections from the upwind side of each face, chosen by
 // the sign of its mass flux (consttransport2, GPU_const_trans.h:121-338), for
 // the edge at cell index c (row j): ec(k, di, dj, dz) is centre EMF k (1..3)
 // of the zone offset by (di, dj, dz) in {-1, 0}^3 from the edge's cell
-// (times the direction flags d1..d3); e[0..2] = E1, E2, E3
+// (times the direction flags d1..d3); e[0..2] = E1, E2, E3.
+// The reference forms both sides' corrections and weighs them by 0 and 1; here
+// the mass flux's sign picks the operands and one difference is formed: the
+// same value for finite operands, in a third of the operations and few enough
+// registers for eight blocks per SM (the loads' latency is what bounds it).
 template <typename T, class EC>
 __device__ __forceinline__ void emf_edge_eval(const Dims &d, EC ec, const T *__restrict__ F1,
                                               const T *__restrict__ F2, const T *__restrict__ F3, long c, int j,
                                               T *e) {
     const long ks = d.ks, jsize = d.G3, isize = (long)d.G2 * d.G3;
-    const long D1 = d.d1, D2 = d.d2, D3 = d.d3;
-    const T *F1r = F1 + RHO * ks, *F2r = F2 + RHO * ks, *F3r = F3 + RHO * ks;
+    const long D1 = d.d1 * isize, D2 = d.d2 * jsize, D3 = d.d3;
     const bool w = d.ct_upwind != 0;
-    // in the non-upwind build every correction is an exact 0.0
-#define CORR(expr) (w ? (expr) : T(0.0))
-    const T dE_LEFT_13_1 = CORR(ec(1, 0, 0, 0) - F3[B2 * ks + c]);
-    const T dE_LEFT_13_2 = CORR(ec(1, 0, -1, 0) - F3[B2 * ks + c - jsize * D2]);
-    const T dE_RIGHT_13_1 = CORR(F3[B2 * ks + c] - ec(1, 0, 0, -1));
-    const T dE_RIGHT_13_2 = CORR(F3[B2 * ks + c - jsize * D2] - ec(1, 0, -1, -1));
-    const T dE_LEFT_12_1 = CORR(ec(1, 0, 0, 0) + F2[B3 * ks + c]);
-    const T dE_LEFT_12_2 = CORR(ec(1, 0, 0, -1) + F2[B3 * ks + c - D3]);
-    const T dE_RIGHT_12_1 = CORR(-F2[B3 * ks + c] - ec(1, 0, -1, 0));
-    const T dE_RIGHT_12_2 = CORR(-F2[B3 * ks + c - D3] - ec(1, 0, -1, -1));
-    const T dE_LEFT_21_1 = CORR(ec(2, 0, 0, 0) - F1[B3 * ks + c]);
-    const T dE_LEFT_21_2 = CORR(ec(2, 0, 0, -1) - F1[B3 * ks + c - D3]);
-    const T dE_RIGHT_21_1 = CORR(F1[B3 * ks + c] - ec(2, -1, 0, 0));
-    const T dE_RIGHT_21_2 = CORR(F1[B3 * ks + c - D3] - ec(2, -1, 0, -1));
-    const T dE_LEFT_23_1 = CORR(ec(2, 0, 0, 0) + F3[B1 * ks + c]);
-    const T dE_LEFT_23_2 = CORR(ec(2, -1, 0, 0) + F3[B1 * ks + c - D1 * isize]);
-    const T dE_RIGHT_23_1 = CORR(-F3[B1 * ks + c] - ec(2, 0, 0, -1));
-    const T dE_RIGHT_23_2 = CORR(-F3[B1 * ks + c - isize * D1] - ec(2, -1, 0, -1));
-    const T dE_LEFT_31_1 = CORR(ec(3, 0, 0, 0) + F1[B2 * ks + c]);
-    const T dE_LEFT_31_2 = CORR(ec(3, 0, -1, 0) + F1[B2 * ks + c - D2 * jsize]);
-    const T dE_RIGHT_31_1 = CORR(-F1[B2 * ks + c] - ec(3, -1, 0, 0));
-    const T dE_RIGHT_31_2 = CORR(-F1[B2 * ks + c - D2 * jsize] - ec(3, -1, -1, 0));
-    const T dE_LEFT_32_1 = CORR(ec(3, 0, 0, 0) - F2[B1 * ks + c]);
-    const T dE_LEFT_32_2 = CORR(ec(3, -1, 0, 0) - F2[B1 * ks + c - D1 * isize]);
-    const T dE_RIGHT_32_1 = CORR(F2[B1 * ks + c] - ec(3, 0, -1, 0));
-    const T dE_RIGHT_32_2 = CORR(F2[B1 * ks + c - D1 * isize] - ec(3, -1, -1, 0));
-#undef CORR
-    T e1 = T(0.25) * ((-F2[B3 * ks + c] - (dE_LEFT_13_1 * up(F2r[c]) + dE_LEFT_13_2 * dn(F2r[c])))
-        + (-F2[B3 * ks + c - D3] + (dE_RIGHT_13_1 * up(F2r[c - D3]) + dE_RIGHT_13_2 * dn(F2r[c - D3]))) +
-        +(F3[B2 * ks + c] - (dE_LEFT_12_1 * up(F3r[c]) + dE_LEFT_12_2 * dn(F3r[c])))
-        + (F3[B2 * ks + c - D2 * jsize] + (dE_RIGHT_12_1 * up(F3r[c - D2 * jsize]) + dE_RIGHT_12_2 * dn(F3r[c - D2 * jsize]))));
-    const T e2 = T(0.25) * ((-F3[B1 * ks + c] - (dE_LEFT_21_1 * up(F3r[c]) + dE_LEFT_21_2 * dn(F3r[c])))
-        + (-F3[B1 * ks + c - D1 * isize] + (dE_RIGHT_21_1 * up(F3r[c - D1 * isize]) + dE_RIGHT_21_2 * dn(F3r[c - D1 * isize])))
-        + (F1[B3 * ks + c] - (dE_LEFT_23_1 * up(F1r[c]) + dE_LEFT_23_2 * dn(F1r[c])))
-        + (F1[B3 * ks + c - D3] + (dE_RIGHT_23_1 * up(F1r[c - D3]) + dE_RIGHT_23_2 * dn(F1r[c - D3]))));
-    T e3 = T(0.25) * ((F2[B1 * ks + c] - (dE_LEFT_31_1 * up(F2r[c]) + dE_LEFT_31_2 * dn(F2r[c])))
-        + (F2[B1 * ks + c - D1 * isize] + (dE_RIGHT_31_1 * up(F2r[c - D1 * isize]) + dE_RIGHT_31_2 * dn(F2r[c - D1 * isize])))
-        + (-F1[B2 * ks + c] - (dE_LEFT_32_1 * up(F1r[c]) + dE_LEFT_32_2 * dn(F1r[c])))
-        + (-F1[B2 * ks + c - D2 * jsize] + (dE_RIGHT_32_1 * up(F1r[c - D2 * jsize]) + dE_RIGHT_32_2 * dn(F1r[c - D2 * jsize]))));
+    // the correction x - y of a face from its upwind side (mass flux m): the
+    // first pair for m <= 0, else the second; zero without upwinding
+    auto corr = [&](T m, T x1, T y1, T x2, T y2) {
+        const bool up = m <= T(0.0);
+        return w ? (up ? x1 : x2) - (up ? y1 : y2) : T(0.0);
+    };
+    // E_k from the faces of the two other directions a and b (cyclic): pa, pb
+    // the face EMFs and ma, mb the mass fluxes, _s at the cell below along the
+    // other face's direction; c0 the centre EMF at the edge's cell, ca, cb, cab below
+    // it along a, along b and along both
+    auto edge = [&](T pa, T pas, T pb, T pbs, T ma, T mas, T mb, T mbs, T c0, T ca, T cb, T cab) {
+        return T(0.25) * ((pa - corr(ma, c0, pb, ca, pbs)) + (pas + corr(mas, pb, cb, pbs, cab)) +
+                          (pb - corr(mb, c0, pa, cb, pas)) + (pbs + corr(mbs, pa, ca, pas, cab)));
+    };
+    const T *F1r = F1 + RHO * ks + c, *F2r = F2 + RHO * ks + c, *F3r = F3 + RHO * ks + c;
+    const T f23 = F2[B3 * ks + c], f23s = F2[B3 * ks + c - D3], f32 = F3[B2 * ks + c], f32s = F3[B2 * ks + c - D2];
+    e[0] = edge(-f23, -f23s, f32, f32s, F2r[0], F2r[-D3], F3r[0], F3r[-D2], ec(1, 0, 0, 0), ec(1, 0, -1, 0),
+                ec(1, 0, 0, -1), ec(1, 0, -1, -1));
+    const T f31 = F3[B1 * ks + c], f31s = F3[B1 * ks + c - D1], f13 = F1[B3 * ks + c], f13s = F1[B3 * ks + c - D3];
+    e[1] = edge(-f31, -f31s, f13, f13s, F3r[0], F3r[-D1], F1r[0], F1r[-D3], ec(2, 0, 0, 0), ec(2, 0, 0, -1),
+                ec(2, -1, 0, 0), ec(2, -1, 0, -1));
+    const T f12 = F1[B2 * ks + c], f12s = F1[B2 * ks + c - D2], f21 = F2[B1 * ks + c], f21s = F2[B1 * ks + c - D1];
+    // (a = x2, b = x1 up to the sign of both: the reference's order of the sum)
+    e[2] = edge(f21, f21s, -f12, -f12s, F2r[0], F2r[-D1], F1r[0], F1r[-D2], ec(3, 0, 0, 0), ec(3, 0, -1, 0),
+                ec(3, -1, 0, 0), ec(3, -1, -1, 0));
     if ((d.pole1 && j == d.ng2) || (d.pole2 && j == d.n2 + d.ng2)) {
-        e3 = T(0.);
-        e1 = T(-0.5) * (F2[B3 * ks + c] + F2[B3 * ks + c - D3]);
+        e[2] = T(0.);
+        e[0] = T(-0.5) * (f23 + f23s);
     }
-    e[0] = e1;
-    e[1] = e2;
-    e[2] = e3;
 }
 
 template <typename T>
@@ -902,8 +885,11 @@ __device__ __forceinline__ void k_emf_edge_at(const Dims &d, const T *__restrict
 
 // (two z edges per thread, as k_face_update takes two face triples, measured
 // slower: 0.58 -> 0.63 ms per mixed 384 x 192 x 192 step, 1.03 -> 1.07 FP64)
+#ifndef HAMR_EMF_EDGE_MINB
+#define HAMR_EMF_EDGE_MINB 8
+#endif
 template <typename T>
-__global__ void __launch_bounds__(BLK) k_emf_edge(const Dims d, const T *__restrict__ Ec,
+__global__ void __launch_bounds__(BLK, HAMR_EMF_EDGE_MINB) k_emf_edge(const Dims d, const T *__restrict__ Ec,
                                                    const T *__restrict__ F1, const T *__restrict__ F2,
                                                    const T *__restrict__ F3, T *__restrict__ emf) {
     const int ni = d.n1 + d.d1, nj = d.n2 + d.d2, nz = d.n3 + d.d3;
