@@ -230,13 +230,16 @@ __device__ __forceinline__ double dt_of_ctop(const Dims &d, int dir, double cmax
 
 template <int DIR, typename T, int REC>
 __device__ __forceinline__ double flux_eval(const Dims &d, const Geo<T> &gm, const double *__restrict__ ps, T *pl,
-                                            T *pr, T *__restrict__ F, const long c, const int j);
+                                            T *pr, T *__restrict__ F, const long c, const int j, int drop = -1);
 
 // one face of direction DIR (t < n_faces): reconstruction, two states, four
 // flux evaluations, HLL (or HLLC); returns the face's signal-speed
 // contribution to the CFL limit (ctop_term). REC: bit 0 MC reconstruction,
-// bit 1 HLLC.
-template <int DIR, typename T, int REC>
+// bit 1 HLLC. FIX (2-D blocks with a reflective axis): the faces' part of
+// fix_flux with it -- the x1 flux of B2 mirrored into the row beyond the axis
+// by the face next to it (the row's own faces leave it out), no x2 flux through
+// the axis, no inflow through the radial edges.
+template <int DIR, typename T, int REC, bool FIX = false>
 __device__ __forceinline__ double flux_face(const Dims &d, const Geom &m, const double *__restrict__ pv,
                                             const double *__restrict__ ps, T *__restrict__ F, const long t) {
     constexpr int idel = DIR == 1, jdel = DIR == 2, zdel = DIR == 3;
@@ -273,17 +276,33 @@ __device__ __forceinline__ double flux_face(const Dims &d, const Geom &m, const 
             para_face(x, pl[k], pr[k]);   // upper edge of zone c-1, lower edge of zone c
         }
     }
-    return flux_eval<DIR, T, REC>(d, gm, ps, pl, pr, F, c, j);
+    if constexpr (!FIX) {
+        return flux_eval<DIR, T, REC>(d, gm, ps, pl, pr, F, c, j);
+    } else {
+        const long ks = d.ks;
+        const int ja = d.ng2, jb = d.n2 + d.ng2;   // the active rows are [ja, jb)
+        const bool beyond = (d.pole1 && j == ja - 1) || (d.pole2 && j == jb);
+        const double cmx = flux_eval<DIR, T, REC>(d, gm, ps, pl, pr, F, c, j, DIR == 1 && beyond ? (int)B2 : -1);
+        if constexpr (DIR == 1) {
+            if (d.pole1 && j == ja) F[B2 * ks + c - 1] = -F[B2 * ks + c];
+            if (d.pole2 && j == jb - 1) F[B2 * ks + c + 1] = -F[B2 * ks + c];
+            if (!(d.halo & 1) && i == d.ng1 && F[RHO * ks + c] > T(0.)) F[RHO * ks + c] = T(0.);
+            if (!(d.halo & 2) && i == d.n1 + d.ng1 && F[RHO * ks + c] < T(0.)) F[RHO * ks + c] = T(0.);
+        } else if ((d.pole1 && j == ja) || (d.pole2 && j == jb)) {
+            for (int k = 0; k < NPR; k++) F[k * ks + c] = T(0.);
+        }
+        return cmx;
+    }
 }
 
 // The face flux from the reconstructed states pl, pr (the normal field and
 // the polar B1 fix applied here): two states, four flux evaluations, HLL (or
 // HLLC), the flux written at cell index c, all but the normal field's, which
-// is zero and which nothing reads; returns the face's signal-speed
-// contribution to the CFL limit (ctop_term).
+// is zero and which nothing reads, and component `drop`; returns the face's
+// signal-speed contribution to the CFL limit (ctop_term).
 template <int DIR, typename T, int REC>
 __device__ __forceinline__ double flux_eval(const Dims &d, const Geo<T> &gm, const double *__restrict__ ps, T *pl,
-                                            T *pr, T *__restrict__ F, const long c, const int j) {
+                                            T *pr, T *__restrict__ F, const long c, const int j, int drop) {
     double dtf = 1.e9;
     const T bn = (T)__ldg(&ps[(long)(DIR - 1) * d.ks + c]);
     pl[B1 + DIR - 1] = bn;
@@ -300,7 +319,7 @@ __device__ __forceinline__ double flux_eval(const Dims &d, const Geo<T> &gm, con
         const T ctop = hllc_face<DIR, T, (REC & 4) != 0>(gam, pl, pr, gm, Fo);
 #pragma unroll
         for (int k = 0; k < NPR; k++)
-            if (k != B1 + DIR - 1) F[(long)k * d.ks + c] = Fo[k];
+            if (k != B1 + DIR - 1 && k != drop) F[(long)k * d.ks + c] = Fo[k];
         (void)dxd;
         (void)dtf;
         return ctop_term(d, DIR, (double)ctop);
@@ -316,7 +335,7 @@ __device__ __forceinline__ double flux_eval(const Dims &d, const Geo<T> &gm, con
         const T wl = cmax * rg, wr = cmin * rg, wu = cmax * wr;
 #pragma unroll
         for (int k = 0; k < NPR; k++)
-            if (k != B1 + DIR - 1) F[(long)k * d.ks + c] = wl * Fl[k] + wr * Fr[k] - wu * (Ur[k] - Ul[k]);
+            if (k != B1 + DIR - 1 && k != drop) F[(long)k * d.ks + c] = wl * Fl[k] + wr * Fr[k] - wu * (Ur[k] - Ul[k]);
         return ctop_term(d, DIR, (double)d_max(cmax, cmin));
     }
     State<T> q;
@@ -336,7 +355,7 @@ __device__ __forceinline__ double flux_eval(const Dims &d, const Geo<T> &gm, con
     const Divisor<T> dh(cmax + cmin + T(SMALL_D));   // the nine HLL quotients share it
 #pragma unroll
     for (int k = 0; k < NPR; k++)
-        if (k != B1 + DIR - 1)
+        if (k != B1 + DIR - 1 && k != drop)
             F[(long)k * d.ks + c] = dh.div(cmax * t1[k] + cmin * t3[k] - cmax * cmin * (t4[k] - t2[k]));
     (void)dxd;
     (void)dtf;
@@ -814,6 +833,35 @@ __global__ void __launch_bounds__(BLK) k_emf_centre(const Dims d, const Geom m, 
     k_emf_centre_at(d, m, pv, Ec, t);
 }
 
+// The fluxes of both directions, the polar and radial flux rules and the centre
+// EMFs of a 2-D block in one launch: CTAs [0, nb1) the x1 faces, [nb1, nb2) the
+// x2 faces, the rest the zones. Each alone is a wave or less of the device and
+// bound by the latency of one face's chain; together the chains overlap: 256 x
+// 256 torus, per step, 0.108 -> 0.049 ms (four blocks per SM; 3: 0.052, 5:
+// 0.055). Same values as k_flux, k_fix_flux and k_emf_centre.
+#ifndef HAMR_FLUX_2D_MINB
+#define HAMR_FLUX_2D_MINB 4
+#endif
+template <typename T, int REC, bool FIX>
+__global__ void __launch_bounds__(BLK, HAMR_FLUX_2D_MINB)
+    k_flux_2d(const Dims d, const Geom m, const double *__restrict__ pv, const double *__restrict__ ps,
+              T *__restrict__ F1, T *__restrict__ F2, T *__restrict__ Ec, unsigned long long *__restrict__ dtbits,
+              int calc_dt, int nb1, int nb2) {
+    const int b = blockIdx.x;
+    if (b < nb1) {
+        const long t = (long)b * BLK + threadIdx.x;
+        const double cmx = t < n_faces<1>(d) ? flux_face<1, T, REC, FIX>(d, m, pv, ps, F1, t) : 0.0;
+        if (calc_dt) cta_max_ctop(d, 1, cmx, &dtbits[1]);
+    } else if (b < nb2) {
+        const long t = (long)(b - nb1) * BLK + threadIdx.x;
+        const double cmx = t < n_faces<2>(d) ? flux_face<2, T, REC, FIX>(d, m, pv, ps, F2, t) : 0.0;
+        if (calc_dt) cta_max_ctop(d, 2, cmx, &dtbits[2]);
+    } else {
+        const long t = (long)(b - nb2) * BLK + threadIdx.x;
+        if (t < (long)(d.n1 + 2 * d.d1) * (d.n2 + 2 * d.d2)) k_emf_centre_at(d, m, pv, Ec, t);
+    }
+}
+
 // edge EMFs: average of the four face EMFs plus, when ct_upwind, the
 // centre-minus-face corrections from the upwind side of each face, chosen by
 // the sign of its mass flux (consttransport2, GPU_const_trans.h:121-338), for
@@ -824,6 +872,36 @@ __global__ void __launch_bounds__(BLK) k_emf_centre(const Dims d, const Geom m, 
 // the mass flux's sign picks the operands and one difference is formed: the
 // same value for finite operands, in a third of the operations and few enough
 // registers for eight blocks per SM (the loads' latency is what bounds it).
+//
+// edge_emf: E_k from the faces of the two other directions a and b: pa, pb the
+// face EMFs and ma, mb the mass fluxes, _s at the cell below along the other
+// face's direction; c0 the centre EMF of the edge's cell, ca, cb, cab of the
+// cells below it along a, along b and along both.
+template <typename T>
+__device__ __forceinline__ T edge_emf(bool upwind, T pa, T pas, T pb, T pbs, T ma, T mas, T mb, T mbs, T c0, T ca, T cb,
+                                      T cab) {
+    // the correction x - y of a face from its upwind side (mass flux m): the
+    // first pair for m <= 0, else the second; zero without upwinding
+    auto corr = [&](T m, T x1, T y1, T x2, T y2) {
+        const bool up = m <= T(0.0);
+        return upwind ? (up ? x1 : x2) - (up ? y1 : y2) : T(0.0);
+    };
+    return T(0.25) * ((pa - corr(ma, c0, pb, ca, pbs)) + (pas + corr(mas, pb, cb, pbs, cab)) +
+                      (pb - corr(mb, c0, pa, cb, pas)) + (pbs + corr(mbs, pa, ca, pas, cab)));
+}
+
+// E3: from the x2 and x1 faces (the reference's order of the sum)
+template <typename T, class EC>
+__device__ __forceinline__ T emf_edge3(const Dims &d, EC ec, const T *__restrict__ F1, const T *__restrict__ F2, long c,
+                                       int j) {
+    if ((d.pole1 && j == d.ng2) || (d.pole2 && j == d.n2 + d.ng2)) return T(0.);
+    const long ks = d.ks, D1 = d.d1 * (long)d.G2 * d.G3, D2 = d.d2 * (long)d.G3;
+    const T *F1r = F1 + RHO * ks + c, *F2r = F2 + RHO * ks + c;
+    return edge_emf<T>(d.ct_upwind != 0, F2[B1 * ks + c], F2[B1 * ks + c - D1], -F1[B2 * ks + c], -F1[B2 * ks + c - D2],
+                       F2r[0], F2r[-D1], F1r[0], F1r[-D2], ec(3, 0, 0, 0), ec(3, 0, -1, 0), ec(3, -1, 0, 0),
+                       ec(3, -1, -1, 0));
+}
+
 template <typename T, class EC>
 __device__ __forceinline__ void emf_edge_eval(const Dims &d, EC ec, const T *__restrict__ F1,
                                               const T *__restrict__ F2, const T *__restrict__ F3, long c, int j,
@@ -831,35 +909,15 @@ __device__ __forceinline__ void emf_edge_eval(const Dims &d, EC ec, const T *__r
     const long ks = d.ks, jsize = d.G3, isize = (long)d.G2 * d.G3;
     const long D1 = d.d1 * isize, D2 = d.d2 * jsize, D3 = d.d3;
     const bool w = d.ct_upwind != 0;
-    // the correction x - y of a face from its upwind side (mass flux m): the
-    // first pair for m <= 0, else the second; zero without upwinding
-    auto corr = [&](T m, T x1, T y1, T x2, T y2) {
-        const bool up = m <= T(0.0);
-        return w ? (up ? x1 : x2) - (up ? y1 : y2) : T(0.0);
-    };
-    // E_k from the faces of the two other directions a and b (cyclic): pa, pb
-    // the face EMFs and ma, mb the mass fluxes, _s at the cell below along the
-    // other face's direction; c0 the centre EMF at the edge's cell, ca, cb, cab below
-    // it along a, along b and along both
-    auto edge = [&](T pa, T pas, T pb, T pbs, T ma, T mas, T mb, T mbs, T c0, T ca, T cb, T cab) {
-        return T(0.25) * ((pa - corr(ma, c0, pb, ca, pbs)) + (pas + corr(mas, pb, cb, pbs, cab)) +
-                          (pb - corr(mb, c0, pa, cb, pas)) + (pbs + corr(mbs, pa, ca, pas, cab)));
-    };
     const T *F1r = F1 + RHO * ks + c, *F2r = F2 + RHO * ks + c, *F3r = F3 + RHO * ks + c;
     const T f23 = F2[B3 * ks + c], f23s = F2[B3 * ks + c - D3], f32 = F3[B2 * ks + c], f32s = F3[B2 * ks + c - D2];
-    e[0] = edge(-f23, -f23s, f32, f32s, F2r[0], F2r[-D3], F3r[0], F3r[-D2], ec(1, 0, 0, 0), ec(1, 0, -1, 0),
-                ec(1, 0, 0, -1), ec(1, 0, -1, -1));
+    e[0] = edge_emf<T>(w, -f23, -f23s, f32, f32s, F2r[0], F2r[-D3], F3r[0], F3r[-D2], ec(1, 0, 0, 0), ec(1, 0, -1, 0),
+                       ec(1, 0, 0, -1), ec(1, 0, -1, -1));
     const T f31 = F3[B1 * ks + c], f31s = F3[B1 * ks + c - D1], f13 = F1[B3 * ks + c], f13s = F1[B3 * ks + c - D3];
-    e[1] = edge(-f31, -f31s, f13, f13s, F3r[0], F3r[-D1], F1r[0], F1r[-D3], ec(2, 0, 0, 0), ec(2, 0, 0, -1),
-                ec(2, -1, 0, 0), ec(2, -1, 0, -1));
-    const T f12 = F1[B2 * ks + c], f12s = F1[B2 * ks + c - D2], f21 = F2[B1 * ks + c], f21s = F2[B1 * ks + c - D1];
-    // (a = x2, b = x1 up to the sign of both: the reference's order of the sum)
-    e[2] = edge(f21, f21s, -f12, -f12s, F2r[0], F2r[-D1], F1r[0], F1r[-D2], ec(3, 0, 0, 0), ec(3, 0, -1, 0),
-                ec(3, -1, 0, 0), ec(3, -1, -1, 0));
-    if ((d.pole1 && j == d.ng2) || (d.pole2 && j == d.n2 + d.ng2)) {
-        e[2] = T(0.);
-        e[0] = T(-0.5) * (f23 + f23s);
-    }
+    e[1] = edge_emf<T>(w, -f31, -f31s, f13, f13s, F3r[0], F3r[-D1], F1r[0], F1r[-D3], ec(2, 0, 0, 0), ec(2, 0, 0, -1),
+                       ec(2, -1, 0, 0), ec(2, -1, 0, -1));
+    e[2] = emf_edge3<T>(d, ec, F1, F2, c, j);
+    if ((d.pole1 && j == d.ng2) || (d.pole2 && j == d.n2 + d.ng2)) e[0] = T(-0.5) * (f23 + f23s);
 }
 
 template <typename T>
@@ -1020,6 +1078,34 @@ __global__ void __launch_bounds__(BLK) k_face_update(const Dims d, const Geom m,
 #pragma unroll
     for (int q = 0; q < ZP; q++)
         if (z0 + q < nz) k_face_update_at(d, m, psi, psf, Et, st, row * nz + z0 + q);
+}
+
+// Edge EMF and face update of a 2-D block in one launch: a thread evaluates
+// the E3 of its zone's corner and of the two next to it, which its two faces
+// need (each corner three times over, a few loads from cache against a launch
+// and a round trip; 256 x 256 torus, per step, 0.036 -> 0.021 ms). It also
+// empties the inversion's failed-zone list. Same values as k_emf_edge and
+// k_face_update.
+template <typename T>
+__global__ void __launch_bounds__(BLK) k_ct_2d(const Dims d, const Geom m, const double *psi, double *psf,
+                                                const T *__restrict__ Ec, const T *__restrict__ F1,
+                                                const T *__restrict__ F2, StepSize st, int *__restrict__ nfail) {
+    const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t == 0) *nfail = 0;
+    const int nj = d.n2 + d.d2;
+    if (t >= (long)(d.n1 + d.d1) * nj) return;
+    const int j = d.ng2 + (int)(t % nj), i = d.ng1 + (int)(t / nj);
+    const long isize = d.G2;
+    // E3 at the corner (di, dj) up, zero where neither face needs it
+    auto e3 = [&](int di, int dj) -> double {
+        if (i + di > d.n1 + d.ng1 || j + dj > d.n2 + d.ng2) return 0.;
+        const long c = cix(d, i + di, j + dj, 0);
+        auto ec = [&](int k, int ei, int ej, int) { return Ec[k * d.ks + c + ei * isize + ej]; };
+        return (double)emf_edge3<T>(d, ec, F1, F2, c, j + dj);
+    };
+    const double e00 = e3(0, 0), e10 = e3(1, 0), e01 = e3(0, 1);
+    auto E = [&](int, int di, int dj, int) { return di ? e10 : (dj ? e01 : e00); };
+    face_update_eval(d, m, psi, psf, E, st.sub(), i, j, 0, cix(d, i, j, 0), gix(d, i, j), 7);
 }
 
 // ---------------------------------------------------------------- fused CT
@@ -1911,6 +1997,48 @@ __global__ void __launch_bounds__(BLK, HAMR_UPD_MINB)
     invert_epilogue<FIX>(d, gm, c, flag, pf, pout, pflag, failimage);
 }
 
+// The conserved update and the primary inversion of small blocks in one
+// kernel, a zone per thread (the inversion's U[B] from the updated faces): one
+// launch, and the update's primitives are the inversion's guess (256 x 256
+// torus, per step with the fallback pass, 0.072 -> 0.053 ms; 64 x 64 box 0.055
+// -> 0.041). Larger blocks keep k_cons and k_invert_primary, whose separate
+// register budgets hold more zones in flight (the tiled update and inversion of
+// the 64-torus ensemble lost a tenth fused). W is written for every zone: the fallback reads it, and so
+// does a recorded step's reverse. *nfail must be zero on entry. Same values as
+// the two kernels.
+#ifndef HAMR_CONS_INV_MINB
+#define HAMR_CONS_INV_MINB 4
+#endif
+template <typename T, int INV, int FIX>
+__global__ void __launch_bounds__(BLK, HAMR_CONS_INV_MINB)
+    k_cons_inv(const Dims d, const Geom m, const double *__restrict__ pin, const double *__restrict__ pb,
+               double *__restrict__ Ucache, const T *__restrict__ F1, const T *__restrict__ F2,
+               const T *__restrict__ F3, double *__restrict__ W, int full, StepSize st,
+               const double *__restrict__ psf, double *__restrict__ pout, int *__restrict__ pflag,
+               int *__restrict__ failimage, int *__restrict__ flist, int *__restrict__ nfail) {
+    const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= (long)d.n1 * d.n2 * d.n3) return;
+    const int z = d.ng3 + (int)(t % d.n3);
+    const int j = d.ng2 + (int)((t / d.n3) % d.n2);
+    const int i = d.ng1 + (int)(t / ((long)d.n3 * d.n2));
+    const long c = cix(d, i, j, z), gi = gix(d, i, j);
+    Geo<double> gm;
+    load_geo(d, m, i, j, CENT, gm);
+    double pf[NPR], U[NPR];
+    cons_update<T>(d, m, pin, pb, Ucache, F1, F2, F3, full, st.sub(), i, j, c, gi, gm, ConnTable{m.conn, d.gs, gi},
+                   pf, U);
+#pragma unroll
+    for (int q = 0; q < N_ADV; q++) W[q * d.ks + c] = U[adv_comp(q)];
+    if (d.ng3 == 0) W[6 * d.ks + c] = U[B3];
+    face_average_b(d, m, psf, i, j, c, gi, U);
+    const int flag = invert_primary<INV>(d, inv_k(d, m, gi, gm), gm, U, pf);
+    if (flag) {
+        flist[atomicAdd(nfail, 1)] = (int)t;
+        return;
+    }
+    invert_epilogue<FIX>(d, gm, c, flag, pf, pout, pflag, failimage);
+}
+
 // the fallback chain and epilogue of one listed zone (active-zone index t)
 template <int FIX>
 __device__ __forceinline__ void invert_fallback_at(const Dims &d, const Geom &m, const double *__restrict__ pg,
@@ -2234,8 +2362,18 @@ __device__ __forceinline__ void k_bound_x2_at(const Dims &d, double *pv, double 
     }
 }
 
-__global__ void k_bound_x2(const Dims d, double *pv, double *ps) {
+// The step-size update of a full sub-step (k_dt_finalize's work), done by the
+// last launch of the step; ndt null: none
+struct DtFinal {
+    unsigned long long *dtbits;
+    double *ndt, *dt_state;
+    int *counter, interval;
+};
+__device__ __forceinline__ void dt_finalize(const DtFinal &f);
+
+__global__ void k_bound_x2(const Dims d, double *pv, double *ps, const DtFinal fin) {
     const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t == 0 && fin.ndt) dt_finalize(fin);
     if (t >= n_bound_x2(d)) return;
     k_bound_x2_at(d, pv, ps, t);
 }
@@ -2295,21 +2433,21 @@ __global__ void k_dt_reset(unsigned long long *dtbits) {
 // CFL step 1/(1/dt1 + 1/dt2 + 1/dt3) of the last full sub-step
 // (step_ch.c:1320-1331). In advance mode (dt_state != NULL) the device step
 // size follows min(ndt, 1.3 dt) every `interval` steps (step_ch.c:973-975).
-__global__ void k_dt_finalize(unsigned long long *dtbits, double *ndt_out, double *dt_state, int *counter, int interval) {
-    if (threadIdx.x != 0) return;
-    const double d1 = __longlong_as_double((long long)dtbits[1]);
-    const double d2 = __longlong_as_double((long long)dtbits[2]);
-    const double d3 = __longlong_as_double((long long)dtbits[3]);
+// One thread of the step's last launch.
+__device__ __forceinline__ void dt_finalize(const DtFinal &f) {
+    const double d1 = __longlong_as_double((long long)f.dtbits[1]);
+    const double d2 = __longlong_as_double((long long)f.dtbits[2]);
+    const double d3 = __longlong_as_double((long long)f.dtbits[3]);
     const double ndt = 1. / (1. / d1 + 1. / d2 + 1. / d3);
-    *ndt_out = ndt;
-    if (dt_state) {
-        const int n = ++(*counter);
-        if (interval <= 1 || n % interval == 0) {
-            double dt = *dt_state;
-            *dt_state = ndt > 1.3 * dt ? 1.3 * dt : ndt;
+    *f.ndt = ndt;
+    if (f.dt_state) {
+        const int n = ++(*f.counter);
+        if (f.interval <= 1 || n % f.interval == 0) {
+            double dt = *f.dt_state;
+            *f.dt_state = ndt > 1.3 * dt ? 1.3 * dt : ndt;
         }
     }
-    dtbits[0] = dtbits[1] = dtbits[2] = dtbits[3] = BITS_1E9;
+    f.dtbits[0] = f.dtbits[1] = f.dtbits[2] = f.dtbits[3] = BITS_1E9;
 }
 
 // |div B| max over active zones (divb_calc, diag.c:153-199)
@@ -2380,6 +2518,9 @@ struct hamr_ctx {
     // 3-D blocks: the centre EMFs computed by the x3 flux kernel instead of
     // k_emf_centre (HAMR_EMF_IN_X3=0 keeps the separate kernel)
     bool emf_in_x3 = true;
+    // zones up to which the update without bulk copies takes the primary
+    // inversion into its kernel (HAMR_CONS_INV_MAX overrides)
+    long cons_inv_max = 1L << 17;
     // the primary inversion inside the TMA-staged update kernel (no floors or
     // repair; HAMR_FUSE_INV=0 keeps the separate inversion kernel)
     bool fuse_inv = true;
@@ -2450,7 +2591,7 @@ inline void prof_mark(Prof *pf, int slot, cudaStream_t s) {
 // ghost fill of the state written by a sub-step (full: p, ps; else ph, psh)
 // in direction dim (1, 2, 3), on the block's physical sides; dim 0: all
 // three, in the order x1, x3, x2
-int launch_bound_dim(hamr_ctx *ctx, int full, int dim) {
+int launch_bound_dim(hamr_ctx *ctx, int full, int dim, const DtFinal &fin = {}) {
     const Dims &d = ctx->d;
     cudaStream_t s = ctx->stream;
     double *pw = full ? ctx->p : ctx->ph;
@@ -2458,7 +2599,7 @@ int launch_bound_dim(hamr_ctx *ctx, int full, int dim) {
     if ((dim == 0 || dim == 1) && d.d1)
         k_bound_x1<<<nblk((long)d.ng1 * d.G2 * d.G3), BLK, 0, s>>>(d, geom_of(ctx), pw, psw);
     if ((dim == 0 || dim == 3) && d.d3) k_bound_x3<<<nblk(n_bound_x3(d)), BLK, 0, s>>>(d, pw, psw);
-    if ((dim == 0 || dim == 2) && d.d2) k_bound_x2<<<nblk(n_bound_x2(d)), BLK, 0, s>>>(d, pw, psw);
+    if ((dim == 0 || dim == 2) && d.d2) k_bound_x2<<<nblk(n_bound_x2(d)), BLK, 0, s>>>(d, pw, psw, fin);
     CK(cudaGetLastError());
     return HAMR_OK;
 }
@@ -2511,6 +2652,26 @@ void launch_flux(long n, cudaStream_t s, const Dims &d, const Geom &m, const dou
     }
 }
 
+// fluxes of both directions and centre EMFs of a 2-D block (k_flux_2d)
+template <typename T>
+void launch_flux_2d(cudaStream_t s, const Dims &d, const Geom &m, const double *pin, const double *psin, T *F1, T *F2,
+                    T *Ec, unsigned long long *dtbits, int cd) {
+    const int nb1 = nblk(n_faces<1>(d)), nb2 = nb1 + nblk(n_faces<2>(d));
+    const unsigned nb = nb2 + nblk((long)(d.n1 + 2 * d.d1) * (d.n2 + 2 * d.d2));
+    const bool fix = d.bc2 == HAMR_BC_POLE_REFL;
+    auto run = [&](auto plain, auto fixed) {
+        (fix ? fixed : plain)<<<nb, BLK, 0, s>>>(d, m, pin, psin, F1, F2, Ec, dtbits, cd, nb1, nb2);
+    };
+    switch (rec_key(d)) {
+    case 1: run(k_flux_2d<T, 1, false>, k_flux_2d<T, 1, true>); break;
+    case 2: run(k_flux_2d<T, 2, false>, k_flux_2d<T, 2, true>); break;
+    case 3: run(k_flux_2d<T, 3, false>, k_flux_2d<T, 3, true>); break;
+    case 6: run(k_flux_2d<T, 6, false>, k_flux_2d<T, 6, true>); break;
+    case 7: run(k_flux_2d<T, 7, false>, k_flux_2d<T, 7, true>); break;
+    default: run(k_flux_2d<T, 0, false>, k_flux_2d<T, 0, true>); break;
+    }
+}
+
 // the bulk copies of k_cons_tma need 16-byte aligned flux planes
 template <typename T>
 bool cons_tma_aligned(const hamr_ctx *ctx, const Dims &d, const T *F1, const T *F2, const T *F3) {
@@ -2522,7 +2683,7 @@ bool cons_tma_aligned(const hamr_ctx *ctx, const Dims &d, const T *F1, const T *
 // type of the fluxes and EMFs (double, or float in the mixed-precision step);
 // the float arrays reuse the double allocations with the same plane stride.
 template <typename T>
-int launch_stage_t(hamr_ctx *ctx, int full, StepSize st, bool calc_dt, Prof *pf) {
+int launch_stage_t(hamr_ctx *ctx, int full, StepSize st, bool calc_dt, Prof *pf, const DtFinal &fin) {
     const Dims &d = ctx->d;
     T *F1 = reinterpret_cast<T *>(ctx->F1), *F2 = reinterpret_cast<T *>(ctx->F2);
     T *F3 = reinterpret_cast<T *>(ctx->F3), *Ec = reinterpret_cast<T *>(ctx->Ec);
@@ -2539,6 +2700,10 @@ int launch_stage_t(hamr_ctx *ctx, int full, StepSize st, bool calc_dt, Prof *pf)
     cudaStream_t s2 = conc ? ctx->side[0] : s, s3 = conc ? ctx->side[1] : s;
     // 3-D: the centre EMFs come out of the x3 flux kernel
     const bool ec_x3 = d.d3 && !ctx->ct_fused && ctx->emf_in_x3;
+    // a 2-D block whose faces do not fill the device: one launch for both
+    // directions' fluxes, their polar and radial rules and the centre EMFs, one
+    // for the edge EMF and the face update
+    const bool flat = !d.d3 && !conc && n_flux_rows<1>(d) < ctx->rows_min && n_flux_rows<2>(d) < ctx->rows_min;
     if (conc) {
         CK(cudaEventRecord(ctx->ev[0], s));
         CK(cudaStreamWaitEvent(s2, ctx->ev[0], 0));
@@ -2549,12 +2714,13 @@ int launch_stage_t(hamr_ctx *ctx, int full, StepSize st, bool calc_dt, Prof *pf)
         launch_flux<3, T>(n, s, d, m, pin, psin, F3, ctx->dtbits, cd, ctx->rows_min, ec_x3 ? Ec : nullptr);
     }
     prof_mark(pf, PROF_FLUX3, s);
-    {
+    if (flat) launch_flux_2d<T>(s, d, m, pin, psin, F1, F2, Ec, ctx->dtbits, cd);
+    else {
         long n = (long)(d.n1 + 2 * d.d1) * (d.n2 + 2 * d.d2 - 1) * (d.n3 + 2 * d.d3);
         launch_flux<2, T>(n, s2, d, m, pin, psin, F2, ctx->dtbits, cd, ctx->rows_min);
     }
     prof_mark(pf, PROF_FLUX2, s);
-    {
+    if (!flat) {
         long n = (long)(d.n1 + 2 * d.d1 - 1) * (d.n2 + 2 * d.d2) * (d.n3 + 2 * d.d3);
         launch_flux<1, T>(n, s3, d, m, pin, psin, F1, ctx->dtbits, cd, ctx->rows_min);
     }
@@ -2567,7 +2733,7 @@ int launch_stage_t(hamr_ctx *ctx, int full, StepSize st, bool calc_dt, Prof *pf)
         CK(cudaStreamWaitEvent(s, ctx->ev[1], 0));
         CK(cudaStreamWaitEvent(s, ctx->ev[2], 0));
     }
-    if (d.bc2 == HAMR_BC_POLE_REFL) {
+    if (d.bc2 == HAMR_BC_POLE_REFL && !flat) {
         long n = (long)d.G1 * d.G3 + (long)d.G2 * d.G3;
         k_fix_flux<T><<<nblk(n), BLK, 0, s>>>(d, F1, F2, F3);
     }
@@ -2579,7 +2745,14 @@ int launch_stage_t(hamr_ctx *ctx, int full, StepSize st, bool calc_dt, Prof *pf)
         CK(cudaEventRecord(ctx->ev[3], s));
         CK(cudaStreamWaitEvent(s2, ctx->ev[3], 0));
     }
-    if (d.d3 && ctx->ct_fused) {
+    if (flat) {
+        prof_mark(pf, PROF_EMF_CENTRE, s);
+        prof_mark(pf, PROF_EMF_EDGE, s);
+        prof_mark(pf, PROF_POLE_AVG, s);
+        k_ct_2d<T><<<nblk((long)(d.n1 + d.d1) * (d.n2 + d.d2)), BLK, 0, s>>>(
+            d, m, ctx->ps, full ? ctx->ps : ctx->psh, Ec, F1, F2, st, ctx->nfail);
+        prof_mark(pf, PROF_FACE, s);
+    } else if (d.d3 && ctx->ct_fused) {
         // centre EMFs, edge EMFs and the face update in one kernel (polar
         // rows of transmissive poles after the phi average); timed as the
         // edge-EMF group
@@ -2624,6 +2797,9 @@ int launch_stage_t(hamr_ctx *ctx, int full, StepSize st, bool calc_dt, Prof *pf)
         // the primary inversion inside the update kernel (the face update, which
         // it reads, has run in this stream)
         const bool fuse = tma && ctx->fuse_inv && fix == 0 && ctx->prm.repair != 2 && !conc;
+        // small blocks without the bulk-copy update: update and primary
+        // inversion in one kernel
+        const bool small = !tma && !conc && ctx->fuse_inv && n <= ctx->cons_inv_max;
         if (tma) {   // one row of zones per CTA, flux operands staged by bulk copies
             const int npiece = (d.n3 + 255) / 256, lpiece = (d.n3 + npiece - 1) / npiece;
             const dim3 grid(d.n1 * d.n2 * npiece), block((lpiece + 31) / 32 * 32);
@@ -2638,6 +2814,18 @@ int launch_stage_t(hamr_ctx *ctx, int full, StepSize st, bool calc_dt, Prof *pf)
                 k_cons_tma<T><<<grid, block, sm, s>>>(d, m, ctx->p, pg, ctx->U, F1, F2, F3, ctx->W, full, st,
                                                       ctx->nfail, ctx->kerr, npiece, lpiece);
             }
+        } else if (small) {
+            if (!flat) CK(cudaMemsetAsync(ctx->nfail, 0, sizeof(int), s));   // else emptied by k_ct_2d
+            using ConsInv = void (*)(const Dims, const Geom, const double *, const double *, double *, const T *,
+                                     const T *, const T *, double *, int, StepSize, const double *, double *, int *,
+                                     int *, int *, int *);
+            static const ConsInv ci[2][4] = {
+                {k_cons_inv<T, HAMR_INV_2D, 0>, k_cons_inv<T, HAMR_INV_2D, 1>, k_cons_inv<T, HAMR_INV_2D, 2>,
+                 k_cons_inv<T, HAMR_INV_2D, 3>},
+                {k_cons_inv<T, HAMR_INV_NM, 0>, k_cons_inv<T, HAMR_INV_NM, 1>, k_cons_inv<T, HAMR_INV_NM, 2>,
+                 k_cons_inv<T, HAMR_INV_NM, 3>}};
+            ci[nm][fix]<<<nblk(n), BLK, 0, s>>>(d, m, ctx->p, pg, ctx->U, F1, F2, F3, ctx->W, full, st, psf, pout,
+                                                ctx->pflag, ctx->failimage, ctx->flist, ctx->nfail);
         } else if (d.n3 >= 64 && ctx->cons_cols)   // metric and connection staged per CTA
             k_cons_cols<T><<<nblk(n), BLK, 0, s>>>(d, m, ctx->p, full ? ctx->ph : ctx->p, ctx->U, F1, F2, F3, ctx->W,
                                                    full, st, ctx->nfail);
@@ -2666,7 +2854,7 @@ int launch_stage_t(hamr_ctx *ctx, int full, StepSize st, bool calc_dt, Prof *pf)
              k_invert_fallback<HAMR_INV_2D, 3>},
             {k_invert_fallback<HAMR_INV_NM, 0>, k_invert_fallback<HAMR_INV_NM, 1>, k_invert_fallback<HAMR_INV_NM, 2>,
              k_invert_fallback<HAMR_INV_NM, 3>}};
-        if (!fuse)
+        if (!fuse && !small)
             inv_p[nm][fix]<<<nblk(n), BLK, 0, s>>>(d, m, pg, ctx->W, psf, pout, ctx->pflag, ctx->failimage,
                                                    ctx->flist, ctx->nfail);
         inv_f[nm][fix]<<<FALLBACK_CTAS, BLK, 0, s>>>(d, m, pg, ctx->W, psf, pout, ctx->pflag, ctx->failimage,
@@ -2681,25 +2869,23 @@ int launch_stage_t(hamr_ctx *ctx, int full, StepSize st, bool calc_dt, Prof *pf)
     prof_mark(pf, PROF_INVERT, s);
     // ghost fill of the written state; a block of a decomposed domain leaves
     // it to the caller (hamr_bound_dim around the halo exchange)
-    if (!d.halo) launch_bound_dim(ctx, full, 0);
+    if (!d.halo) launch_bound_dim(ctx, full, 0, fin);
     prof_mark(pf, PROF_BOUND, s);
     CK(cudaGetLastError());
     return HAMR_OK;
 }
 
-int launch_stage(hamr_ctx *ctx, int full, StepSize st, bool calc_dt, Prof *pf = nullptr) {
-    if (ctx->prm.precision == HAMR_MIXED) return launch_stage_t<float>(ctx, full, st, calc_dt, pf);
-    return launch_stage_t<double>(ctx, full, st, calc_dt, pf);
+int launch_stage(hamr_ctx *ctx, int full, StepSize st, bool calc_dt, Prof *pf = nullptr, const DtFinal &fin = {}) {
+    if (ctx->prm.precision == HAMR_MIXED) return launch_stage_t<float>(ctx, full, st, calc_dt, pf, fin);
+    return launch_stage_t<double>(ctx, full, st, calc_dt, pf, fin);
 }
 
 int launch_step(hamr_ctx *ctx, StepSize half, StepSize full, double *dt_state, int interval) {
     int rc = launch_stage(ctx, 0, half, false);
     if (rc) return rc;
-    rc = launch_stage(ctx, 1, full, true);
-    if (rc) return rc;
-    k_dt_finalize<<<1, 32, 0, ctx->stream>>>(ctx->dtbits, ctx->ndt, dt_state, ctx->counter, interval);
-    CK(cudaGetLastError());
-    return HAMR_OK;
+    // the step size with the last ghost fill (blocks with halo sides, whose
+    // ghost fill is the caller's, do not step here)
+    return launch_stage(ctx, 1, full, true, nullptr, DtFinal{ctx->dtbits, ctx->ndt, dt_state, ctx->counter, interval});
 }
 
 }  // namespace
@@ -2772,6 +2958,7 @@ int hamr_ctx_create(const hamr_params *prm, hamr_ctx **out) {
         if (const char *e = getenv("HAMR_CONS_TMA")) ctx->cons_tma = atoi(e) != 0;
         if (const char *e = getenv("HAMR_CONCURRENT")) ctx->concurrent = atoi(e) != 0;
         if (const char *e = getenv("HAMR_EMF_IN_X3")) ctx->emf_in_x3 = atoi(e) != 0;
+        if (const char *e = getenv("HAMR_CONS_INV_MAX")) ctx->cons_inv_max = atol(e);
         if (const char *e = getenv("HAMR_FUSE_INV")) ctx->fuse_inv = atoi(e) != 0;
     }
     if (ctx->concurrent) {
