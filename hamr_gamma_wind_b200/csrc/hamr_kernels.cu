@@ -123,6 +123,20 @@ __device__ __forceinline__ void load_geo_block(const T *q, Geo<T> &o) {
     o.lapse = v[GT_LAPSE];
 }
 
+// Item t of an (i, j, z) range, z fastest: t = (i nj + j) nz + z. In 32 bits:
+// an item is a zone, face or ghost cell of one block, whose 75 planes of eight
+// bytes fill the device's memory long before 2^31 of them; a 64-bit quotient
+// by a run-time divisor costs three times as much, and a kernel that moves a
+// few values per item (edge EMFs, face update) issued a quarter to a half of
+// its instructions for them.
+struct Item3 {
+    int i, j, z;
+};
+__device__ __forceinline__ Item3 item3(long t, int nz, int nj) {
+    const unsigned u = (unsigned)t, q = u / (unsigned)nz, i = q / (unsigned)nj;
+    return Item3{(int)i, (int)(q - i * (unsigned)nj), (int)(u - q * (unsigned)nz)};
+}
+
 __device__ __forceinline__ long cix(const Dims &d, int i, int j, int z) { return ((long)i * d.G2 + j) * d.G3 + z; }
 __device__ __forceinline__ long gix(const Dims &d, int i, int j) { return (long)i * d.G2 + j; }
 
@@ -247,9 +261,10 @@ __device__ __forceinline__ double flux_face(const Dims &d, const Geom &m, const 
     const int j0 = (d.ng2 - 1) * d.d2 + jdel, nj = d.n2 + 2 * d.d2 - jdel;
     const int z0 = (d.ng3 - 1) * d.d3 + zdel, nz = d.n3 + 2 * d.d3 - zdel;
     (void)ni;
-    const int z = z0 + (int)(t % nz);
-    const int j = j0 + (int)((t / nz) % nj);
-    const int i = i0 + (int)(t / ((long)nz * nj));
+    const Item3 it = item3(t, nz, nj);
+    const int z = z0 + it.z;
+    const int j = j0 + it.j;
+    const int i = i0 + it.i;
     const long c = cix(d, i, j, z);
     const long stride = idel ? (long)d.G2 * d.G3 : (jdel ? (long)d.G3 : 1L);
     const int face = DIR == 1 ? FACE1 : (DIR == 2 ? FACE2 : FACE3);
@@ -506,10 +521,10 @@ __device__ __forceinline__ double flux_x3_slots(const Dims &d, const Geom &m, co
     const int rz = d.n3 + 2 * d.d3 + 2 * H;   // slots per row
     const int nj = d.n2 + 2 * d.d2;
     const long sl = blk * STEP + l;
-    const int zl = (int)(sl % rz);
-    const long row = sl / rz;
-    const int j = (d.ng2 - 1) * d.d2 + (int)(row % nj);
-    const int i = (d.ng1 - 1) * d.d1 + (int)(row / nj);
+    const Item3 it = item3(sl, rz, nj);
+    const int zl = it.z;
+    const int j = (d.ng2 - 1) * d.d2 + it.j;
+    const int i = (d.ng1 - 1) * d.d1 + it.i;
     const long c = cix(d, i, j, d.ng3 - 1 - H + zl);   // the slot's zone
     T hi[NPR];
     if constexpr (H == 0) {
@@ -698,11 +713,11 @@ __device__ __forceinline__ double flux_row(const Dims &d, const Geom &m, const d
                                            const double *__restrict__ ps, T *__restrict__ F, T *wbuf, const long t) {
     using Win = RowWindow<DIR, T, REC>;
     double cmx = 0.0;
-    const int nz = d.n3 + 2 * d.d3, z = (d.ng3 - 1) * d.d3 + (int)(t % nz);
-    const long r = t / nz;
     const int nt = DIR == 1 ? d.n2 + 2 * d.d2 : d.n1 + 2 * d.d1;
-    const int a = (DIR == 1 ? (d.ng2 - 1) * d.d2 : (d.ng1 - 1) * d.d1) + (int)(r % nt);   // j or i
-    const int seg = (int)(r / nt);
+    const Item3 it = item3(t, d.n3 + 2 * d.d3, nt);
+    const int z = (d.ng3 - 1) * d.d3 + it.z;
+    const int a = (DIR == 1 ? (d.ng2 - 1) * d.d2 : (d.ng1 - 1) * d.d1) + it.j;   // j or i
+    const int seg = it.i;
     const int nf = DIR == 1 ? d.n1 + 2 * d.d1 - 1 : d.n2 + 2 * d.d2 - 1;
     const int ng = DIR == 1 ? d.ng1 : d.ng2;
     const int f0 = ng + seg * FLUX_ROW;
@@ -810,9 +825,10 @@ template <typename T>
 __device__ __forceinline__ void k_emf_centre_at(const Dims &d, const Geom &m, const double *__restrict__ pv,
                                                      T *__restrict__ Ec, const long t) {
     const int ni = d.n1 + 2 * d.d1, nj = d.n2 + 2 * d.d2, nz = d.n3 + 2 * d.d3;
-    const int z = (d.ng3 - d.d3) * d.d3 + (int)(t % nz);
-    const int j = (d.ng2 - d.d2) * d.d2 + (int)((t / nz) % nj);
-    const int i = (d.ng1 - d.d1) * d.d1 + (int)(t / ((long)nz * nj));
+    const Item3 it = item3(t, nz, nj);
+    const int z = (d.ng3 - d.d3) * d.d3 + it.z;
+    const int j = (d.ng2 - d.d2) * d.d2 + it.j;
+    const int i = (d.ng1 - d.d1) * d.d1 + it.i;
     (void)ni;
     const long c = cix(d, i, j, z);
     T e[3];
@@ -871,7 +887,9 @@ __global__ void __launch_bounds__(BLK, HAMR_FLUX_2D_MINB)
 // The reference forms both sides' corrections and weighs them by 0 and 1; here
 // the mass flux's sign picks the operands and one difference is formed: the
 // same value for finite operands, in a third of the operations and few enough
-// registers for eight blocks per SM (the loads' latency is what bounds it).
+// registers for eight blocks per SM in float, six in FP64 (the loads' latency
+// is what bounds it). 384 x 192 x 192 torus, per step: FP64 1.04 -> 0.69 ms (8
+// blocks 0.72-0.79, 10 0.75), float 0.58 -> 0.41 (6 blocks 0.48, 10 0.51).
 //
 // edge_emf: E_k from the faces of the two other directions a and b: pa, pb the
 // face EMFs and ma, mb the mass fluxes, _s at the cell below along the other
@@ -894,12 +912,13 @@ __device__ __forceinline__ T edge_emf(bool upwind, T pa, T pas, T pb, T pbs, T m
 template <typename T, class EC>
 __device__ __forceinline__ T emf_edge3(const Dims &d, EC ec, const T *__restrict__ F1, const T *__restrict__ F2, long c,
                                        int j) {
-    if ((d.pole1 && j == d.ng2) || (d.pole2 && j == d.n2 + d.ng2)) return T(0.);
+    const bool pole = (d.pole1 && j == d.ng2) || (d.pole2 && j == d.n2 + d.ng2);
     const long ks = d.ks, D1 = d.d1 * (long)d.G2 * d.G3, D2 = d.d2 * (long)d.G3;
     const T *F1r = F1 + RHO * ks + c, *F2r = F2 + RHO * ks + c;
-    return edge_emf<T>(d.ct_upwind != 0, F2[B1 * ks + c], F2[B1 * ks + c - D1], -F1[B2 * ks + c], -F1[B2 * ks + c - D2],
+    const T e = edge_emf<T>(d.ct_upwind != 0, F2[B1 * ks + c], F2[B1 * ks + c - D1], -F1[B2 * ks + c], -F1[B2 * ks + c - D2],
                        F2r[0], F2r[-D1], F1r[0], F1r[-D2], ec(3, 0, 0, 0), ec(3, 0, -1, 0), ec(3, -1, 0, 0),
                        ec(3, -1, -1, 0));
+    return pole ? T(0.) : e;
 }
 
 template <typename T, class EC>
@@ -925,9 +944,10 @@ __device__ __forceinline__ void k_emf_edge_at(const Dims &d, const T *__restrict
                                                    const T *__restrict__ F1, const T *__restrict__ F2,
                                                    const T *__restrict__ F3, T *__restrict__ emf, const long t) {
     const int ni = d.n1 + d.d1, nj = d.n2 + d.d2, nz = d.n3 + d.d3;
-    const int z = d.ng3 * d.d3 + (int)(t % nz);
-    const int j = d.ng2 * d.d2 + (int)((t / nz) % nj);
-    const int i = d.ng1 * d.d1 + (int)(t / ((long)nz * nj));
+    const Item3 it = item3(t, nz, nj);
+    const int z = d.ng3 * d.d3 + it.z;
+    const int j = d.ng2 * d.d2 + it.j;
+    const int i = d.ng1 * d.d1 + it.i;
     (void)ni;
     const long c = cix(d, i, j, z);
     const long ks = d.ks, jsize = d.G3, isize = (long)d.G2 * d.G3;
@@ -944,10 +964,13 @@ __device__ __forceinline__ void k_emf_edge_at(const Dims &d, const T *__restrict
 // (two z edges per thread, as k_face_update takes two face triples, measured
 // slower: 0.58 -> 0.63 ms per mixed 384 x 192 x 192 step, 1.03 -> 1.07 FP64)
 #ifndef HAMR_EMF_EDGE_MINB
-#define HAMR_EMF_EDGE_MINB 8
+#define HAMR_EMF_EDGE_MINB 6
+#endif
+#ifndef HAMR_EMF_EDGE_MINB_F
+#define HAMR_EMF_EDGE_MINB_F 8
 #endif
 template <typename T>
-__global__ void __launch_bounds__(BLK, HAMR_EMF_EDGE_MINB) k_emf_edge(const Dims d, const T *__restrict__ Ec,
+__global__ void __launch_bounds__(BLK, sizeof(T) == 8 ? HAMR_EMF_EDGE_MINB : HAMR_EMF_EDGE_MINB_F) k_emf_edge(const Dims d, const T *__restrict__ Ec,
                                                    const T *__restrict__ F1, const T *__restrict__ F2,
                                                    const T *__restrict__ F3, T *__restrict__ emf) {
     const int ni = d.n1 + d.d1, nj = d.n2 + d.d2, nz = d.n3 + d.d3;
@@ -1047,9 +1070,10 @@ template <typename T>
 __device__ __forceinline__ void k_face_update_at(const Dims &d, const Geom &m, const double *psi, double *psf,
                                                       const T *__restrict__ Et, StepSize st, const long t) {
     const int ni = d.n1 + d.d1, nj = d.n2 + d.d2, nz = d.n3 + d.d3;
-    const int z = d.ng3 * d.d3 + (int)(t % nz);
-    const int j = d.ng2 * d.d2 + (int)((t / nz) % nj);
-    const int i = d.ng1 * d.d1 + (int)(t / ((long)nz * nj));
+    const Item3 it = item3(t, nz, nj);
+    const int z = d.ng3 * d.d3 + it.z;
+    const int j = d.ng2 * d.d2 + it.j;
+    const int i = d.ng1 * d.d1 + it.i;
     (void)ni;
     const long c = cix(d, i, j, z), gi = gix(d, i, j);
     const long ks = d.ks, isize = (long)d.G2 * d.G3, jsz = d.G3;
@@ -1073,8 +1097,8 @@ __global__ void __launch_bounds__(BLK) k_face_update(const Dims d, const Geom m,
     const int nzp = (nz + ZP - 1) / ZP;
     const long u = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (u >= (long)ni * nj * nzp) return;
-    const long row = u / nzp;
-    const int z0 = (int)(u % nzp) * ZP;
+    const long row = (unsigned)u / (unsigned)nzp;
+    const int z0 = (int)((unsigned)u % (unsigned)nzp) * ZP;
 #pragma unroll
     for (int q = 0; q < ZP; q++)
         if (z0 + q < nz) k_face_update_at(d, m, psi, psf, Et, st, row * nz + z0 + q);
@@ -1094,7 +1118,8 @@ __global__ void __launch_bounds__(BLK) k_ct_2d(const Dims d, const Geom m, const
     if (t == 0) *nfail = 0;
     const int nj = d.n2 + d.d2;
     if (t >= (long)(d.n1 + d.d1) * nj) return;
-    const int j = d.ng2 + (int)(t % nj), i = d.ng1 + (int)(t / nj);
+    const Item3 it = item3(t, nj, 1 << 30);
+    const int j = d.ng2 + it.z, i = d.ng1 + it.j;
     const long isize = d.G2;
     // E3 at the corner (di, dj) up, zero where neither face needs it
     auto e3 = [&](int di, int dj) -> double {
@@ -1622,9 +1647,10 @@ __device__ __forceinline__ void k_cons_at(const Dims &d, const Geom &m, const do
                                                const T *__restrict__ F1, const T *__restrict__ F2,
                                                const T *__restrict__ F3, double *__restrict__ W, int full,
                                                StepSize st, const long t) {
-    const int z = d.ng3 + (int)(t % d.n3);
-    const int j = d.ng2 + (int)((t / d.n3) % d.n2);
-    const int i = d.ng1 + (int)(t / ((long)d.n3 * d.n2));
+    const Item3 it = item3(t, d.n3, d.n2);
+    const int z = d.ng3 + it.z;
+    const int j = d.ng2 + it.j;
+    const int i = d.ng1 + it.i;
     const long c = cix(d, i, j, z), gi = gix(d, i, j);
     Geo<double> gm;
     load_geo(d, m, i, j, CENT, gm);
@@ -1678,12 +1704,12 @@ __global__ void __launch_bounds__(BLK, HAMR_CONS_MINB) k_cons_cols(const Dims d,
     const long nzone = (long)d.n1 * d.n2 * d.n3;
     const long t0 = (long)blockIdx.x * blockDim.x;
     const long tl = (t0 + blockDim.x < nzone ? t0 + blockDim.x : nzone) - 1;
-    const long col0 = t0 / d.n3, ncol = tl / d.n3 - col0 + 1;   // <= 3 for n3 >= 64
+    const int col0 = (int)((unsigned)t0 / (unsigned)d.n3), ncol = (int)((unsigned)tl / (unsigned)d.n3) - col0 + 1;   // <= 3 for n3 >= 64
     const long gs = d.gs;
     for (int e = threadIdx.x; e < ncol * COL_VALS; e += blockDim.x) {
-        const long col = col0 + e / COL_VALS;
+        const int col = col0 + e / COL_VALS;
         const int v = e % COL_VALS;
-        const long gi = gix(d, d.ng1 + (int)(col / d.n2), d.ng2 + (int)(col % d.n2));
+        const long gi = gix(d, d.ng1 + col / d.n2, d.ng2 + col % d.n2);
         double x;
         if (v < 10) x = m.gcov[(long)(v * 5 + CENT) * gs + gi];
         else if (v < 20) x = m.gcon[(long)((v - 10) * 5 + CENT) * gs + gi];
@@ -1694,11 +1720,12 @@ __global__ void __launch_bounds__(BLK, HAMR_CONS_MINB) k_cons_cols(const Dims d,
     __syncthreads();
     const long t = t0 + threadIdx.x;
     if (t >= nzone) return;
-    const int z = d.ng3 + (int)(t % d.n3);
-    const int j = d.ng2 + (int)((t / d.n3) % d.n2);
-    const int i = d.ng1 + (int)(t / ((long)d.n3 * d.n2));
+    const Item3 it = item3(t, d.n3, d.n2);
+    const int z = d.ng3 + it.z;
+    const int j = d.ng2 + it.j;
+    const int i = d.ng1 + it.i;
     const long c = cix(d, i, j, z), gi = gix(d, i, j);
-    const double *g = sg[t / d.n3 - col0];
+    const double *g = sg[(unsigned)t / (unsigned)d.n3 - col0];
     Geo<double> gm;
 #pragma unroll
     for (int q = 0; q < 10; q++) { gm.gcov[q] = g[q]; gm.gcon[q] = g[10 + q]; }
@@ -1954,9 +1981,10 @@ __device__ __forceinline__ void k_invert_at(const Dims &d, const Geom &m, const 
                                                  const double *__restrict__ W, const double *__restrict__ psf,
                                                  double *__restrict__ pout, int *__restrict__ pflag,
                                                  int *__restrict__ failimage, const long t) {
-    const int z = d.ng3 + (int)(t % d.n3);
-    const int j = d.ng2 + (int)((t / d.n3) % d.n2);
-    const int i = d.ng1 + (int)(t / ((long)d.n3 * d.n2));
+    const Item3 it = item3(t, d.n3, d.n2);
+    const int z = d.ng3 + it.z;
+    const int j = d.ng2 + it.j;
+    const int i = d.ng1 + it.i;
     const long c = cix(d, i, j, z), gi = gix(d, i, j);
     Geo<double> gm;
     load_geo(d, m, i, j, CENT, gm);
@@ -1981,9 +2009,10 @@ __global__ void __launch_bounds__(BLK, HAMR_UPD_MINB)
                      int *__restrict__ failimage, int *__restrict__ flist, int *__restrict__ nfail) {
     const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= (long)d.n1 * d.n2 * d.n3) return;
-    const int z = d.ng3 + (int)(t % d.n3);
-    const int j = d.ng2 + (int)((t / d.n3) % d.n2);
-    const int i = d.ng1 + (int)(t / ((long)d.n3 * d.n2));
+    const Item3 it = item3(t, d.n3, d.n2);
+    const int z = d.ng3 + it.z;
+    const int j = d.ng2 + it.j;
+    const int i = d.ng1 + it.i;
     const long c = cix(d, i, j, z), gi = gix(d, i, j);
     Geo<double> gm;
     load_geo(d, m, i, j, CENT, gm);
@@ -2018,9 +2047,10 @@ __global__ void __launch_bounds__(BLK, HAMR_CONS_INV_MINB)
                int *__restrict__ failimage, int *__restrict__ flist, int *__restrict__ nfail) {
     const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= (long)d.n1 * d.n2 * d.n3) return;
-    const int z = d.ng3 + (int)(t % d.n3);
-    const int j = d.ng2 + (int)((t / d.n3) % d.n2);
-    const int i = d.ng1 + (int)(t / ((long)d.n3 * d.n2));
+    const Item3 it = item3(t, d.n3, d.n2);
+    const int z = d.ng3 + it.z;
+    const int j = d.ng2 + it.j;
+    const int i = d.ng1 + it.i;
     const long c = cix(d, i, j, z), gi = gix(d, i, j);
     Geo<double> gm;
     load_geo(d, m, i, j, CENT, gm);
@@ -2045,9 +2075,10 @@ __device__ __forceinline__ void invert_fallback_at(const Dims &d, const Geom &m,
                                                    const double *__restrict__ W, const double *__restrict__ psf,
                                                    double *__restrict__ pout, int *__restrict__ pflag,
                                                    int *__restrict__ failimage, const long t) {
-    const int z = d.ng3 + (int)(t % d.n3);
-    const int j = d.ng2 + (int)((t / d.n3) % d.n2);
-    const int i = d.ng1 + (int)(t / ((long)d.n3 * d.n2));
+    const Item3 it = item3(t, d.n3, d.n2);
+    const int z = d.ng3 + it.z;
+    const int j = d.ng2 + it.j;
+    const int i = d.ng1 + it.i;
     const long c = cix(d, i, j, z), gi = gix(d, i, j);
     Geo<double> gm;
     load_geo(d, m, i, j, CENT, gm);
@@ -2236,7 +2267,8 @@ __device__ __forceinline__ void copy_cell(const Dims &d, double *pv, long dst, l
 
 // x1 ghosts over every (j, z): periodic copy, or outflow copy + no-inflow
 __device__ __forceinline__ void k_bound_x1_at(const Dims &d, const Geom &m, double *pv, double *ps, const long t) {
-    const int z = (int)(t % d.G3), j = (int)((t / d.G3) % d.G2), g = (int)(t / ((long)d.G3 * d.G2));
+    const Item3 it = item3(t, d.G3, d.G2);
+    const int z = it.z, j = it.j, g = it.i;
     const int ilo = g, ihi = d.n1 + d.ng1 + g;
     const long ks = d.ks;
     if (d.bc1 == HAMR_BC_PERIODIC) {
@@ -2288,9 +2320,9 @@ constexpr int X3_COMPS = NPR + 3;
 __host__ __device__ __forceinline__ long n_bound_x3(const Dims &d) { return (long)X3_COMPS * d.ng3 * d.G1 * d.G2; }
 
 __device__ __forceinline__ void k_bound_x3_at(const Dims &d, double *pv, double *ps, const long t) {
-    const int g = (int)(t % d.ng3);
-    const long r = t / d.ng3;
-    const int j = (int)(r % d.G2), i = (int)((r / d.G2) % d.G1), comp = (int)(r / ((long)d.G2 * d.G1));
+    const int g = (int)((unsigned)t % (unsigned)d.ng3);
+    const Item3 it = item3((unsigned)t / (unsigned)d.ng3, d.G2, d.G1);
+    const int j = it.z, i = it.j, comp = it.i;
     double *a = comp < NPR ? pv + (long)comp * d.ks : ps + (long)(comp - NPR) * d.ks;
     a[cix(d, i, j, g)] = a[cix(d, i, j, g + d.n3)];
     a[cix(d, i, j, d.n3 + d.ng3 + g)] = a[cix(d, i, j, d.ng3 + g)];
@@ -2312,7 +2344,8 @@ constexpr int X2_COMPS = NPR + 3;
 __host__ __device__ __forceinline__ long n_bound_x2(const Dims &d) { return (long)X2_COMPS * d.G1 * d.G3; }
 
 __device__ __forceinline__ void k_bound_x2_at(const Dims &d, double *pv, double *ps, const long t) {
-    const int z = (int)(t % d.G3), i = (int)((t / d.G3) % d.G1), comp = (int)(t / ((long)d.G3 * d.G1));
+    const Item3 it = item3(t, d.G3, d.G1);
+    const int z = it.z, i = it.j, comp = it.i;
     const int n2 = d.n2, ng = d.ng2;
     const bool face = comp >= NPR;
     const int k = face ? comp - NPR : comp;
@@ -2455,9 +2488,10 @@ __global__ void k_divb(const Dims d, const Geom m, const double *ps, unsigned lo
     const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
     double v = 0.;
     if (t < (long)d.n1 * d.n2 * d.n3) {
-        const int z = d.ng3 + (int)(t % d.n3);
-        const int j = d.ng2 + (int)((t / d.n3) % d.n2);
-        const int i = d.ng1 + (int)(t / ((long)d.n3 * d.n2));
+        const Item3 it = item3(t, d.n3, d.n2);
+        const int z = d.ng3 + it.z;
+        const int j = d.ng2 + it.j;
+        const int i = d.ng1 + it.i;
         const long c = cix(d, i, j, z), ks = d.ks;
         double divb = 0.;
         if (d.d1) divb += 0.25 * (ps[0 * ks + c + (long)d.G2 * d.G3] * m.gdet[FACE1 * d.gs + gix(d, i + 1, j)] - ps[0 * ks + c] * m.gdet[FACE1 * d.gs + gix(d, i, j)]) / d.dx1;
