@@ -390,7 +390,7 @@ __device__ __forceinline__ void grid_barrier(unsigned *bar, int *kerr) {
     __syncthreads();
 }
 
-constexpr int PERSIST_MINB = HAMR_FLUX_MINB;   // the FP64 flux phases' budget
+constexpr int PERSIST_MINB = 5;   // a compromise between the phases' budgets
 
 template <typename T>
 __global__ void __launch_bounds__(BLK, PERSIST_MINB)

@@ -211,7 +211,7 @@ struct StepSize {
 // build options: minimum resident blocks of 128 threads per SM for the
 // double and float flux kernels (caps their registers per thread)
 #ifndef HAMR_FLUX_MINB
-#define HAMR_FLUX_MINB 5
+#define HAMR_FLUX_MINB 4
 #endif
 #ifndef HAMR_FLUX_MINB_F
 #define HAMR_FLUX_MINB_F 6
@@ -493,7 +493,7 @@ __host__ __device__ __forceinline__ long n_x3_slots(const Dims &d) {
 #define HAMR_FLUX_FT_X3_MINB_F 7
 #endif
 #ifndef HAMR_FLUX_X3_MINB
-#define HAMR_FLUX_X3_MINB 5
+#define HAMR_FLUX_X3_MINB 4
 #endif
 #ifndef HAMR_FLUX_X3_MINB_F
 #define HAMR_FLUX_X3_MINB_F 10
@@ -1828,29 +1828,34 @@ __host__ __device__ __forceinline__ ConsTmaLayout cons_tma_layout(int lpiece) {
     return L;
 }
 
-// build option: resident CTAs per SM of the TMA-staged update (caps its
-// registers; measured on the 384 x 192 x 192 torus, per step: float 3 (2.86
-// ms; 2: 4.05, 4: 2.88), double 4 (3.67 ms; 2: 4.05, 3: 3.86))
+// FUSE: 0 writes the planes of W for the inversion kernels; HAMR_INV_2D + 1 or
+// HAMR_INV_NM + 1 runs the primary inversion of each zone right after its
+// update (no floors or repair): the guess is pb (the state the update read),
+// the face field psf, the output pout, and only a zone whose primary solver
+// fails writes W and goes to the list for k_invert_fallback (*nfail cleared
+// before the launch). The W round trip and the inversion's reload of the guess
+// disappear; same values as the update followed by k_invert_primary.
+//
+// Resident CTAs of 256 threads per SM, which cap the registers (4: 64, 3: 80,
+// 2: 128). Per step, update with inversion, 384 x 192 x 192 torus (CTAs of 192
+// threads): FP64 3 3.09 ms, 2 3.85, 4 3.32; float 4 3.14, 3 3.19, 2 3.18.
+// Rows of at most 128 zones have CTAs small enough that the register file
+// still holds many at looser caps: 192 x 96 x 64 FP64 2 0.305 ms, 3 0.330, 4
+// 0.367; 131 x 77 x 50 float 2 and 3 0.171, 4 0.184. The update alone (FUSE 0):
+// float 3, FP64 4 (before the magnetic components left it: 2.86 ms against 2.88
+// at 4, and 3.67 against 3.86 at 3).
 #ifndef HAMR_CONS_TMA_MINB_F
 #define HAMR_CONS_TMA_MINB_F 3
 #endif
 #ifndef HAMR_CONS_TMA_MINB
 #define HAMR_CONS_TMA_MINB 4
 #endif
-// FUSE: 0 writes the seven planes of W for the inversion kernels; HAMR_INV_2D
-// + 1 or HAMR_INV_NM + 1 runs the primary inversion of each zone right after
-// its update (no floors or repair): the guess is pb (the state the update
-// read), the face field psf, the output pout, and only a zone whose primary
-// solver fails writes W and goes to the list for k_invert_fallback (*nfail
-// cleared before the launch). The W round trip and the inversion's reload of
-// the guess disappear; same values as the update followed by
-// k_invert_primary.
-#ifndef HAMR_CONS_INV_TMA_MINB   // the same kernel with the primary inversion inside (FUSE != 0);
-#define HAMR_CONS_INV_TMA_MINB 3    // FP64 at 4 blocks spills 0.6 KB a thread (measured C3 update+inversion
-#endif                              // 5.35 ms at 3 blocks, 6.0 at 4, 5.43 at 2)
-#ifndef HAMR_CONS_INV_TMA_MINB_F
-#define HAMR_CONS_INV_TMA_MINB_F HAMR_CONS_TMA_MINB_F
-#endif
+constexpr int CONS_SHORT_ROW = 128;
+template <typename T>
+__host__ __device__ constexpr int cons_tma_minb(int fuse, bool short_rows) {
+    return fuse == 0 ? (sizeof(T) == 8 ? HAMR_CONS_TMA_MINB : HAMR_CONS_TMA_MINB_F)
+                     : (sizeof(T) == 8 ? (short_rows ? 2 : 3) : (short_rows ? 3 : 4));
+}
 // The body of one CTA: row piece `blk` (row * npiece + piece) of the block,
 // `smem` the CTA's dynamic shared memory (cons_tma_layout(lpiece).total bytes).
 template <typename T, int FUSE>
@@ -1962,9 +1967,8 @@ __device__ __forceinline__ void cons_tma_row(const Dims &d, const Geom &m, const
     }
 }
 
-template <typename T, int FUSE = 0>
-__global__ void __launch_bounds__(256, sizeof(T) == 8 ? (FUSE ? HAMR_CONS_INV_TMA_MINB : HAMR_CONS_TMA_MINB)
-                                                       : (FUSE ? HAMR_CONS_INV_TMA_MINB_F : HAMR_CONS_TMA_MINB_F))
+template <typename T, int FUSE = 0, int MINB = cons_tma_minb<T>(0, false)>
+__global__ void __launch_bounds__(256, MINB)
     k_cons_tma(const Dims d, const Geom m, const double *__restrict__ pin, const double *__restrict__ pb,
                double *__restrict__ Ucache, const T *__restrict__ F1, const T *__restrict__ F2,
                const T *__restrict__ F3, double *__restrict__ W, int full, StepSize st, int *__restrict__ nfail,
@@ -2686,6 +2690,20 @@ void launch_flux(long n, cudaStream_t s, const Dims &d, const Geom &m, const dou
     }
 }
 
+// the TMA-staged update's shared memory for rows of up to 256 zones (as the
+// launch picks the kernel: short rows and long ones)
+template <typename T>
+void cons_tma_attributes() {
+    constexpr int S = cons_tma_minb<T>(1, true), L = cons_tma_minb<T>(1, false);
+    const int all = cons_tma_layout<T>(256).total, few = cons_tma_layout<T>(CONS_SHORT_ROW).total;
+    auto set = [](auto *k, int bytes) { cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes); };
+    set(k_cons_tma<T>, all);
+    set(k_cons_tma<T, HAMR_INV_2D + 1, L>, all);
+    set(k_cons_tma<T, HAMR_INV_NM + 1, L>, all);
+    set(k_cons_tma<T, HAMR_INV_2D + 1, S>, few);
+    set(k_cons_tma<T, HAMR_INV_NM + 1, S>, few);
+}
+
 // fluxes of both directions and centre EMFs of a 2-D block (k_flux_2d)
 template <typename T>
 void launch_flux_2d(cudaStream_t s, const Dims &d, const Geom &m, const double *pin, const double *psin, T *F1, T *F2,
@@ -2840,7 +2858,10 @@ int launch_stage_t(hamr_ctx *ctx, int full, StepSize st, bool calc_dt, Prof *pf,
             const size_t sm = cons_tma_layout<T>(lpiece).total;
             if (fuse) {
                 CK(cudaMemsetAsync(ctx->nfail, 0, sizeof(int), s));
-                auto kf = nm ? k_cons_tma<T, HAMR_INV_NM + 1> : k_cons_tma<T, HAMR_INV_2D + 1>;
+                constexpr int S = cons_tma_minb<T>(1, true), L = cons_tma_minb<T>(1, false);
+                auto kf = lpiece <= CONS_SHORT_ROW
+                              ? (nm ? k_cons_tma<T, HAMR_INV_NM + 1, S> : k_cons_tma<T, HAMR_INV_2D + 1, S>)
+                              : (nm ? k_cons_tma<T, HAMR_INV_NM + 1, L> : k_cons_tma<T, HAMR_INV_2D + 1, L>);
                 kf<<<grid, block, sm, s>>>(d, m, ctx->p, pg, ctx->U, F1, F2, F3, ctx->W, full, st, ctx->nfail,
                                            ctx->kerr, npiece, lpiece, psf, pout, ctx->pflag, ctx->failimage,
                                            ctx->flist);
@@ -3030,19 +3051,8 @@ int hamr_ctx_create(const hamr_params *prm, hamr_ctx **out) {
         cudaMemsetAsync(*a.p, 0, a.n, ctx->stream);
     }
     k_dt_reset<<<1, 32, 0, ctx->stream>>>(ctx->dtbits);
-    // the TMA-staged update's shared memory for rows of up to 256 zones
-    cudaFuncSetAttribute(k_cons_tma<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         cons_tma_layout<double>(256).total);
-    cudaFuncSetAttribute(k_cons_tma<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         cons_tma_layout<float>(256).total);
-    cudaFuncSetAttribute(k_cons_tma<double, HAMR_INV_2D + 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         cons_tma_layout<double>(256).total);
-    cudaFuncSetAttribute(k_cons_tma<double, HAMR_INV_NM + 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         cons_tma_layout<double>(256).total);
-    cudaFuncSetAttribute(k_cons_tma<float, HAMR_INV_2D + 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         cons_tma_layout<float>(256).total);
-    cudaFuncSetAttribute(k_cons_tma<float, HAMR_INV_NM + 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         cons_tma_layout<float>(256).total);
+    cons_tma_attributes<double>();
+    cons_tma_attributes<float>();
     if (cudaStreamSynchronize(ctx->stream) != cudaSuccess) {
         hamr_ctx_destroy(ctx);
         return HAMR_E_CUDA;
