@@ -76,9 +76,11 @@ struct Geom {
 // warp share a column wherever phi runs long, so a block is four or eight
 // 16-byte loads, each one transaction for the warp, where the planes above
 // take an address and a load per component (and in the mixed step a
-// conversion). Block (loc, column) at (loc * gs + column) * GT.
-constexpr int GT = 32;
-enum { GT_COV = 0, GT_G = 10, GT_RLAPSE = 11, GT_CON0 = 12, GT_CON = 13, GT_LAPSE = 22 };   // g^tt, then the other nine
+// conversion). Block (loc, column) at (loc * gs + column) * GT<T>: the 24 values
+// in double (two lines), a whole line in float.
+template <typename T>
+constexpr int GT = sizeof(T) == sizeof(double) ? 24 : 32;
+enum { GT_COV = 0, GT_G = 10, GT_RLAPSE = 11, GT_CON0 = 12, GT_CON = 13, GT_LAPSE = 22, GT_AL = 23 };   // g^tt, then the other nine
 
 // Blocks pay where the lanes of a warp read few columns: n3 of half a warp.
 // On 2-D blocks, where every lane has a column of its own, the planes'
@@ -86,19 +88,19 @@ enum { GT_COV = 0, GT_G = 10, GT_RLAPSE = 11, GT_CON0 = 12, GT_CON = 13, GT_LAPS
 constexpr int GEO_TAB_MIN_N3 = 16;
 __host__ __device__ __forceinline__ bool geo_tab_wanted(int n3) { return n3 >= GEO_TAB_MIN_N3; }
 
-__device__ __forceinline__ void load16(const double *p, double *o) {
+__device__ __forceinline__ void load8(const double *p, double *o) {
     const double2 *q = reinterpret_cast<const double2 *>(p);
 #pragma unroll
-    for (int k = 0; k < 8; k++) {
+    for (int k = 0; k < 4; k++) {
         const double2 v = __ldg(q + k);
         o[2 * k] = v.x;
         o[2 * k + 1] = v.y;
     }
 }
-__device__ __forceinline__ void load16(const float *p, float *o) {
+__device__ __forceinline__ void load8(const float *p, float *o) {
     const float4 *q = reinterpret_cast<const float4 *>(p);
 #pragma unroll
-    for (int k = 0; k < 4; k++) {
+    for (int k = 0; k < 2; k++) {
         const float4 v = __ldg(q + k);
         o[4 * k] = v.x;
         o[4 * k + 1] = v.y;
@@ -110,9 +112,9 @@ __device__ __forceinline__ void load16(const float *p, float *o) {
 // metric of a block of the point-by-point table
 template <typename T>
 __device__ __forceinline__ void load_geo_block(const T *q, Geo<T> &o) {
-    T v[GT];
-    load16(q, v);
-    load16(q + 16, v + 16);   // what of it is not used is not loaded
+    T v[24];
+#pragma unroll
+    for (int k = 0; k < 24; k += 8) load8(q + k, v + k);   // what of it is not used is not loaded
 #pragma unroll
     for (int s = 0; s < 10; s++) o.gcov[s] = v[GT_COV + s];
     o.g = v[GT_G];
@@ -121,6 +123,7 @@ __device__ __forceinline__ void load_geo_block(const T *q, Geo<T> &o) {
 #pragma unroll
     for (int s = 1; s < 10; s++) o.gcon[s] = v[GT_CON + s - 1];
     o.lapse = v[GT_LAPSE];
+    o.al = v[GT_AL];
 }
 
 // Item t of an (i, j, z) range, z fastest: t = (i nj + j) nz + z. In 32 bits:
@@ -143,7 +146,7 @@ __device__ __forceinline__ long gix(const Dims &d, int i, int j) { return (long)
 __device__ __forceinline__ void load_geo(const Dims &d, const Geom &m, int i, int j, int loc, Geo<double> &o) {
     long idx = gix(d, i, j);
     if (m.gtab) {
-        load_geo_block(m.gtab + ((long)loc * d.gs + idx) * GT, o);
+        load_geo_block(m.gtab + ((long)loc * d.gs + idx) * GT<double>, o);
         return;
     }
 #pragma unroll
@@ -178,7 +181,7 @@ __device__ __forceinline__ void load_geo_t(const Dims &d, const Geom &m, int i, 
     if constexpr (sizeof(T) == sizeof(double)) tab = m.gtab;
     else tab = m.gtabf;
     if (tab) {
-        load_geo_block(tab + ((long)loc * d.gs + idx) * GT, o);
+        load_geo_block(tab + ((long)loc * d.gs + idx) * GT<T>, o);
         return;
     }
 #pragma unroll
@@ -191,7 +194,11 @@ __device__ __forceinline__ void load_geo_t(const Dims &d, const Geom &m, int i, 
         o.lapse = (T)__ldg(&m.itab[(long)(6 + loc) * d.gs + idx]);
         o.rlapse = (T)__ldg(&m.itab[(long)(11 + loc) * d.gs + idx]);
     } else {
-        geo_lapse(o);   // float: the lapse of the float metric, as before
+        geo_lapse(o);   // float: the lapse of the float metric
+        if (m.itab) {
+            o.al = (T)__ldg(&m.itab[(long)(6 + loc) * d.gs + idx]);
+            o.rlapse = (T)__ldg(&m.itab[(long)(11 + loc) * d.gs + idx]);
+        }
     }
 }
 
@@ -346,11 +353,12 @@ __device__ __forceinline__ double flux_eval(const Dims &d, const Geo<T> &gm, con
         const T cmax = d_max(d_max(T(0.), xl), xr);
         const T cmin = d_max(d_max(T(0.), -nl), -nr);
         // the HLL weights with sqrt(-g)
-        const T rg = gm.g * d_rcp(cmax + cmin + T(SMALL_D));
-        const T wl = cmax * rg, wr = cmin * rg, wu = cmax * wr;
+        const T rg = mul(gm.g, d_rcp(cmax + cmin + T(SMALL_D)));
+        const T wl = mul(cmax, rg), wr = mul(cmin, rg), wu = mul(-cmax, wr);
 #pragma unroll
         for (int k = 0; k < NPR; k++)
-            if (k != B1 + DIR - 1 && k != drop) F[(long)k * d.ks + c] = wl * Fl[k] + wr * Fr[k] - wu * (Ur[k] - Ul[k]);
+            if (k != B1 + DIR - 1 && k != drop)
+                F[(long)k * d.ks + c] = mad(wl, Fl[k], mad(wr, Fr[k], mul(wu, Ur[k] - Ul[k])));
         return ctop_term(d, DIR, (double)d_max(cmax, cmin));
     }
     State<T> q;
@@ -1572,8 +1580,7 @@ __global__ void k_inv_tab(const Dims d, const double *__restrict__ gcon, const d
 
 // the point-by-point table from the planes and the column table: one thread
 // per column and location; every value is the one load_geo_t would form from
-// the planes (in float the converted component, and the lapse of the converted
-// metric)
+// the planes
 template <typename T>
 __global__ void k_geo_tab(const Dims d, const Geom m, T *__restrict__ tab) {
     const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1587,13 +1594,11 @@ __global__ void k_geo_tab(const Dims d, const Geom m, T *__restrict__ tab) {
         o.gcov[s] = (T)m.gcov[(long)(s * 5 + loc) * d.gs + idx];
     }
     o.g = (T)m.gdet[(long)loc * d.gs + idx];
-    if constexpr (sizeof(T) == sizeof(double)) {
-        o.lapse = m.itab[(long)(6 + loc) * d.gs + idx];
-        o.rlapse = m.itab[(long)(11 + loc) * d.gs + idx];
-    } else {
-        geo_lapse(o);
-    }
-    T *q = tab + t * GT;
+    geo_lapse(o);
+    if constexpr (sizeof(T) == sizeof(double)) o.lapse = m.itab[(long)(6 + loc) * d.gs + idx];
+    o.al = (T)m.itab[(long)(6 + loc) * d.gs + idx];
+    o.rlapse = (T)m.itab[(long)(11 + loc) * d.gs + idx];
+    T *q = tab + t * GT<T>;
     for (int s = 0; s < 10; s++) q[GT_COV + s] = o.gcov[s];
     q[GT_G] = o.g;
     q[GT_RLAPSE] = o.rlapse;
@@ -1700,6 +1705,7 @@ __global__ void __launch_bounds__(BLK, HAMR_CONS_MINB) k_cons_cols(const Dims d,
                                                double *__restrict__ W, int full, StepSize st,
                                                int *__restrict__ nfail) {
     __shared__ double sg[3][COL_VALS];
+    q[GT_AL] = o.al;
     if (blockIdx.x == 0 && threadIdx.x == 0) *nfail = 0;   // the inversion's failed-zone list starts empty
     const long nzone = (long)d.n1 * d.n2 * d.n3;
     const long t0 = (long)blockIdx.x * blockDim.x;
@@ -3032,8 +3038,8 @@ int hamr_ctx_create(const hamr_params *prm, hamr_ctx **out) {
         {(void **)&ctx->gcov, 50 * sizeof(double) * d.gs}, {(void **)&ctx->gcon, 50 * sizeof(double) * d.gs},
         {(void **)&ctx->gdet, 5 * sizeof(double) * d.gs}, {(void **)&ctx->conn, 40 * sizeof(double) * d.gs},
         {(void **)&ctx->itab, 16 * sizeof(double) * d.gs},
-        {(void **)&ctx->gtab, geo_tab_wanted(d.n3) && prm->precision == HAMR_FP64 ? 5 * GT * sizeof(double) * d.gs : 0},
-        {(void **)&ctx->gtabf, geo_tab_wanted(d.n3) && prm->precision == HAMR_MIXED ? 5 * GT * sizeof(float) * d.gs : 0},
+        {(void **)&ctx->gtab, geo_tab_wanted(d.n3) && prm->precision == HAMR_FP64 ? 5 * GT<double> * sizeof(double) * d.gs : 0},
+        {(void **)&ctx->gtabf, geo_tab_wanted(d.n3) && prm->precision == HAMR_MIXED ? 5 * GT<float> * sizeof(float) * d.gs : 0},
         {(void **)&ctx->dtbits, 4 * sizeof(unsigned long long)}, {(void **)&ctx->ndt, sizeof(double)},
         {(void **)&ctx->dt_state, sizeof(double)}, {(void **)&ctx->counter, sizeof(int)},
         {(void **)&ctx->divb, sizeof(unsigned long long)},

@@ -47,10 +47,21 @@ constexpr bool STRICT = true;
 constexpr bool STRICT = false;
 #endif
 
+// a b + c as one fused operation, and a b on its own, in the production build:
+// whatever the compiler would contract where it inlines a formula, kernels that
+// share it agree to the last bit (a block alone and in an ensemble). The strict
+// build, compiled without contraction, has no choice to pin.
+__device__ __forceinline__ double mad(double a, double b, double c) { return STRICT ? a * b + c : fma(a, b, c); }
+__device__ __forceinline__ float mad(float a, float b, float c) { return STRICT ? a * b + c : fmaf(a, b, c); }
+__device__ __forceinline__ double mul(double a, double b) { return STRICT ? a * b : __dmul_rn(a, b); }
+__device__ __forceinline__ float mul(float a, float b) { return STRICT ? a * b : __fmul_rn(a, b); }
+
 template <typename T>
 struct Geo {
     T gcov[10], gcon[10], g;
     T lapse, rlapse;   // 1/sqrt(-g^tt) and its reciprocal, each rounded once
+    T al;              // float only: the double lapse rounded once (lapse is the approximate
+                       // root of the converted g^tt, which the face-frame solvers keep)
 };
 
 // the lapse of a filled Geo, computed in place (ucon_calc's operations)
@@ -170,25 +181,26 @@ __device__ __forceinline__ double div_rcp_inf(double a, double b, double rb) {
 template <typename T>
 __device__ __forceinline__ void geo_lapse(Geo<T> &o) {
     o.lapse = T(1.) / d_sqrt(-o.gcon[0]);
-    o.rlapse = T(1.) / o.lapse;   // read by the double-precision quotients only
+    o.rlapse = T(1.) / o.lapse;   // not read by the float quotients
+    o.al = o.lapse;
 }
 
-// Quotients a_k / b that share one divisor: one reciprocal of b, then per
-// quotient a product (within 1.5 ulp, as accurate as the sums these quotients
-// enter), or in the strict build's double precision the exact form
-// (div_rcp_inf: the IEEE quotient bit for bit for 2^-900 <= |a| <= 2^900,
-// zeros and infinities). The adjoint's dual numbers divide as written.
+// Quotients a_k / b that share one divisor. In double precision: one reciprocal
+// of b, then per quotient a product (within 1.5 ulp, as accurate as the sums
+// these quotients enter), or in the strict build the exact form (div_rcp_inf:
+// the IEEE quotient bit for bit for 2^-900 <= |a| <= 2^900, zeros and
+// infinities). Other types (float, whose division is the approximate one, and
+// the adjoint's dual numbers) divide as written.
 template <typename T>
 struct Divisor {
     T b, rb;
     __device__ __forceinline__ explicit Divisor(T b_) : b(b_), rb(b_) {
-        if constexpr (std::is_floating_point<T>::value) rb = d_rcp(b_);
+        if constexpr (std::is_same<T, double>::value) rb = d_rcp(b_);
     }
     // with the divisor's reciprocal already at hand (rounded once, 1/b)
     __device__ __forceinline__ Divisor(T b_, T rb_) : b(b_), rb(rb_) {}
     __device__ __forceinline__ T div(T a) const {
-        if constexpr (std::is_same<T, double>::value && STRICT) return div_rcp_inf(a, b, rb);
-        else if constexpr (std::is_floating_point<T>::value) return a * rb;
+        if constexpr (std::is_same<T, double>::value) return STRICT ? div_rcp_inf(a, b, rb) : a * rb;
         else return a / b;
     }
 };
@@ -202,7 +214,7 @@ struct ExactDivisor {
     __device__ __forceinline__ explicit ExactDivisor(T b_) : b(b_), rb(T(1.0) / b_) {}
     __device__ __forceinline__ T div(T a) const {
         if constexpr (std::is_same<T, double>::value) return div_rcp_inf(a, b, rb);
-        else return a * rb;
+        else return a / b;
     }
 };
 
@@ -244,14 +256,48 @@ __device__ __forceinline__ void ucon_calc(const T *pr, const Geo<G> &gm, T *ucon
     G beta[4];
     T gamma;
     gamma_calc(pr, gm, &gamma);
-    if constexpr (std::is_same<T, G>::value && !STRICT) {
-        // beta^j / alpha = alpha g^tj: no division is left
-        ucon[0] = gamma * gm.rlapse;
-#pragma unroll
-        for (int j = 1; j < 4; j++) ucon[j] = pr[U1 + j - 1] - gamma * (gm.gcon[j] * alpha);
+    if constexpr (std::is_same<T, double>::value && std::is_same<T, G>::value && !STRICT) {
+        ucon_hll(pr, gm, ucon);   // with the lapse and its reciprocal
         return;
     }
 #pragma unroll
+// u_mu, dot product, u^mu and b^mu of the HLL sides and the centre EMFs in both
+// precisions: fused sums, u~^i u~_i nested, one reciprocal and no division
+// (beta^j / alpha = alpha g^tj). The float face-frame solvers, whose star states
+// amplify a changed last bit a thousandfold, keep the forms below.
+template <typename T>
+__device__ __forceinline__ void lower_hll(const T *u, const T *g, T *o) {
+    o[0] = mad(g[3], u[3], mad(g[2], u[2], mad(g[1], u[1], mul(g[0], u[0]))));
+    o[1] = mad(g[6], u[3], mad(g[5], u[2], mad(g[4], u[1], mul(g[1], u[0]))));
+    o[2] = mad(g[8], u[3], mad(g[7], u[2], mad(g[5], u[1], mul(g[2], u[0]))));
+    o[3] = mad(g[9], u[3], mad(g[8], u[2], mad(g[6], u[1], mul(g[3], u[0]))));
+}
+template <typename T>
+__device__ __forceinline__ T dot_hll(const T *a, const T *b) {
+    return mad(a[3], b[3], mad(a[2], b[2], mad(a[1], b[1], mul(a[0], b[0]))));
+}
+template <typename T>
+__device__ __forceinline__ void ucon_hll(const T *pr, const Geo<T> &gm, T *ucon) {
+    const T *g = gm.gcov;
+    const T u1 = pr[U1], u2 = pr[U2], u3 = pr[U3];
+    const T q1 = mad(g[4], u1, mul(T(2.), mad(g[5], u2, mul(g[6], u3))));
+    const T q2 = mad(g[7], u2, mul(T(2.), mul(g[8], u3)));
+    const T qsq = mad(u1, q1, mad(u2, q2, mul(mul(g[9], u3), u3)));
+    // clamped as gamma_calc: 1 where it is negative beyond rounding
+    const T gamma = qsq < T(-1.E-10) ? T(1.) : d_sqrt(T(1.) + (qsq < T(0.) ? T(1.E-10) : qsq));
+    const T alpha = sizeof(T) == sizeof(double) ? gm.lapse : gm.al;
+    ucon[0] = mul(gamma, gm.rlapse);
+#pragma unroll
+    for (int j = 1; j < 4; j++) ucon[j] = mad(-gamma, mul(gm.gcon[j], alpha), pr[U1 + j - 1]);
+}
+template <typename T>
+__device__ __forceinline__ void bcon_hll(const T *pr, const T *ucon, const T *ucov, T *bcon) {
+    bcon[0] = mad(pr[B3], ucov[3], mad(pr[B2], ucov[2], mul(pr[B1], ucov[1])));
+    const T ru = d_rcp(ucon[0]);
+#pragma unroll
+    for (int j = 1; j < 4; j++) bcon[j] = mul(mad(bcon[0], ucon[j], pr[B1 - 1 + j]), ru);
+}
+
     for (int j = 1; j < 4; j++) beta[j] = gm.gcon[j] * alpha * alpha;
     if constexpr (std::is_same<T, G>::value) {
         const Divisor<T> da(alpha, gm.rlapse);   // four quotients by the lapse
@@ -348,52 +394,57 @@ __device__ __forceinline__ void primtoflux(T gam, const T *pr, const State<T> &q
 // directions in one, sharing what they share, and with
 //   b^i u^t - b^t u^i = B^i                 (the conserved field)
 //   c_s^2 + v_A^2 - c_s^2 v_A^2 = (gamma P + b^2) / (w + b^2)
-// and the halved quadratic for the speeds. The normal field's flux is zero and
-// left out.
+//   (w + b^2) u_t + rho = rho (1 + u_t) + (gamma u + b^2) u_t
+// the last because the energy row carries the rest-mass flux, which cancels
+// most of it: 1 + u_t is formed first, without the rounding of either, and the
+// halved quadratic for the speeds. The normal field's flux is zero and left
+// out.
 template <int DIR, typename T>
 __device__ __forceinline__ void hll_side(T gam, const T *pr, const Geo<T> &gm, T *F, T *U, T &vmax, T &vmin) {
     T u[4], ul[4], b[4], bl[4];
-    ucon_calc(pr, gm, u);
-    lower4(u, gm.gcov, ul);
-    bcon_calc(pr, u, ul, b);
-    lower4(b, gm.gcov, bl);
-    const T P = (gam - T(1.)) * pr[UU], gP = gam * P;
-    const T bsq = dot4(b, bl);
-    const T eta = pr[RHO] + gam * pr[UU] + bsq;
-    const T ptot = P + T(0.5) * bsq;
-    const T ent = P * d_pow(pr[RHO], -gam);
-    F[RHO] = pr[RHO] * u[DIR];
-    U[RHO] = pr[RHO] * u[0];
-    F[KTOT] = F[RHO] * ent;
-    U[KTOT] = U[RHO] * ent;
-    const T ed = eta * u[DIR], e0 = eta * u[0];
+    ucon_hll(pr, gm, u);
+    lower_hll(u, gm.gcov, ul);
+    bcon_hll(pr, u, ul, b);
+    lower_hll(b, gm.gcov, bl);
+    const T rho = pr[RHO];
+    const T P = mul(gam - T(1.), pr[UU]);
+    const T bsq = dot_hll(b, bl);
+    const T gub = mad(gam, pr[UU], bsq), eta = rho + gub;
+    const T ptot = mad(T(0.5), bsq, P);
+    const T ent = mul(P, d_pow(rho, -gam));
+    F[RHO] = mul(rho, u[DIR]);
+    U[RHO] = mul(rho, u[0]);
+    F[KTOT] = mul(F[RHO], ent);
+    U[KTOT] = mul(U[RHO], ent);
+    const T et = mad(rho, T(1.) + ul[0], mul(gub, ul[0]));
+    F[UU] = mad(et, u[DIR], mul(-b[DIR], bl[0]));
+    U[UU] = mad(et, u[0], mul(-b[0], bl[0])) + ptot;
+    const T ed = mul(eta, u[DIR]), e0 = mul(eta, u[0]);
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-        F[UU + j] = ed * ul[j] - b[DIR] * bl[j];
-        U[UU + j] = e0 * ul[j] - b[0] * bl[j];
+    for (int j = 1; j < 4; j++) {
+        F[UU + j] = mad(ed, ul[j], mul(-b[DIR], bl[j]));
+        U[UU + j] = mad(e0, ul[j], mul(-b[0], bl[j]));
     }
     F[UU + DIR] += ptot;
-    F[UU] += F[RHO];
-    U[UU] += ptot + U[RHO];
 #pragma unroll
     for (int j = 1; j < 4; j++)
         if (j != DIR) {
-            F[B1 + j - 1] = b[j] * u[DIR] - b[DIR] * u[j];
+            F[B1 + j - 1] = mad(b[j], u[DIR], mul(-b[DIR], u[j]));
             U[B1 + j - 1] = pr[B1 + j - 1];
         }
-    T c2 = (gP + bsq) * d_rcp(eta);
+    T c2 = mul(mad(gam, P, bsq), d_rcp(eta));
     if (c2 < T(0.)) c2 = T(SMALL_D);
     if (c2 > T(1.)) c2 = T(1.);
     constexpr int sdd = DIR == 1 ? 4 : (DIR == 2 ? 7 : 9);
-    const T u02 = u[0] * u[0], u0d = u[0] * u[DIR], ud2 = u[DIR] * u[DIR];
-    const T A = u02 - (gm.gcon[0] + u02) * c2;
-    const T B = u0d - (gm.gcon[DIR] + u0d) * c2;
-    const T C = ud2 - (gm.gcon[sdd] + ud2) * c2;
-    T disc = B * B - A * C;
+    const T u02 = mul(u[0], u[0]), u0d = mul(u[0], u[DIR]), ud2 = mul(u[DIR], u[DIR]);
+    const T A = mad(-c2, gm.gcon[0] + u02, u02);
+    const T B = mad(-c2, gm.gcon[DIR] + u0d, u0d);
+    const T C = mad(-c2, gm.gcon[sdd] + ud2, ud2);
+    T disc = mad(B, B, mul(-A, C));
     if (disc < T(0.)) disc = T(0.);
     disc = d_sqrt(disc);
     const T rA = d_rcp(A);
-    const T vp = (B - disc) * rA, vm = (B + disc) * rA;
+    const T vp = mul(B - disc, rA), vm = mul(B + disc, rA);
     vmax = d_max(vp, vm);
     vmin = d_min(vp, vm);
 }
@@ -415,11 +466,12 @@ __device__ __forceinline__ T slope_lim(T y1, T y2, T y3) {
 // a / 6 for PPM's edge correction: in the strict build's double precision by
 // the exact reciprocal form (div_rcp; the IEEE quotient bit for bit for
 // 2^-900 <= |a| <= 2^900 and zeros, the range of differences of limited
-// slopes of the state), else a product
+// slopes of the state), in the production build's a product, else the type's
+// own division
 template <typename T>
 __device__ __forceinline__ T div6(T a) {
-    if constexpr (std::is_same<T, double>::value && STRICT) return div_rcp(a, 6.0, 1.0 / 6.0);
-    else return a * T(1.0 / 6.0);
+    if constexpr (std::is_same<T, double>::value) return STRICT ? div_rcp(a, 6.0, 1.0 / 6.0) : mul(a, 1.0 / 6.0);
+    else return a / T(6.0);
 }
 
 // x < 0 and x > 0 of a double from the bits of its upper word, so that the
@@ -454,16 +506,16 @@ __device__ __forceinline__ T ppm_slope(T y0, T y1, T y2) {
 }
 template <typename T>
 __device__ __forceinline__ T ppm_face(T y1, T y2, T dq1, T dq2) {
-    return T(0.5) * (y2 + y1) - div6(dq2 - dq1);
+    return mad(T(0.5), y2 + y1, -div6(dq2 - dq1));
 }
 template <typename T>
 __device__ __forceinline__ void ppm_limit(T y, T l, T r, T &lout, T &rout) {
     const T qa = (r - y) * (y - l);
     const T qd = (r - l);
-    const T qe = T(6.0) * (y - T(0.5) * (l + r));
+    const T qe = mul(T(6.0), mad(T(-0.5), l + r, y));
     if (qa <= T(0.)) { l = y; r = y; }
-    if (is_neg(qd * (qd - qe))) l = T(3.0) * y - T(2.0) * r;
-    else if (is_neg(qd * (qd + qe))) r = T(3.0) * y - T(2.0) * l;
+    if (is_neg(qd * (qd - qe))) l = mad(T(3.0), y, T(-2.0) * r);
+    else if (is_neg(qd * (qd + qe))) r = mad(T(3.0), y, T(-2.0) * l);
     lout = l;
     rout = r;
 }
