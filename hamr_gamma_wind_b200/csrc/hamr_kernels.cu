@@ -504,9 +504,31 @@ __host__ __device__ __forceinline__ long n_x3_slots(const Dims &d) {
 #define HAMR_FLUX_X3_MINB 4
 #endif
 #ifndef HAMR_FLUX_X3_MINB_F
-#define HAMR_FLUX_X3_MINB_F 10
+#define HAMR_FLUX_X3_MINB_F 9
 #endif
 
+// cell-centre EMF, -gdet (u x b), of a zone with primitives pb (velocities and
+// field) in column (i, j): e[0..2] = E1, E2, E3 (E1, E2 only in 3-D)
+template <typename T>
+__device__ __forceinline__ void emf_centre_of(const Dims &d, const Geom &m, const T *pb, int i, int j, T *e) {
+    Geo<T> gm;
+    load_geo_t(d, m, i, j, CENT, gm);
+    T ucon[4], ucov[4], bcon[4];
+    if constexpr (std::is_same<T, double>::value && STRICT) {
+        ucon_calc(pb, gm, ucon);
+        lower4(ucon, gm.gcov, ucov);
+        bcon_calc(pb, ucon, ucov, bcon);
+    } else {
+        ucon_hll(pb, gm, ucon);
+        lower_hll(ucon, gm.gcov, ucov);
+        bcon_hll(pb, ucon, ucov, bcon);
+    }
+    if (d.ng3 > 0) {
+        e[0] = -gm.g * mad(ucon[2], bcon[3], -mul(ucon[3], bcon[2]));
+        e[1] = -gm.g * mad(ucon[3], bcon[1], -mul(ucon[1], bcon[3]));
+    }
+    e[2] = -gm.g * mad(ucon[1], bcon[2], -mul(ucon[2], bcon[1]));
+}
 template <typename T>
 __device__ __forceinline__ void emf_centre_eval(const Dims &d, const Geom &m, const double *__restrict__ pv, int i,
                                                 int j, long c, T *e);
@@ -534,7 +556,7 @@ __device__ __forceinline__ double flux_x3_slots(const Dims &d, const Geom &m, co
     const int j = (d.ng2 - 1) * d.d2 + it.j;
     const int i = (d.ng1 - 1) * d.d1 + it.i;
     const long c = cix(d, i, j, d.ng3 - 1 - H + zl);   // the slot's zone
-    T hi[NPR];
+    T hi[NPR], y0[NK];   // upper edges; the zone's values (PPM)
     if constexpr (H == 0) {
         if (sl < nslot) {
             T lo[NPR];
@@ -544,7 +566,7 @@ __device__ __forceinline__ double flux_x3_slots(const Dims &d, const Geom &m, co
                 if (k != B3) sa[q++][l] = lo[k];
         }
     } else {
-        T y0[NK], y1[NK];
+        T y1[NK];
         if (sl < nslot) {
 #pragma unroll
             for (int k = 0, q = 0; k < NPR; k++) {
@@ -575,7 +597,14 @@ __device__ __forceinline__ double flux_x3_slots(const Dims &d, const Geom &m, co
     const bool mine = l >= H && (l < H + STEP || sl + 1 + H == nslot);
     if (Ec && mine && zl >= H && zl < rz - H && sl < nslot) {
         T e[3];
-        emf_centre_eval(d, m, pv, i, j, c, e);
+        if constexpr (H == 0) {
+            emf_centre_eval(d, m, pv, i, j, c, e);
+        } else {
+            T pb[NPR];
+#pragma unroll
+            for (int k = 0, q = 0; k < NPR; k++) pb[k] = k == B3 ? (T)__ldg(pv + (long)k * d.ks + c) : y0[q++];
+            emf_centre_of(d, m, pb, i, j, e);
+        }
         Ec[1 * d.ks + c] = e[0];
         Ec[2 * d.ks + c] = e[1];
         Ec[3 * d.ks + c] = e[2];
@@ -807,25 +836,13 @@ __global__ void k_fix_flux(const Dims d, T *F1, T *F2, T *F3) {
     if (t < n_fix_flux(d)) fix_flux_at(d, F1, F2, F3, t);
 }
 
-// cell-centre EMF, -gdet (u x b), of zone (i, j, z): e[0..2] = E1, E2, E3
-// (E1, E2 only in 3-D)
 template <typename T>
 __device__ __forceinline__ void emf_centre_eval(const Dims &d, const Geom &m, const double *__restrict__ pv, int i,
                                                 int j, long c, T *e) {
     T pb[NPR];
 #pragma unroll
-    for (int k = 0; k < NPR; k++) pb[k] = (T)__ldg(&pv[k * d.ks + c]);
-    Geo<T> gm;
-    load_geo_t(d, m, i, j, CENT, gm);
-    T ucon[4], ucov[4], bcon[4];
-    ucon_calc(pb, gm, ucon);
-    lower4(ucon, gm.gcov, ucov);
-    bcon_calc(pb, ucon, ucov, bcon);
-    if (d.ng3 > 0) {
-        e[0] = -gm.g * (ucon[2] * bcon[3] - ucon[3] * bcon[2]);
-        e[1] = -gm.g * (ucon[3] * bcon[1] - ucon[1] * bcon[3]);
-    }
-    e[2] = -gm.g * (ucon[1] * bcon[2] - ucon[2] * bcon[1]);
+    for (int k = U1; k <= B3; k++) pb[k] = (T)__ldg(&pv[k * d.ks + c]);
+    emf_centre_of(d, m, pb, i, j, e);
 }
 
 // on the active zones plus one ghost layer
