@@ -741,6 +741,9 @@ struct RowWindow {
     }
 };
 
+// brings the line at p into L1 (p: within an allocation)
+__device__ __forceinline__ void prefetch_l1(const void *p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
+
 // One row of FLUX_ROW faces along DIR (row t < n_flux_rows), reconstructed
 // through the thread's state in `wbuf` (a CTA's NV * NK * BLK values; column
 // threadIdx.x); returns the row's largest signal-speed contribution
@@ -749,6 +752,11 @@ template <int DIR, typename T, int REC>
 __device__ __forceinline__ double flux_row(const Dims &d, const Geom &m, const double *__restrict__ pv,
                                            const double *__restrict__ ps, T *__restrict__ F, T *wbuf, const long t) {
     using Win = RowWindow<DIR, T, REC>;
+    // A face's evaluation is long against its loads, but few warps are resident
+    // to hide them. Per step on the 384 x 192 x 192 torus: FP64 x2 2.19 -> 2.07
+    // ms, x1 2.15 -> 2.07; float x1 1.16 -> 1.05, x2 1.04 -> 1.06 (its rows, G3
+    // apart, are mostly in cache): not there
+    constexpr bool PREFETCH = sizeof(T) == 8 || DIR == 1;
     double cmx = 0.0;
     const int nt = DIR == 1 ? d.n2 + 2 * d.d2 : d.n1 + 2 * d.d1;
     const Item3 it = item3(t, d.n3 + 2 * d.d3, nt);
@@ -771,6 +779,21 @@ __device__ __forceinline__ double flux_row(const Dims &d, const Geom &m, const d
     int par = 1;
     for (int f = f0; f < f1; f++) {
         const int i = DIR == 1 ? f : a, j = DIR == 1 ? a : f;
+        // the next face's lines on their way while this one is evaluated
+        if (PREFETCH && f + 1 < f1) {
+#pragma unroll
+            for (int k = 0; k < NPR; k++)
+                if (k != B1 + DIR - 1) prefetch_l1(pv + (long)k * d.ks + c + (Win::H + 1) * stride);
+            prefetch_l1(ps + (long)(DIR - 1) * d.ks + c + stride);
+            const T *tab;
+            if constexpr (sizeof(T) == sizeof(double)) tab = m.gtab;
+            else tab = m.gtabf;
+            if (tab) {
+                const T *q = tab + ((long)face * d.gs + (DIR == 1 ? gix(d, f + 1, a) : gix(d, a, f + 1))) * GT<T>;
+                prefetch_l1(q);
+                if (sizeof(T) == 8) prefetch_l1(q + 16);
+            }
+        }
         win.edges(d, pv, c, stride, par, lo, hi);
         par ^= 1;
         Geo<T> gm;
@@ -3022,13 +3045,19 @@ int hamr_ctx_create(const hamr_params *prm, hamr_ctx **out) {
         ctx->own_stream = true;
     }
     {
-        // six waves of the row kernels' residency (blocks of 128 per SM: the
-        // FP64 and float register caps)
+        // a wave of the row kernels' residency (blocks of 128 per SM: the FP64
+        // and float register caps). x1 + x2 fluxes per step, rows against
+        // faces: 192 x 96 x 64 FP64 (1.45 waves of rows) 0.49 and 0.58 ms, 160
+        // x 96 x 128 float (1.3) 0.40 and 0.46; 131 x 77 x 50 float (0.4) 0.17
+        // and 0.15, 64^3 MC (0.35) 0.19 and 0.11. The face-frame solvers, whose
+        // evaluation dwarfs the reconstruction, take six: 192 x 96 x 64 HLLC in
+        // float (0.8) 0.54 and 0.47 ms; 2-D blocks too, where a warp's lanes lie
+        // a row of zones apart in one of the directions
         int dev = 0, nsm = 148;
         if (cudaGetDevice(&dev) == cudaSuccess)
             cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
         const int per_sm = prm->precision == HAMR_MIXED ? HAMR_FLUX_ROWS_MINB_F : HAMR_FLUX_ROWS_MINB;
-        ctx->rows_min = 6L * nsm * per_sm * BLK;
+        ctx->rows_min = (prm->riemann == HAMR_RIEMANN_HLL && d.d3 ? 1L : 6L) * nsm * per_sm * BLK;
         // tuning override (threads; 0: always by rows), read once per context
         if (const char *e = getenv("HAMR_FLUX_ROWS_MIN")) ctx->rows_min = atol(e);
         if (const char *e = getenv("HAMR_CONS_COLS")) ctx->cons_cols = atoi(e) != 0;
