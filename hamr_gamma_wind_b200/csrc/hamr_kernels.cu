@@ -1091,25 +1091,23 @@ __device__ __forceinline__ void face_update_eval(const Dims &d, const Geom &m, c
     const long ks = d.ks;
     if ((faces & 1) && i < d.n1 + d.ng1 + d.d1 && j < d.n2 + d.ng2 && z < d.n3 + d.ng3) {
         const double gdf = __ldg(&m.gdet[FACE1 * d.gs + gi]);
-        double temp = 0.;
-        temp += 1.0 / ((double)1) * psi[c] * gdf;
-        temp += div_rcp(-Dt, d.dx2, d.rdx2) * (E(3, 0, 1, 0) - E(3, 0, 0, 0));
-        if (d.ng3 > 0) temp += div_rcp(Dt, d.dx3, d.rdx3) * (E(2, 0, 0, 1) - E(2, 0, 0, 0));
+        double temp = psi[c] * gdf;
+        temp = mad(div_rcp(-Dt, d.dx2, d.rdx2), E(3, 0, 1, 0) - E(3, 0, 0, 0), temp);
+        if (d.ng3 > 0) temp = mad(div_rcp(Dt, d.dx3, d.rdx3), E(2, 0, 0, 1) - E(2, 0, 0, 0), temp);
         psf[c] = div_face_volume(d, m, temp, gdf, 3, gi);
     }
     if ((faces & 4) && d.ng3 > 0 && i < d.n1 + d.ng1 && j < d.n2 + d.ng2 && z < d.n3 + d.ng3 + d.d3) {
         const double gdf = __ldg(&m.gdet[FACE3 * d.gs + gi]);
         double temp = psi[2 * ks + c] * gdf;
-        temp += div_rcp(-Dt, d.dx1, d.rdx1) * (E(2, 1, 0, 0) - E(2, 0, 0, 0));
-        temp += div_rcp(Dt, d.dx2, d.rdx2) * (E(1, 0, 1, 0) - E(1, 0, 0, 0));
+        temp = mad(div_rcp(-Dt, d.dx1, d.rdx1), E(2, 1, 0, 0) - E(2, 0, 0, 0), temp);
+        temp = mad(div_rcp(Dt, d.dx2, d.rdx2), E(1, 0, 1, 0) - E(1, 0, 0, 0), temp);
         psf[2 * ks + c] = div_face_volume(d, m, temp, gdf, 5, gi);
     }
     if ((faces & 2) && i < d.n1 + d.ng1 && j < d.n2 + d.ng2 + d.d2 && z < d.n3 + d.ng3) {
         const double gdf = __ldg(&m.gdet[FACE2 * d.gs + gi]);
-        double temp = 0.;
-        temp += 1.0 / ((double)1) * psi[1 * ks + c] * gdf;
-        temp += div_rcp(Dt, d.dx1, d.rdx1) * (E(3, 1, 0, 0) - E(3, 0, 0, 0));
-        if (d.ng3 > 0) temp += div_rcp(-Dt, d.dx3, d.rdx3) * (E(1, 0, 0, 1) - E(1, 0, 0, 0));
+        double temp = psi[1 * ks + c] * gdf;
+        temp = mad(div_rcp(Dt, d.dx1, d.rdx1), E(3, 1, 0, 0) - E(3, 0, 0, 0), temp);
+        if (d.ng3 > 0) temp = mad(div_rcp(-Dt, d.dx3, d.rdx3), E(1, 0, 0, 1) - E(1, 0, 0, 0), temp);
         psf[1 * ks + c] = div_face_volume(d, m, temp, gdf, 4, gi);
     }
 }
@@ -1136,13 +1134,21 @@ __host__ __device__ __forceinline__ long n_face_threads(const Dims &d) {
     return (long)(d.n1 + d.d1) * (d.n2 + d.d2) * ((d.n3 + d.d3 + 1) / 2);
 }
 
-// Two consecutive z face triples per thread (ZP = 2), so that the edge-EMF
-// loads of both are in flight together; each triple is the one-item body.
-template <typename T, int ZP = 2>
-__global__ void __launch_bounds__(BLK) k_face_update(const Dims d, const Geom m, const double *psi, double *psf,
-                                                      const T *__restrict__ Et, StepSize st) {
+// Two consecutive z face triples per thread, so that the loads of both are in
+// flight together; bound by their latency. Float EMFs: the column's face volumes
+// and the step's quotients by the zone widths once, and every load of both
+// triples issued before the first store (the field may be updated in place, so
+// the compiler would not move the second triple's loads across it); 384 x 192 x
+// 192 torus, per step, 0.498 -> 0.448 ms at 6 blocks per SM (80 registers; 8:
+// 0.462, 5: 0.508). In FP64 that takes 91 registers, and the one-item body
+// twice, at 40, is the faster (0.450 against 0.49 ms at 5, 6 and 8 blocks); 2-D
+// blocks (one z) run it too.
+template <typename T>
+__global__ void __launch_bounds__(BLK, sizeof(T) == 8 ? 10 : 6) k_face_update(const Dims d, const Geom m,
+                                                      const double *psi, double *psf, const T *__restrict__ Et,
+                                                      StepSize st) {
     const int ni = d.n1 + d.d1, nj = d.n2 + d.d2, nz = d.n3 + d.d3;
-    const int nzp = (nz + ZP - 1) / ZP;
+    const int nzp = (nz + 1) / 2;
     const long u = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (u >= (long)ni * nj * nzp) return;
     const long row = (unsigned)u / (unsigned)nzp;
@@ -2848,7 +2854,7 @@ int launch_stage_t(hamr_ctx *ctx, int full, StepSize st, bool calc_dt, Prof *pf,
         prof_mark(pf, PROF_EMF_EDGE, s);
         prof_mark(pf, PROF_POLE_AVG, s);
         k_ct_2d<T><<<nblk((long)(d.n1 + d.d1) * (d.n2 + d.d2)), BLK, 0, s>>>(
-            d, m, ctx->ps, full ? ctx->ps : ctx->psh, Ec, F1, F2, st, ctx->nfail);
+            d, m, ctx->ps, full ? ctx->ps : ctx->psh, Ec, F1, F2, st);
         prof_mark(pf, PROF_FACE, s);
     } else if (d.d3 && ctx->ct_fused) {
         // centre EMFs, edge EMFs and the face update in one kernel (polar
