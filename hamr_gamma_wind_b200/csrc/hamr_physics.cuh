@@ -102,6 +102,14 @@ __device__ __forceinline__ double rcp_nr(double b) {
     const double r = fma(r0, fma(e, e, e), r0);
     return not_finite(r) ? r0 : r;
 }
+// the same where a zero or infinite operand needs no answer (its NaN is caught
+// by the caller)
+__device__ __forceinline__ double rcp_nr_finite(double b) {
+    double r0;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r0) : "d"(b));
+    const double e = fma(-b, r0, 1.0);
+    return fma(r0, fma(e, e, e), r0);
+}
 // sqrt(x) and 1/sqrt(x) of a positive normal x
 __device__ __forceinline__ double sqrt_nr_pos(double x, double &rs) {
     double r0;
@@ -176,6 +184,12 @@ __device__ __forceinline__ double div_rcp_inf(double a, double b, double rb) {
     const double r = fma(-q0, b, a);
     if constexpr (!STRICT) return not_finite(r) ? q0 : fma(r, rb, q0);
     return (r == 0.0 || !(fabs(r) <= 1.7976931348623157e308)) ? q0 : fma(r, rb, q0);
+}
+
+// the same where an infinite operand need not give the IEEE quotient (the
+// conserved variables of a zone: an infinite one fails the inversion either way)
+__device__ __forceinline__ double div_rcp_fin(double a, double b, double rb) {
+    return STRICT ? div_rcp_inf(a, b, rb) : div_rcp(a, b, rb);
 }
 
 template <typename T>
@@ -611,11 +625,11 @@ __device__ __forceinline__ void set_velocity(const InvQ &s, double gamma, double
 // the same with the divisions by gdet in the exact reciprocal form
 __device__ __forceinline__ int inv_prologue_k(const double *U, const InvK &k, double *prim, double *Ut) {
     if (U[0] <= 0.) return -100;
-    for (int i = B1; i <= B3; i++) prim[i] = div_rcp_inf(U[i], k.gdet, k.rgdet);
-    Ut[RHO] = div_rcp_inf(k.alpha * U[RHO], k.gdet, k.rgdet);
-    Ut[UU] = div_rcp_inf(k.alpha * (U[UU] - U[RHO]), k.gdet, k.rgdet);
-    for (int i = U1; i <= U3; i++) Ut[i] = div_rcp_inf(k.alpha * U[i], k.gdet, k.rgdet);
-    for (int i = B1; i <= B3; i++) Ut[i] = div_rcp_inf(k.alpha * U[i], k.gdet, k.rgdet);
+    for (int i = B1; i <= B3; i++) prim[i] = div_rcp_fin(U[i], k.gdet, k.rgdet);
+    Ut[RHO] = div_rcp_fin(k.alpha * U[RHO], k.gdet, k.rgdet);
+    Ut[UU] = div_rcp_fin(k.alpha * (U[UU] - U[RHO]), k.gdet, k.rgdet);
+    for (int i = U1; i <= U3; i++) Ut[i] = div_rcp_fin(k.alpha * U[i], k.gdet, k.rgdet);
+    for (int i = B1; i <= B3; i++) Ut[i] = div_rcp_fin(k.alpha * U[i], k.gdet, k.rgdet);
     return 0;
 }
 
@@ -670,6 +684,7 @@ __device__ __forceinline__ int utoprim_2d_k(const InvK &k, const double *U, cons
     double x1 = (vs > 1.) ? (1.0 - 1.e-15) : vs;
     // Newton iterations (general_newton_raphson, func_vsq)
     double f = 1., df = 1., errx = 1.;
+    bool converged = false;
     int n_iter = 0, i_extra = 0, doing_extra = 0, keep = 1;
     const double Bsq = s.Bsq, Qtsq = s.Qtsq, QdotBsq = s.QdotBsq, Qdotn = s.Qdotn, D = s.D;
     // 1/x0 of the current iterate: t23 of this iteration, and the divisor of
@@ -719,7 +734,7 @@ __device__ __forceinline__ int utoprim_2d_k(const InvK &k, const double *U, cons
             t18 = -Qdotn - 0.5 * Bsq * (1.0 + x1) + 0.5 * t16 - x0 + p_tmp;
             const double t25 = fma(kg, gtmp, -1.0) - t24;
             const double t35 = fma(t25, t3, fma(-2.0, dPdvsq, Bsq) * t40);
-            const double r = d_rcp(t3 * t35);
+            const double r = rcp_nr_finite(t3 * t35);
             dx0 = -fma(t2, t11, t4 * t18) * r;
             dx1 = fma(t25, t11, 2.0 * (t40 * t3) * t18) * r;
         }
@@ -732,17 +747,26 @@ __device__ __forceinline__ int utoprim_2d_k(const InvK &k, const double *U, cons
         x0 = (x0 > W_TOO_BIG) ? xo0 : x0;
         x1 = (x1 < 0.) ? 0. : x1;
         x1 = (x1 > 1.) ? (1. - 1.e-15) : x1;
-        rx0 = d_rcp(x0);
-        errx = (x0 == 0.) ? fabs(x0 - xo0) : fabs(div_rcp_inf(x0 - xo0, x0, rx0));
-        if ((fabs(errx) <= NEWT_TOL) && (doing_extra == 0) && (EXTRA_NEWT_ITER > 0)) doing_extra = 1;
+        if constexpr (STRICT) {
+            rx0 = 1. / x0;
+            errx = (x0 == 0.) ? fabs(x0 - xo0) : fabs(div_rcp_inf(x0 - xo0, x0, rx0));
+            converged = fabs(errx) <= NEWT_TOL;
+        } else {
+            // the same test without the quotient; an iterate of zero, which no
+            // root is, does not converge
+            rx0 = rcp_nr_finite(x0);
+            converged = fabs(x0 - xo0) <= NEWT_TOL * x0;
+        }
+        if (converged && (doing_extra == 0) && (EXTRA_NEWT_ITER > 0)) doing_extra = 1;
         if (doing_extra == 1) i_extra++;
-        if (((fabs(errx) <= NEWT_TOL) && (doing_extra == 0)) || (i_extra > EXTRA_NEWT_ITER) || (n_iter >= (MAX_NEWT_ITER - 1)))
+        if ((converged && (doing_extra == 0)) || (i_extra > EXTRA_NEWT_ITER) || (n_iter >= (MAX_NEWT_ITER - 1)))
             keep = 0;
         n_iter++;
     }
+    static_assert(MIN_NEWT_TOL >= NEWT_TOL, "one tolerance decides convergence");
     int retval = 0;
     if ((isfinite(f) == 0) || (isfinite(df) == 0)) retval = 2;
-    else if (fabs(errx) > d_min(NEWT_TOL, MIN_NEWT_TOL)) retval = 1;
+    else if (!converged) retval = 1;
     double W = x0, vsq = x1;
     if ((retval != 0) || (W == FAIL_VAL)) return retval * 100 + 1;
     if (W <= 0. || W > W_TOO_BIG) return 3;
@@ -767,12 +791,16 @@ __device__ __forceinline__ int utoprim_2d(double gam, const double *U, const dou
     return utoprim_2d_k(inv_consts(gam, 1.0 / gam, gdet, gcon), U, gcov, gcon, prim);
 }
 
+// a / b in the arithmetic of the build: the fallback's iterations are one zone's
+// dependent chain, a dozen of them with eight quotients and a power each
+__device__ __forceinline__ double quot(double a, double b) { return STRICT ? a / b : a * rcp_nr(b); }
+
 __device__ __forceinline__ double W_of_vsq2(double gam, double vsq, double *p, double *rho, double *u, double D, double K) {
     double gtmp = (1. - vsq);
-    *rho = D * sqrt(gtmp);
+    *rho = D * d_sqrt(gtmp);
     *p = K * d_pow(*rho, gam);
-    *u = *p / (gam - 1.);
-    return (*rho + *u + *p) / gtmp;
+    *u = quot(*p, gam - 1.);
+    return quot(*rho + *u + *p, gtmp);
 }
 
 // entropy-based 1D solve in v^2
@@ -790,14 +818,16 @@ __device__ __noinline__ int utoprim_1dvsq2fix1(double gam, const double *U, cons
     double x = 1. - 1. / gammasq;
     double f = 1., df = 1., errx = 1., W = 0., W_old;
     int n_iter = 0, i_extra = 0, doing_extra = 0, keep = 1;
+    // W(x) of the current iterate: the one formed for the convergence test of
+    // the iteration before
+    double Wc = W_of_vsq2(gam, x, &p, &rho, &u, s.D, K);
     while (keep) {
-        double Wc = W_of_vsq2(gam, x, &p, &rho, &u, s.D, K);
         double Wsq = Wc * Wc;
-        double dWdvsq = (gam * (2. - gam) * p + (gam - 1.) * rho) / (2. * (gam - 1.) * (1. - x) * (1. - x));
+        double dWdvsq = quot(gam * (2. - gam) * p + (gam - 1.) * rho, 2. * (gam - 1.) * (1. - x) * (1. - x));
         double fact_tmp = (s.Bsq + Wc);
-        double resid = s.Qtsq - x * fact_tmp * fact_tmp + s.QdotBsq * (s.Bsq + 2. * Wc) / Wsq;
-        double jac = -fact_tmp * (fact_tmp + 2. * dWdvsq * (x + s.QdotBsq / (Wc * Wsq)));
-        double dx = -resid / jac;
+        double resid = s.Qtsq - x * fact_tmp * fact_tmp + quot(s.QdotBsq * (s.Bsq + 2. * Wc), Wsq);
+        double jac = -fact_tmp * (fact_tmp + 2. * dWdvsq * (x + quot(s.QdotBsq, Wc * Wsq)));
+        double dx = quot(-resid, jac);
         f = 0.5 * resid * resid;
         df = -2. * f;
         double xo = x;
@@ -806,9 +836,9 @@ __device__ __noinline__ int utoprim_1dvsq2fix1(double gam, const double *U, cons
         x = (x < -1.e-10) ? (0.5 * xo) : x;
         x = fabs(x);
         W_old = W;
-        W = W_of_vsq2(gam, x, &p, &rho, &u, s.D, K);
-        errx = (W == 0.) ? fabs(W - W_old) : fabs((W - W_old) / W);
-        errx += (x == 0.) ? fabs(x - xo) : fabs((x - xo) / x);
+        W = Wc = W_of_vsq2(gam, x, &p, &rho, &u, s.D, K);
+        errx = (W == 0.) ? fabs(W - W_old) : fabs(quot(W - W_old, W));
+        errx += (x == 0.) ? fabs(x - xo) : fabs(quot(x - xo, x));
         if ((fabs(errx) <= NEWT_TOL) && (doing_extra == 0) && (EXTRA_NEWT_ITER > 0)) doing_extra = 1;
         if (doing_extra == 1) i_extra++;
         if (((fabs(errx) <= NEWT_TOL) && (doing_extra == 0)) || (i_extra > EXTRA_NEWT_ITER) || (n_iter >= (MAX_NEWT_ITER - 1)))
