@@ -1151,11 +1151,67 @@ __global__ void __launch_bounds__(BLK, sizeof(T) == 8 ? 10 : 6) k_face_update(co
     const int nzp = (nz + 1) / 2;
     const long u = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (u >= (long)ni * nj * nzp) return;
-    const long row = (unsigned)u / (unsigned)nzp;
-    const int z0 = (int)((unsigned)u % (unsigned)nzp) * ZP;
+    if (sizeof(T) == 8 || d.ng3 == 0) {
+        const long row = (unsigned)u / (unsigned)nzp;
+        const int z0 = (int)((unsigned)u % (unsigned)nzp) * 2;
 #pragma unroll
-    for (int q = 0; q < ZP; q++)
-        if (z0 + q < nz) k_face_update_at(d, m, psi, psf, Et, st, row * nz + z0 + q);
+        for (int q = 0; q < 2; q++)
+            if (z0 + q < nz) k_face_update_at(d, m, psi, psf, Et, st, row * nz + z0 + q);
+        return;
+    }
+    const Item3 it = item3(u, nzp, nj);
+    const int i = d.ng1 + it.i, j = d.ng2 + it.j, z = d.ng3 + 2 * it.z;
+    const long ks = d.ks, isize = (long)d.G2 * d.G3, c = cix(d, i, j, z), gi = gix(d, i, j);
+    const int nq = 2 * it.z + 1 < nz ? 2 : 1;
+    const bool in_i = i < d.n1 + d.ng1, in_j = j < d.n2 + d.ng2;   // an active zone's row, column
+    const double Dt = st.sub();
+    const T *E1 = Et + 1 * ks + c, *E2 = Et + 2 * ks + c, *E3 = Et + 3 * ks + c;
+    // the EMFs around both triples: _i, _j one zone up along x1, x2 (present
+    // in the ghosted block also beyond the last face)
+    T e1[3], e2[3], e3[2], e1j[2], e2i[2], e3i[2], e3j[2];
+    double p1[2], p2[2], p3[2];
+    e1[0] = E1[0];
+    e2[0] = E2[0];
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+        if (q >= nq) break;
+        e1[q + 1] = E1[q + 1];
+        e2[q + 1] = E2[q + 1];
+        e3[q] = E3[q];
+        e1j[q] = E1[q + d.G3];
+        e2i[q] = E2[q + isize];
+        e3i[q] = E3[q + isize];
+        e3j[q] = E3[q + d.G3];
+        p1[q] = psi[c + q];
+        p2[q] = psi[ks + c + q];
+        p3[q] = psi[2 * ks + c + q];
+    }
+    const double gd1 = __ldg(&m.gdet[FACE1 * d.gs + gi]), gd2 = __ldg(&m.gdet[FACE2 * d.gs + gi]),
+                 gd3 = __ldg(&m.gdet[FACE3 * d.gs + gi]);
+    const double w1 = div_rcp(Dt, d.dx1, d.rdx1), w2 = div_rcp(Dt, d.dx2, d.rdx2), w3 = div_rcp(Dt, d.dx3, d.rdx3);
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+        if (q >= nq) break;
+        const bool in_z = z + q < d.n3 + d.ng3;
+        if (in_j && in_z) {
+            double t = p1[q] * gd1;
+            t = mad(-w2, (double)e3j[q] - (double)e3[q], t);
+            t = mad(w3, (double)e2[q + 1] - (double)e2[q], t);
+            psf[c + q] = div_face_volume(d, m, t, gd1, 3, gi);
+        }
+        if (in_i && in_j) {
+            double t = p3[q] * gd3;
+            t = mad(-w1, (double)e2i[q] - (double)e2[q], t);
+            t = mad(w2, (double)e1j[q] - (double)e1[q], t);
+            psf[2 * ks + c + q] = div_face_volume(d, m, t, gd3, 5, gi);
+        }
+        if (in_i && in_z) {
+            double t = p2[q] * gd2;
+            t = mad(w1, (double)e3i[q] - (double)e3[q], t);
+            t = mad(-w3, (double)e1[q + 1] - (double)e1[q], t);
+            psf[1 * ks + c + q] = div_face_volume(d, m, t, gd2, 4, gi);
+        }
+    }
 }
 
 // Edge EMF and face update of a 2-D block in one launch: a thread evaluates
@@ -1651,6 +1707,7 @@ __global__ void k_geo_tab(const Dims d, const Geom m, T *__restrict__ tab) {
     q[GT_CON0] = o.gcon[0];
     for (int s = 1; s < 10; s++) q[GT_CON + s - 1] = o.gcon[s];
     q[GT_LAPSE] = o.lapse;
+    q[GT_AL] = o.al;
 }
 
 // primary solver: Noble 2D, or Newman-Hamlin in its place (NEWMAN builds)
@@ -1751,7 +1808,6 @@ __global__ void __launch_bounds__(BLK, HAMR_CONS_MINB) k_cons_cols(const Dims d,
                                                double *__restrict__ W, int full, StepSize st,
                                                int *__restrict__ nfail) {
     __shared__ double sg[3][COL_VALS];
-    q[GT_AL] = o.al;
     if (blockIdx.x == 0 && threadIdx.x == 0) *nfail = 0;   // the inversion's failed-zone list starts empty
     const long nzone = (long)d.n1 * d.n2 * d.n3;
     const long t0 = (long)blockIdx.x * blockDim.x;
