@@ -1055,7 +1055,6 @@ int afail(hamr_adjoint *a, cudaError_t e, const char *what) {
 
 // one RK2 step of the context with a fixed dt (no step-size bookkeeping)
 int fixed_step(hamr_ctx *ctx, double dt) {
-    k_dt_reset<<<1, 32, 0, ctx->stream>>>(ctx->dtbits);
     return launch_step(ctx, StepSize{nullptr, 0.5, 0.5 * dt, dt}, StepSize{nullptr, 1.0, dt, dt}, nullptr, 0);
 }
 

@@ -1217,15 +1217,13 @@ __global__ void __launch_bounds__(BLK, sizeof(T) == 8 ? 10 : 6) k_face_update(co
 // Edge EMF and face update of a 2-D block in one launch: a thread evaluates
 // the E3 of its zone's corner and of the two next to it, which its two faces
 // need (each corner three times over, a few loads from cache against a launch
-// and a round trip; 256 x 256 torus, per step, 0.036 -> 0.021 ms). It also
-// empties the inversion's failed-zone list. Same values as k_emf_edge and
-// k_face_update.
+// and a round trip; 256 x 256 torus, per step, 0.036 -> 0.021 ms). Same values
+// as k_emf_edge and k_face_update.
 template <typename T>
 __global__ void __launch_bounds__(BLK) k_ct_2d(const Dims d, const Geom m, const double *psi, double *psf,
                                                 const T *__restrict__ Ec, const T *__restrict__ F1,
-                                                const T *__restrict__ F2, StepSize st, int *__restrict__ nfail) {
+                                                const T *__restrict__ F2, StepSize st) {
     const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t == 0) *nfail = 0;
     const int nj = d.n2 + d.d2;
     if (t >= (long)(d.n1 + d.d1) * nj) return;
     const Item3 it = item3(t, nj, 1 << 30);
@@ -2138,15 +2136,13 @@ __global__ void __launch_bounds__(BLK, HAMR_UPD_MINB)
     invert_epilogue<FIX>(d, gm, c, flag, pf, pout, pflag, failimage);
 }
 
-// The conserved update and the primary inversion of small blocks in one
-// kernel, a zone per thread (the inversion's U[B] from the updated faces): one
-// launch, and the update's primitives are the inversion's guess (256 x 256
-// torus, per step with the fallback pass, 0.072 -> 0.053 ms; 64 x 64 box 0.055
-// -> 0.041). Larger blocks keep k_cons and k_invert_primary, whose separate
-// register budgets hold more zones in flight (the tiled update and inversion of
-// the 64-torus ensemble lost a tenth fused). W is written for every zone: the fallback reads it, and so
-// does a recorded step's reverse. *nfail must be zero on entry. Same values as
-// the two kernels.
+// The conserved update and the whole inversion of small blocks in one kernel, a
+// zone per thread (the inversion's U[B] from the updated faces): one launch for
+// three, and the update's primitives are the inversion's guess. Larger blocks
+// keep k_cons and k_invert_primary, whose separate register budgets hold more
+// zones in flight (the tiled update and inversion of the 64-torus ensemble lost
+// a tenth fused). W is written for every zone: a recorded step's reverse reads
+// it. Same values as the separate kernels.
 #ifndef HAMR_CONS_INV_MINB
 #define HAMR_CONS_INV_MINB 4
 #endif
@@ -2156,7 +2152,7 @@ __global__ void __launch_bounds__(BLK, HAMR_CONS_INV_MINB)
                double *__restrict__ Ucache, const T *__restrict__ F1, const T *__restrict__ F2,
                const T *__restrict__ F3, double *__restrict__ W, int full, StepSize st,
                const double *__restrict__ psf, double *__restrict__ pout, int *__restrict__ pflag,
-               int *__restrict__ failimage, int *__restrict__ flist, int *__restrict__ nfail) {
+               int *__restrict__ failimage) {
     const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= (long)d.n1 * d.n2 * d.n3) return;
     const Item3 it = item3(t, d.n3, d.n2);
@@ -2173,12 +2169,7 @@ __global__ void __launch_bounds__(BLK, HAMR_CONS_INV_MINB)
     for (int q = 0; q < N_ADV; q++) W[q * d.ks + c] = U[adv_comp(q)];
     if (d.ng3 == 0) W[6 * d.ks + c] = U[B3];
     face_average_b(d, m, psf, i, j, c, gi, U);
-    const int flag = invert_primary<INV>(d, inv_k(d, m, gi, gm), gm, U, pf);
-    if (flag) {
-        flist[atomicAdd(nfail, 1)] = (int)t;
-        return;
-    }
-    invert_epilogue<FIX>(d, gm, c, flag, pf, pout, pflag, failimage);
+    invert_zone<INV, FIX>(d, inv_k(d, m, gi, gm), gm, c, U, pf, pout, pflag, failimage);
 }
 
 // the fallback chain and epilogue of one listed zone (active-zone index t)
@@ -2507,18 +2498,24 @@ __device__ __forceinline__ void k_bound_x2_at(const Dims &d, double *pv, double 
     }
 }
 
-// The step-size update of a full sub-step (k_dt_finalize's work), done by the
-// last launch of the step; ndt null: none
+// The step-size bookkeeping that rides on a sub-step's last launch: the full
+// sub-step's update (dt_finalize), or the half sub-step's reset of the CFL
+// minima (ndt null) before the full one collects them; dtbits null: neither
 struct DtFinal {
     unsigned long long *dtbits;
     double *ndt, *dt_state;
     int *counter, interval;
 };
 __device__ __forceinline__ void dt_finalize(const DtFinal &f);
+constexpr unsigned long long BITS_1E9 = 0x41CDCD6500000000ULL;  // 1.0e9
 
 __global__ void k_bound_x2(const Dims d, double *pv, double *ps, const DtFinal fin) {
     const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t == 0 && fin.ndt) dt_finalize(fin);
+    if (fin.ndt) {
+        if (t == 0) dt_finalize(fin);
+    } else if (fin.dtbits && t < 4) {
+        fin.dtbits[t] = BITS_1E9;
+    }
     if (t >= n_bound_x2(d)) return;
     k_bound_x2_at(d, pv, ps, t);
 }
@@ -2569,8 +2566,6 @@ __global__ void k_halo(const Dims d, double *pv, double *ps, int side, double *b
 }
 
 // --------------------------------------------------------- step size logic
-constexpr unsigned long long BITS_1E9 = 0x41CDCD6500000000ULL;  // 1.0e9
-
 __global__ void k_dt_reset(unsigned long long *dtbits) {
     if (threadIdx.x < 4) dtbits[threadIdx.x] = BITS_1E9;
 }
@@ -2642,6 +2637,11 @@ static void set_cfl_limits(Dims &d) {
     }
 }
 
+struct StepWords {
+    double ndt, dt_state;   // CFL step of the last full sub-step; the graph's step size
+    int kerr, counter;      // a bounded wait gave up; the graph's steps
+};
+
 struct hamr_ctx {
     hamr_params prm;
     Dims d;
@@ -2664,7 +2664,7 @@ struct hamr_ctx {
     // 3-D blocks: the centre EMFs computed by the x3 flux kernel instead of
     // k_emf_centre (HAMR_EMF_IN_X3=0 keeps the separate kernel)
     bool emf_in_x3 = true;
-    // zones up to which the update without bulk copies takes the primary
+    // zones up to which the update without bulk copies takes the
     // inversion into its kernel (HAMR_CONS_INV_MAX overrides)
     long cons_inv_max = 1L << 17;
     // the primary inversion inside the TMA-staged update kernel (no floors or
@@ -2683,6 +2683,9 @@ struct hamr_ctx {
     double *gtab = nullptr;   // the metric point by point (k_geo_tab), FP64 step, or
     float *gtabf = nullptr;   // mixed step; neither on blocks with short phi rows
     unsigned long long *dtbits = nullptr;
+    // the words a step leaves for the host, side by side so that one copy and
+    // one wait read them (StepWords); the pointers below point into it
+    struct StepWords *words = nullptr;
     double *ndt = nullptr, *dt_state = nullptr;
     int *counter = nullptr;
     unsigned long long *divb = nullptr;
@@ -2708,17 +2711,21 @@ int fail_cuda(hamr_ctx *c, cudaError_t e, const char *what) {
 
 Geom geom_of(const hamr_ctx *c) { return Geom{c->gcov, c->gcon, c->gdet, c->conn, c->itab, c->gtab, c->gtabf}; }
 
-// the error word kernels set when a bounded wait gave up (read after a
-// synchronisation the caller already makes; cleared once reported)
-int check_kerr(hamr_ctx *ctx) {
-    if (!ctx->kerr) return HAMR_OK;
-    int v = 0;
-    CK(cudaMemcpyAsync(&v, ctx->kerr, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+// waits for the stream and reads the step's words; HAMR_E_CUDA where a
+// kernel's bounded wait gave up (cleared once reported)
+int read_words(hamr_ctx *ctx, StepWords &w) {
+    CK(cudaMemcpyAsync(&w, ctx->words, sizeof(w), cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
-    if (!v) return HAMR_OK;
+    if (!w.kerr) return HAMR_OK;
     CK(cudaMemsetAsync(ctx->kerr, 0, sizeof(int), ctx->stream));
     ctx->err = "a kernel's wait for its bulk copies timed out (the step's results are invalid)";
     return HAMR_E_CUDA;
+}
+
+// the start of a graph's steps: the first step size, none counted
+__global__ void k_advance_begin(StepWords *w, double dt) {
+    w->dt_state = dt;
+    w->counter = 0;
 }
 
 // kernel groups timed by hamr_profile_step
@@ -2978,17 +2985,16 @@ int launch_stage_t(hamr_ctx *ctx, int full, StepSize st, bool calc_dt, Prof *pf,
                                                       ctx->nfail, ctx->kerr, npiece, lpiece);
             }
         } else if (small) {
-            if (!flat) CK(cudaMemsetAsync(ctx->nfail, 0, sizeof(int), s));   // else emptied by k_ct_2d
             using ConsInv = void (*)(const Dims, const Geom, const double *, const double *, double *, const T *,
                                      const T *, const T *, double *, int, StepSize, const double *, double *, int *,
-                                     int *, int *, int *);
+                                     int *);
             static const ConsInv ci[2][4] = {
                 {k_cons_inv<T, HAMR_INV_2D, 0>, k_cons_inv<T, HAMR_INV_2D, 1>, k_cons_inv<T, HAMR_INV_2D, 2>,
                  k_cons_inv<T, HAMR_INV_2D, 3>},
                 {k_cons_inv<T, HAMR_INV_NM, 0>, k_cons_inv<T, HAMR_INV_NM, 1>, k_cons_inv<T, HAMR_INV_NM, 2>,
                  k_cons_inv<T, HAMR_INV_NM, 3>}};
             ci[nm][fix]<<<nblk(n), BLK, 0, s>>>(d, m, ctx->p, pg, ctx->U, F1, F2, F3, ctx->W, full, st, psf, pout,
-                                                ctx->pflag, ctx->failimage, ctx->flist, ctx->nfail);
+                                                ctx->pflag, ctx->failimage);
         } else if (d.n3 >= 64 && ctx->cons_cols)   // metric and connection staged per CTA
             k_cons_cols<T><<<nblk(n), BLK, 0, s>>>(d, m, ctx->p, full ? ctx->ph : ctx->p, ctx->U, F1, F2, F3, ctx->W,
                                                    full, st, ctx->nfail);
@@ -3020,7 +3026,8 @@ int launch_stage_t(hamr_ctx *ctx, int full, StepSize st, bool calc_dt, Prof *pf,
         if (!fuse && !small)
             inv_p[nm][fix]<<<nblk(n), BLK, 0, s>>>(d, m, pg, ctx->W, psf, pout, ctx->pflag, ctx->failimage,
                                                    ctx->flist, ctx->nfail);
-        inv_f[nm][fix]<<<FALLBACK_CTAS, BLK, 0, s>>>(d, m, pg, ctx->W, psf, pout, ctx->pflag, ctx->failimage,
+        if (!small)
+            inv_f[nm][fix]<<<FALLBACK_CTAS, BLK, 0, s>>>(d, m, pg, ctx->W, psf, pout, ctx->pflag, ctx->failimage,
                                                      ctx->flist, ctx->nfail);
         if (ctx->prm.repair == 2) {
             k_repair_scan<<<nblk((long)d.G1 * d.G2 * d.G3), BLK, 0, s>>>(d, pout, ctx->pflag, ctx->failimage,
@@ -3044,7 +3051,7 @@ int launch_stage(hamr_ctx *ctx, int full, StepSize st, bool calc_dt, Prof *pf = 
 }
 
 int launch_step(hamr_ctx *ctx, StepSize half, StepSize full, double *dt_state, int interval) {
-    int rc = launch_stage(ctx, 0, half, false);
+    int rc = launch_stage(ctx, 0, half, false, nullptr, DtFinal{ctx->dtbits, nullptr, nullptr, nullptr, 0});
     if (rc) return rc;
     // the step size with the last ghost fill (blocks with halo sides, whose
     // ghost fill is the caller's, do not step here)
@@ -3148,13 +3155,11 @@ int hamr_ctx_create(const hamr_params *prm, hamr_ctx **out) {
         {(void **)&ctx->itab, 16 * sizeof(double) * d.gs},
         {(void **)&ctx->gtab, geo_tab_wanted(d.n3) && prm->precision == HAMR_FP64 ? 5 * GT<double> * sizeof(double) * d.gs : 0},
         {(void **)&ctx->gtabf, geo_tab_wanted(d.n3) && prm->precision == HAMR_MIXED ? 5 * GT<float> * sizeof(float) * d.gs : 0},
-        {(void **)&ctx->dtbits, 4 * sizeof(unsigned long long)}, {(void **)&ctx->ndt, sizeof(double)},
-        {(void **)&ctx->dt_state, sizeof(double)}, {(void **)&ctx->counter, sizeof(int)},
+        {(void **)&ctx->dtbits, 4 * sizeof(unsigned long long)}, {(void **)&ctx->words, sizeof(StepWords)},
         {(void **)&ctx->divb, sizeof(unsigned long long)},
         {(void **)&ctx->rlist, prm->repair == 2 ? sizeof(int) * d.n1 * d.n2 * d.n3 : 0},
         {(void **)&ctx->rcount, prm->repair == 2 ? sizeof(int) : 0},
-        {(void **)&ctx->flist, sizeof(int) * d.n1 * d.n2 * d.n3}, {(void **)&ctx->nfail, sizeof(int)},
-        {(void **)&ctx->kerr, sizeof(int)}};
+        {(void **)&ctx->flist, sizeof(int) * d.n1 * d.n2 * d.n3}, {(void **)&ctx->nfail, sizeof(int)}};
     if (prm->repair == 2 && d.ks > 0x7fffffffL) { hamr_ctx_destroy(ctx); return HAMR_E_ARG; }
     for (auto &a : allocs) {
         if (a.n == 0) continue;
@@ -3164,6 +3169,10 @@ int hamr_ctx_create(const hamr_params *prm, hamr_ctx **out) {
         }
         cudaMemsetAsync(*a.p, 0, a.n, ctx->stream);
     }
+    ctx->ndt = &ctx->words->ndt;   // device addresses
+    ctx->dt_state = &ctx->words->dt_state;
+    ctx->kerr = &ctx->words->kerr;
+    ctx->counter = &ctx->words->counter;
     k_dt_reset<<<1, 32, 0, ctx->stream>>>(ctx->dtbits);
     cons_tma_attributes<double>();
     cons_tma_attributes<float>();
@@ -3182,8 +3191,7 @@ int hamr_ctx_destroy(hamr_ctx *ctx) {
     void *bufs[] = {ctx->p, ctx->ph, ctx->ps, ctx->psh, ctx->U, ctx->F1, ctx->F2, ctx->F3, ctx->Ec, ctx->emf,
                     ctx->W, ctx->pflag, ctx->failimage, ctx->gcov, ctx->gcon, ctx->gdet, ctx->conn, ctx->itab,
                     ctx->gtab, ctx->gtabf, ctx->dtbits,
-                    ctx->ndt, ctx->dt_state, ctx->counter, ctx->divb, ctx->rlist, ctx->rcount,
-                    ctx->flist, ctx->nfail, ctx->kerr};
+                    ctx->words, ctx->divb, ctx->rlist, ctx->rcount, ctx->flist, ctx->nfail};
     for (void *b : bufs)
         if (b) cudaFree(b);
     for (auto st : ctx->side)
@@ -3308,13 +3316,13 @@ int hamr_step(hamr_ctx *ctx, double dt, double *dt_next) {
         return HAMR_E_STATE;
     }
     if (!(dt > 0)) return HAMR_E_ARG;
-    k_dt_reset<<<1, 32, 0, ctx->stream>>>(ctx->dtbits);
     int rc = launch_step(ctx, StepSize{nullptr, 0.5, 0.5 * dt, dt}, StepSize{nullptr, 1.0, dt, dt}, nullptr, 0);
     if (rc) return rc;
     if (dt_next) {
-        CK(cudaMemcpyAsync(dt_next, ctx->ndt, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-        CK(cudaStreamSynchronize(ctx->stream));
-        if (int rc2 = check_kerr(ctx)) return rc2;
+        StepWords w{};
+        rc = read_words(ctx, w);
+        *dt_next = w.ndt;
+        if (rc) return rc;
         if (!(*dt_next > 0) || !isfinite(*dt_next)) {
             ctx->err = "non-finite or non-positive CFL step";
             return HAMR_E_PHYSICS;
@@ -3331,9 +3339,8 @@ int hamr_advance(hamr_ctx *ctx, int nsteps, int interval, double *dt_inout) {
         return HAMR_E_STATE;
     }
     if (!(*dt_inout > 0)) return HAMR_E_ARG;
-    CK(cudaMemcpyAsync(ctx->dt_state, dt_inout, sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
-    CK(cudaMemsetAsync(ctx->counter, 0, sizeof(int), ctx->stream));
-    k_dt_reset<<<1, 32, 0, ctx->stream>>>(ctx->dtbits);
+    k_advance_begin<<<1, 1, 0, ctx->stream>>>(ctx->words, *dt_inout);
+    CK(cudaGetLastError());
     if (!ctx->graph || ctx->graph_steps != nsteps || ctx->graph_interval != interval) {
         if (ctx->graph) {
             cudaGraphExecDestroy(ctx->graph);
@@ -3355,9 +3362,10 @@ int hamr_advance(hamr_ctx *ctx, int nsteps, int interval, double *dt_inout) {
         ctx->graph_interval = interval;
     }
     CK(cudaGraphLaunch(ctx->graph, ctx->stream));
-    CK(cudaMemcpyAsync(dt_inout, ctx->dt_state, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaStreamSynchronize(ctx->stream));
-    return check_kerr(ctx);
+    StepWords w{};
+    const int rc = read_words(ctx, w);
+    *dt_inout = w.dt_state;
+    return rc;
 }
 
 int hamr_profile_step(hamr_ctx *ctx, double dt, int reps, double *ms, int nslots) {
@@ -3544,7 +3552,6 @@ extern "C" int hamr_step_noalloc(const hamr_params *prm, const double *gcov, con
         if (cudaMemsetAsync(c.F3, 0, 9 * sizeof(double) * ks, c.stream) != cudaSuccess) return HAMR_E_CUDA;
         if (cudaMemsetAsync(c.Ec, 0, 4 * sizeof(double) * ks, c.stream) != cudaSuccess) return HAMR_E_CUDA;
     }
-    k_dt_reset<<<1, 32, 0, c.stream>>>(c.dtbits);
     int rc = launch_step(&c, StepSize{nullptr, 0.5, 0.5 * dt, dt}, StepSize{nullptr, 1.0, dt, dt}, nullptr, 0);
     c.p = c.ps = nullptr;  // caller-owned: not ours to release
     if (rc) return rc;
