@@ -1936,10 +1936,11 @@ __host__ __device__ __forceinline__ ConsTmaLayout cons_tma_layout(int lpiece) {
 
 // FUSE: 0 writes the planes of W for the inversion kernels; HAMR_INV_2D + 1 or
 // HAMR_INV_NM + 1 runs the primary inversion of each zone right after its
-// update (no floors or repair): the guess is pb (the state the update read),
-// the face field psf, the output pout, and only a zone whose primary solver
-// fails writes W and goes to the list for k_invert_fallback (*nfail cleared
-// before the launch). The W round trip and the inversion's reload of the guess
+// update: the guess is pb (the state the update read), the face field psf, the
+// output pout, and only a zone whose primary solver fails writes W and goes to
+// the list for k_invert_fallback (*nfail cleared before the launch). FIX: 0 or
+// FIX_FLOORS, the floors on each zone it solves (the reset of failed zones keeps
+// the separate kernels; the neighbour repair follows either way). The W round trip and the inversion's reload of the guess
 // disappear; same values as the update followed by k_invert_primary.
 //
 // Resident CTAs of 256 threads per SM, which cap the registers (4: 64, 3: 80,
@@ -1964,7 +1965,7 @@ __host__ __device__ constexpr int cons_tma_minb(int fuse, bool short_rows) {
 }
 // The body of one CTA: row piece `blk` (row * npiece + piece) of the block,
 // `smem` the CTA's dynamic shared memory (cons_tma_layout(lpiece).total bytes).
-template <typename T, int FUSE>
+template <typename T, int FUSE, int FIX = 0>
 __device__ __forceinline__ void cons_tma_row(const Dims &d, const Geom &m, const double *__restrict__ pin,
                                              const double *__restrict__ pb, double *__restrict__ Ucache,
                                              const T *__restrict__ F1, const T *__restrict__ F2,
@@ -2069,11 +2070,11 @@ __device__ __forceinline__ void cons_tma_row(const Dims &d, const Geom &m, const
             flist[atomicAdd(nfail, 1)] = (int)t;
             return;
         }
-        invert_epilogue<0>(d, gm, c, flag, pf, pout, pflag, failimage);
+        invert_epilogue<FIX>(d, gm, c, flag, pf, pout, pflag, failimage);
     }
 }
 
-template <typename T, int FUSE = 0, int MINB = cons_tma_minb<T>(0, false)>
+template <typename T, int FUSE = 0, int MINB = cons_tma_minb<T>(0, false), int FIX = 0>
 __global__ void __launch_bounds__(256, MINB)
     k_cons_tma(const Dims d, const Geom m, const double *__restrict__ pin, const double *__restrict__ pb,
                double *__restrict__ Ucache, const T *__restrict__ F1, const T *__restrict__ F2,
@@ -2082,8 +2083,8 @@ __global__ void __launch_bounds__(256, MINB)
                double *__restrict__ pout = nullptr, int *__restrict__ pflag = nullptr,
                int *__restrict__ failimage = nullptr, int *__restrict__ flist = nullptr) {
     extern __shared__ __align__(16) unsigned char smem[];
-    cons_tma_row<T, FUSE>(d, m, pin, pb, Ucache, F1, F2, F3, W, full, st, nfail, kerr, npiece, lpiece, blockIdx.x,
-                          smem, psf, pout, pflag, failimage, flist);
+    cons_tma_row<T, FUSE, FIX>(d, m, pin, pb, Ucache, F1, F2, F3, W, full, st, nfail, kerr, npiece, lpiece, blockIdx.x,
+                               smem, psf, pout, pflag, failimage, flist);
 }
 
 template <int INV, int FIX = 0>
@@ -2815,6 +2816,10 @@ void cons_tma_attributes() {
     set(k_cons_tma<T>, all);
     set(k_cons_tma<T, HAMR_INV_2D + 1, L>, all);
     set(k_cons_tma<T, HAMR_INV_NM + 1, L>, all);
+    set(k_cons_tma<T, HAMR_INV_2D + 1, L, FIX_FLOORS>, all);
+    set(k_cons_tma<T, HAMR_INV_NM + 1, L, FIX_FLOORS>, all);
+    set(k_cons_tma<T, HAMR_INV_2D + 1, S, FIX_FLOORS>, few);
+    set(k_cons_tma<T, HAMR_INV_NM + 1, S, FIX_FLOORS>, few);
     set(k_cons_tma<T, HAMR_INV_2D + 1, S>, few);
     set(k_cons_tma<T, HAMR_INV_NM + 1, S>, few);
 }
@@ -2963,9 +2968,9 @@ int launch_stage_t(hamr_ctx *ctx, int full, StepSize st, bool calc_dt, Prof *pf,
         const int nm = d.inversion == HAMR_INV_NM;
         // the primary inversion inside the update kernel (the face update, which
         // it reads, has run in this stream)
-        const bool fuse = tma && ctx->fuse_inv && fix == 0 && ctx->prm.repair != 2 && !conc;
-        // small blocks without the bulk-copy update: update and primary
-        // inversion in one kernel
+        const bool fuse = tma && ctx->fuse_inv && !(fix & FIX_RESET) && !conc;
+        // small blocks without the bulk-copy update: update and inversion in one
+        // kernel
         const bool small = !tma && !conc && ctx->fuse_inv && n <= ctx->cons_inv_max;
         if (tma) {   // one row of zones per CTA, flux operands staged by bulk copies
             const int npiece = (d.n3 + 255) / 256, lpiece = (d.n3 + npiece - 1) / npiece;
@@ -2974,9 +2979,13 @@ int launch_stage_t(hamr_ctx *ctx, int full, StepSize st, bool calc_dt, Prof *pf,
             if (fuse) {
                 CK(cudaMemsetAsync(ctx->nfail, 0, sizeof(int), s));
                 constexpr int S = cons_tma_minb<T>(1, true), L = cons_tma_minb<T>(1, false);
-                auto kf = lpiece <= CONS_SHORT_ROW
-                              ? (nm ? k_cons_tma<T, HAMR_INV_NM + 1, S> : k_cons_tma<T, HAMR_INV_2D + 1, S>)
-                              : (nm ? k_cons_tma<T, HAMR_INV_NM + 1, L> : k_cons_tma<T, HAMR_INV_2D + 1, L>);
+                auto pick = [&](auto k2d, auto knm) { return nm ? knm : k2d; };
+                constexpr int I2 = HAMR_INV_2D + 1, IN = HAMR_INV_NM + 1;
+                const bool brief = lpiece <= CONS_SHORT_ROW;
+                auto kf = fix ? (brief ? pick(k_cons_tma<T, I2, S, FIX_FLOORS>, k_cons_tma<T, IN, S, FIX_FLOORS>)
+                                       : pick(k_cons_tma<T, I2, L, FIX_FLOORS>, k_cons_tma<T, IN, L, FIX_FLOORS>))
+                              : (brief ? pick(k_cons_tma<T, I2, S>, k_cons_tma<T, IN, S>)
+                                       : pick(k_cons_tma<T, I2, L>, k_cons_tma<T, IN, L>));
                 kf<<<grid, block, sm, s>>>(d, m, ctx->p, pg, ctx->U, F1, F2, F3, ctx->W, full, st, ctx->nfail,
                                            ctx->kerr, npiece, lpiece, psf, pout, ctx->pflag, ctx->failimage,
                                            ctx->flist);
