@@ -2369,49 +2369,41 @@ __device__ __forceinline__ void copy_cell(const Dims &d, double *pv, long dst, l
     for (int k = 0; k < NPR; k++) pv[k * d.ks + dst] = pv[k * d.ks + src];
 }
 
-// x1 ghosts over every (j, z): periodic copy, or outflow copy + no-inflow
+// x1 ghosts over every (j, z): periodic copy, or outflow copy + no-inflow. One
+// item per (side, layer, j, z): an item's loads, no-inflow check and stores are
+// one dependent chain, and both sides' in one item were two
+__host__ __device__ __forceinline__ long n_bound_x1(const Dims &d) { return 2L * d.ng1 * d.G2 * d.G3; }
+
 __device__ __forceinline__ void k_bound_x1_at(const Dims &d, const Geom &m, double *pv, double *ps, const long t) {
     const Item3 it = item3(t, d.G3, d.G2);
-    const int z = it.z, j = it.j, g = it.i;
-    const int ilo = g, ihi = d.n1 + d.ng1 + g;
-    const long ks = d.ks;
+    const int z = it.z, j = it.j, g = it.i % d.ng1;
+    const bool upper = it.i >= d.ng1;
+    const int i = upper ? d.n1 + d.ng1 + g : g;
+    const long ks = d.ks, dst = cix(d, i, j, z);
     if (d.bc1 == HAMR_BC_PERIODIC) {
-        copy_cell(d, pv, cix(d, ilo, j, z), cix(d, ilo + d.n1, j, z));
-        copy_cell(d, pv, cix(d, ihi, j, z), cix(d, ihi - d.n1, j, z));
-        for (int k = 0; k < 3; k++) {
-            ps[k * ks + cix(d, ilo, j, z)] = ps[k * ks + cix(d, ilo + d.n1, j, z)];
-            ps[k * ks + cix(d, ihi, j, z)] = ps[k * ks + cix(d, ihi - d.n1, j, z)];
-        }
+        const long src = cix(d, upper ? i - d.n1 : i + d.n1, j, z);
+        copy_cell(d, pv, dst, src);
+        for (int k = 0; k < 3; k++) ps[k * ks + dst] = ps[k * ks + src];
         return;
     }
+    if (d.halo & (upper ? 2 : 1)) return;   // a side shared with a neighbouring block is filled by the exchange
+    const long src = cix(d, upper ? d.n1 + d.ng1 - 1 : d.ng1, j, z);
     double pr[NPR];
     Geo<double> gm;
-    long src, dst;
-    if (!(d.halo & 1)) {   // a side shared with a neighbouring block is filled by the exchange
-        src = cix(d, d.ng1, j, z);
-        dst = cix(d, ilo, j, z);
-        for (int k = 0; k < NPR; k++) pr[k] = pv[k * ks + src];
-        load_geo(d, m, ilo, j, CENT, gm);
-        inflow_check(pr, gm, 0);
-        for (int k = 0; k < NPR; k++) pv[k * ks + dst] = pr[k];
-        ps[1 * ks + dst] = ps[1 * ks + src];
-        ps[2 * ks + dst] = ps[2 * ks + src];
-    }
-    if (!(d.halo & 2)) {
-        src = cix(d, d.n1 + d.ng1 - 1, j, z);
-        dst = cix(d, ihi, j, z);
-        for (int k = 0; k < NPR; k++) pr[k] = pv[k * ks + src];
-        load_geo(d, m, ihi, j, CENT, gm);
-        inflow_check(pr, gm, 1);
-        for (int k = 0; k < NPR; k++) pv[k * ks + dst] = pr[k];
-        ps[1 * ks + dst] = ps[1 * ks + src];
-        ps[2 * ks + dst] = ps[2 * ks + src];
-    }
+#pragma unroll
+    for (int k = 0; k < NPR; k++) pr[k] = pv[k * ks + src];
+    const double s2 = ps[1 * ks + src], s3 = ps[2 * ks + src];
+    load_geo(d, m, i, j, CENT, gm);
+    inflow_check(pr, gm, upper ? 1 : 0);
+#pragma unroll
+    for (int k = 0; k < NPR; k++) pv[k * ks + dst] = pr[k];
+    ps[1 * ks + dst] = s2;
+    ps[2 * ks + dst] = s3;
 }
 
 __global__ void k_bound_x1(const Dims d, const Geom m, double *pv, double *ps) {
     const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (long)d.ng1 * d.G2 * d.G3) return;
+    if (t >= n_bound_x1(d)) return;
     k_bound_x1_at(d, m, pv, ps, t);
 }
 
@@ -2751,7 +2743,7 @@ int launch_bound_dim(hamr_ctx *ctx, int full, int dim, const DtFinal &fin = {}) 
     double *pw = full ? ctx->p : ctx->ph;
     double *psw = full ? ctx->ps : ctx->psh;
     if ((dim == 0 || dim == 1) && d.d1)
-        k_bound_x1<<<nblk((long)d.ng1 * d.G2 * d.G3), BLK, 0, s>>>(d, geom_of(ctx), pw, psw);
+        k_bound_x1<<<nblk(n_bound_x1(d)), BLK, 0, s>>>(d, geom_of(ctx), pw, psw);
     if ((dim == 0 || dim == 3) && d.d3) k_bound_x3<<<nblk(n_bound_x3(d)), BLK, 0, s>>>(d, pw, psw);
     if ((dim == 0 || dim == 2) && d.d2) k_bound_x2<<<nblk(n_bound_x2(d)), BLK, 0, s>>>(d, pw, psw, fin);
     CK(cudaGetLastError());
