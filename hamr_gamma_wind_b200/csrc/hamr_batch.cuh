@@ -24,7 +24,7 @@ struct BEntry {
     Geom m;
     double *p, *ph, *ps, *psh, *U, *F1, *F2, *F3, *Ec, *emf, *W;
     int *pflag, *failimage;
-    int *nfail, *kerr;           // the block's failed-zone count; the batch's error word
+    int *flist, *nfail, *kerr;   // the block's failed zones and their count; the batch's error word
     unsigned long long *dtbits;  // 4 per block
     double *ndt, *dt_state;      // 1 per block
     int *counter;                // 1 per block
@@ -156,20 +156,23 @@ struct OpInvert {
 // The conserved update phase with the single-block kernel's bulk-copy
 // staging (cons_tma_row): one CTA per row piece of a block, rstart[k] the
 // first CTA of block k (every block 3-D with n3 >= 32 and aligned flux
-// planes). Same values as OpCons. (The primary inversion inside, as the
-// single-block kernel runs it, measured slower here: rows of 32-96 zones.)
-// resident CTAs (of up to 256 threads) per SM, FP64 / float fluxes; on the
-// 64-torus ensemble (rows of 32-96 zones) the float update took 2.37 ms per
-// sub-step at 3 (80 registers), 2.61 at 4 (64), and at 5 (48 registers,
-// 0.7 KB of spills) lost to the tiled update
+// planes). FUSE as there: 0 the update alone, same values as OpCons; else the
+// primary inversion inside it, the zones it fails to their block's list
+// (emptied by k_batch_begin_lists) for k_batch_fallback.
+// Resident CTAs (of up to 256 threads) per SM, FP64 / float fluxes, of the
+// update alone: on the 64-torus ensemble (rows of 32-96 zones) the float update
+// took 2.37 ms per sub-step at 3 (80 registers), 2.61 at 4 (64), and at 5 (48
+// registers, 0.7 KB of spills) lost to the tiled update, before the magnetic
+// components left it. With the inversion: the single block's short rows.
 #ifndef HAMR_BATCH_CONS_TMA_MINB
 #define HAMR_BATCH_CONS_TMA_MINB HAMR_CONS_TMA_MINB
 #endif
 #ifndef HAMR_BATCH_CONS_TMA_MINB_F
 #define HAMR_BATCH_CONS_TMA_MINB_F HAMR_CONS_TMA_MINB_F
 #endif
-template <typename T>
-__global__ void __launch_bounds__(256, sizeof(T) == 8 ? HAMR_BATCH_CONS_TMA_MINB : HAMR_BATCH_CONS_TMA_MINB_F)
+template <typename T, int FUSE>
+__global__ void __launch_bounds__(256, FUSE ? cons_tma_minb<T>(1, true)
+                                            : (sizeof(T) == 8 ? HAMR_BATCH_CONS_TMA_MINB : HAMR_BATCH_CONS_TMA_MINB_F))
     k_batch_cons_tma(const BEntry *__restrict__ E, const long *__restrict__ rstart, int n, const StageArg a) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ BEntry e;
@@ -186,10 +189,26 @@ __global__ void __launch_bounds__(256, sizeof(T) == 8 ? HAMR_BATCH_CONS_TMA_MINB
     }
     __syncthreads();
     const int npiece = (e.d.n3 + 255) / 256, lpiece = (e.d.n3 + npiece - 1) / npiece;
-    cons_tma_row<T, 0>(e.d, e.m, e.p, a.full ? e.ph : e.p, e.U, reinterpret_cast<const T *>(e.F1),
-                       reinterpret_cast<const T *>(e.F2), reinterpret_cast<const T *>(e.F3), e.W, a.full,
-                       entry_step(e, a), e.nfail, e.kerr, npiece, lpiece, (int)(blockIdx.x - rstart[lo]), smem,
-                       nullptr, nullptr, nullptr, nullptr, nullptr);
+    cons_tma_row<T, FUSE>(e.d, e.m, e.p, a.full ? e.ph : e.p, e.U, reinterpret_cast<const T *>(e.F1),
+                          reinterpret_cast<const T *>(e.F2), reinterpret_cast<const T *>(e.F3), e.W, a.full,
+                          entry_step(e, a), e.nfail, e.kerr, npiece, lpiece, (int)(blockIdx.x - rstart[lo]), smem,
+                          a.full ? e.ps : e.psh, a.full ? e.p : e.ph, e.pflag, e.failimage, e.flist);
+}
+
+__global__ void k_batch_begin_lists(const BEntry *__restrict__ E, int n) {
+    const int b = blockIdx.x * blockDim.x + threadIdx.x;
+    if (b < n) *E[b].nfail = 0;
+}
+
+// the fallback chain over every block's list (k_invert_fallback's work): CTA
+// (q, b) takes entries q BLK, q BLK + gridDim.x BLK, ... of block b
+constexpr int BATCH_FALLBACK_CTAS = 8;   // per block
+__global__ void __launch_bounds__(BLK) k_batch_fallback(const BEntry *__restrict__ E, const StageArg a) {
+    const BEntry &e = E[blockIdx.y];
+    const int n = *e.nfail;
+    for (int q = blockIdx.x * BLK + threadIdx.x; q < n; q += gridDim.x * BLK)
+        invert_fallback_at<0>(e.d, e.m, a.full ? e.ph : e.p, e.W, a.full ? e.ps : e.psh, a.full ? e.p : e.ph, e.pflag,
+                              e.failimage, e.flist[q]);
 }
 
 // The x3 fluxes of the batch by zone slots, with the centre EMFs: the
@@ -453,6 +472,8 @@ struct hamr_batch {
     // block allows it (cons_tma_ok) and it is in use (cons_tma: by default in
     // the mixed step; the autotuner times it against the tiled update)
     bool cons_tma_ok = false, cons_tma = false;
+    // the primary inversion inside it (no floors or reset): allowed, and in use
+    bool fused_ok = false, fused = false;
     // x3 fluxes and centre EMFs by zone slots (k_batch_flux_x3): every block
     // 3-D; off with HAMR_BATCH_FLUX_X3=0
     bool flux3_slots = false;
@@ -501,6 +522,20 @@ int build_tiles(hamr_batch *b, int ph) {
     return HAMR_OK;
 }
 
+// Default items per tile: a tile costs its CTA a search for the block and a
+// copy of the block's description, so as many of a thread's items share one
+// as leave every multiprocessor 16 tiles; at most 4 a thread for the fluxes
+// and 16 for the phases that move a few values per item. The 64-torus ensemble
+// (15.6 M zones), per step without the autotuner: mixed 16.7 -> 14.8 ms against
+// BLK-item tiles, FP64 24.8 -> 22.5 (there with the bulk-copy update); the
+// autotuner then finds another 0.1 %.
+int default_tile(const hamr_batch *b, int ph) {
+    long items = 0;
+    for (long x : b->items[ph]) items += x;
+    const long most = ph == PH_FLUX3 || ph == PH_FLUX2 || ph == PH_FLUX1 ? 4 : 16;
+    return BLK * (int)std::max(1L, std::min(most, items / (16L * BLK * b->nsm)));
+}
+
 template <class Op>
 void launch_phase(hamr_batch *b, const StageArg &a) {
     const int ph = Op::PH;
@@ -530,14 +565,19 @@ void batch_stage_t(hamr_batch *b, int full, bool calc_dt, int only) {
     if (want(PH_EMFE)) launch_phase<OpEmfEdge<T>>(b, a);
     if (want(PH_POLE)) launch_phase<OpPole<T>>(b, a);
     if (want(PH_FACE)) launch_phase<OpFace<T>>(b, a);
-    if (want(PH_CONS)) {
+    if (want(PH_CONS) && b->fused) {   // with the inversion
+        k_batch_begin_lists<<<nblk_b(b->n), 128, 0, b->stream>>>(b->E, b->n);
+        k_batch_cons_tma<T, INV + 1><<<(unsigned)b->ncons_ctas, b->cons_block, b->cons_smem, b->stream>>>(
+            b->E, b->rstart, b->n, a);
+        k_batch_fallback<<<dim3(BATCH_FALLBACK_CTAS, (unsigned)b->n), BLK, 0, b->stream>>>(b->E, a);
+    } else if (want(PH_CONS)) {
         if (b->cons_tma)
-            k_batch_cons_tma<T><<<(unsigned)b->ncons_ctas, b->cons_block, b->cons_smem, b->stream>>>(b->E, b->rstart,
+            k_batch_cons_tma<T, 0><<<(unsigned)b->ncons_ctas, b->cons_block, b->cons_smem, b->stream>>>(b->E, b->rstart,
                                                                                                  b->n, a);
         else
             launch_phase<OpCons<T>>(b, a);
     }
-    if (want(PH_INV)) {
+    if (want(PH_INV) && !b->fused) {
         switch (b->fix) {
             case FIX_FLOORS: launch_phase<OpInvert<INV, FIX_FLOORS>>(b, a); break;
             case FIX_RESET: launch_phase<OpInvert<INV, FIX_RESET>>(b, a); break;
@@ -663,7 +703,8 @@ int batch_setup_cons_tma(hamr_batch *b) {
         sm = std::max(sm, cons_tma_layout<T>(lpiece).total);
     }
     if (rs[b->n] > 0x7fffffffL) return HAMR_OK;   // more CTAs than one launch's grid holds
-    BCK(cudaFuncSetAttribute(k_batch_cons_tma<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
+    for (auto k : {k_batch_cons_tma<T, 0>, k_batch_cons_tma<T, HAMR_INV_2D + 1>, k_batch_cons_tma<T, HAMR_INV_NM + 1>})
+        BCK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
     BCK(cudaMemcpyAsync(b->rstart, rs.data(), sizeof(long) * (b->n + 1), cudaMemcpyHostToDevice, b->stream));
     BCK(cudaStreamSynchronize(b->stream));   // rs goes out of scope
     b->ncons_ctas = rs[b->n];
@@ -671,10 +712,13 @@ int batch_setup_cons_tma(hamr_batch *b) {
     b->cons_smem = (size_t)sm;
     b->cons_tma_ok = true;
     // measured on the 64-torus ensemble (rows of 32-96 zones), per sub-step:
-    // float fluxes 2.37 ms against 2.69 for the tiled update; FP64 3.20
-    // against 2.59 (the FP64 staging holds 6 CTAs of at most 96 threads per SM)
-    b->cons_tma = sizeof(T) == 4;
-    if (const char *e = getenv("HAMR_BATCH_CONS_TMA")) b->cons_tma = atoi(e) != 0;   // 1: also FP64; 0: off
+    // float fluxes 1.64 ms, FP64 2.06 against 2.3 for the tiled update (whose
+    // FP64 form was the faster one, 2.59 against 3.20 ms, while the staging held
+    // the magnetic components and fewer CTAs fitted an SM)
+    b->cons_tma = true;
+    if (const char *e = getenv("HAMR_BATCH_CONS_TMA")) b->cons_tma = atoi(e) != 0;   // 0: off
+    b->fused_ok = b->fused = b->cons_tma && b->fix == 0 && b->n <= 65535;
+    if (const char *e = getenv("HAMR_BATCH_FUSE_INV")) b->fused = b->fused_ok = b->fused_ok && atoi(e) != 0;
     return HAMR_OK;
 }
 
@@ -746,6 +790,7 @@ int hamr_batch_create(hamr_ctx *const *blocks, int n, void *stream, hamr_batch *
         e.ndt = b->ndts + k;
         e.dt_state = b->dts + k;
         e.counter = b->counters + k;
+        e.flist = c->flist;
         e.nfail = c->nfail;
         e.kerr = b->kerr;
         for (int ph = 0; ph < PH_N; ph++) b->items[ph].push_back(phase_items(ph, c->d));
@@ -758,7 +803,7 @@ int hamr_batch_create(hamr_ctx *const *blocks, int n, void *stream, hamr_batch *
         cudaMemcpyAsync(b->E, host.data(), sizeof(BEntry) * n, cudaMemcpyHostToDevice, b->stream) != cudaSuccess)
         rc = HAMR_E_CUDA;
     for (int ph = 0; ph < PH_N && rc == HAMR_OK; ph++) {
-        b->tile[ph] = BLK;      // default: one BLK-item tile per CTA, caller's order
+        b->tile[ph] = default_tile(b, ph);   // one tile per CTA, caller's order
         b->grid[ph] = 0;
         b->order_mode[ph] = 0;
         rc = build_tiles(b, ph);
@@ -933,6 +978,9 @@ int hamr_batch_autotune(hamr_batch *b, const double *dt, int reps) {
             cudaEventElapsedTime(&ms, e0, e1);
             return ms / reps;
         };
+        // the update with the inversion inside is timed once both phases have
+        // their own best
+        if (ph == PH_CONS) b->fused = false;
         // the conserved update's bulk-copy kernel is one more candidate (its
         // launch shape is fixed)
         bool tma_best = false;
@@ -963,6 +1011,28 @@ int hamr_batch_autotune(hamr_batch *b, const double *dt, int reps) {
         b->order_mode[ph] = bo;
         b->tuned_ms[ph] = best;
         if (rc == HAMR_OK) rc = build_tiles(b, ph);
+        if (ph == PH_INV && b->fused_ok && rc == HAMR_OK) {
+            batch_stage(b, 0, false, PH_CONS);
+            b->fused = true;
+            auto both = [&]() -> float {
+                batch_stage(b, 0, false, PH_CONS);
+                cudaEventRecord(e0, b->stream);
+                for (int r = 0; r < reps; r++) batch_stage(b, 0, false, PH_CONS);
+                cudaEventRecord(e1, b->stream);
+                if (cudaEventSynchronize(e1) != cudaSuccess) return -1.f;
+                float ms = 0.f;
+                cudaEventElapsedTime(&ms, e0, e1);
+                return ms / reps;
+            };
+            const float ms = both();
+            if (ms < 0) rc = bfail(b, cudaGetLastError(), "autotune");
+            b->fused = ms < b->tuned_ms[PH_CONS] + b->tuned_ms[PH_INV];
+            if (b->fused) {
+                b->tuned_ms[PH_CONS] = ms;   // the inversion phase launches nothing
+                b->tuned_ms[PH_INV] = 0.f;
+            }
+            if (rc == HAMR_OK) batch_stage(b, 0, false, PH_CONS);
+        }
         if (rc == HAMR_OK) batch_stage(b, 0, false, ph);   // leave this phase's outputs for the next phase
     }
     cudaEventDestroy(e0);
@@ -986,7 +1056,7 @@ int hamr_batch_tuning(hamr_batch *b, int *tile, int *grid, int *order, float *ms
     if (!b || nphases < PH_N) return HAMR_E_ARG;
     for (int ph = 0; ph < PH_N; ph++) {
         if (tile)
-            tile[ph] = (ph == PH_CONS && b->cons_tma) || ((ph == PH_FLUX3 || ph == PH_EMFC) && b->flux3_slots)
+            tile[ph] = (ph == PH_CONS && (b->cons_tma || b->fused)) || ((ph == PH_FLUX3 || ph == PH_EMFC) && b->flux3_slots)
                            ? 0 : b->tile[ph];
         if (grid) grid[ph] = b->grid[ph];
         if (order) order[ph] = b->order_mode[ph];
