@@ -250,7 +250,7 @@ __device__ __forceinline__ void state_back(const double *pr, const Geo<double> &
     a.u += a.w + a.P * (gam - 1.);
     a.gam += a.P * u;
     if (a.K != 0.) {
-        const double rg = pow(rho, -gam);
+        const double rg = d_pow(rho, -gam);
         a.u += a.K * (gam - 1.) * rg;
         a.gam += a.K * (u * rg - f.K * log(rho));
         a.rho -= a.K * gam * f.K / rho;
@@ -269,7 +269,7 @@ __device__ __forceinline__ void state_back(const double *pr, const Geo<double> &
     }
     // b^j = (B^j + b^0 u^j) / u^0, then b^0 = B^i u_i
     double Bb[3];
-    const double ru0 = 1. / q.ucon[0];
+    const double ru0 = d_rcp(q.ucon[0]);
 #pragma unroll
     for (int j = 1; j < 4; j++) {
         const double bj = a.bcon[j] * ru0;
@@ -292,14 +292,14 @@ __device__ __forceinline__ void state_back(const double *pr, const Geo<double> &
     }
     // u^0 = gamma / alpha, u^j = u~^j - gamma beta^j / alpha, beta^j = g^{0j} alpha^2
     // (1/alpha = sqrt(-g^tt); beta^j / alpha = g^{0j} alpha)
-    const double sg = d_sqrt(-gn[0]), alpha = 1. / sg;
+    const double sg = gm.rlapse, alpha = gm.lapse;
     double gb = a.ucon[0] * sg;
 #pragma unroll
     for (int j = 1; j < 4; j++) gb -= a.ucon[j] * (gn[j] * alpha);
     double ub3[3] = {a.ucon[1], a.ucon[2], a.ucon[3]};
     if (f.gfree) {
         const double u1 = pr[U1], u2 = pr[U2], u3 = pr[U3];
-        const double qb = 0.5 * gb / f.gam_l;   // gamma = sqrt(1 + q^2)
+        const double qb = 0.5 * gb * d_rcp(f.gam_l);   // gamma = sqrt(1 + q^2)
         ub3[0] += 2. * qb * (gc[4] * u1 + gc[5] * u2 + gc[6] * u3);
         ub3[1] += 2. * qb * (gc[5] * u1 + gc[7] * u2 + gc[8] * u3);
         ub3[2] += 2. * qb * (gc[6] * u1 + gc[8] * u2 + gc[9] * u3);
@@ -332,7 +332,7 @@ __device__ void state_vjp_from(const double *pr, const Geo<double> &gm, double g
         flux_rev<DIR>(pr, q, gm.g, eta, f.K, fb, a);
         // fast speeds: the roots of A v^2 - B v + C = 0 (forward in primtoflux)
         const double Acon_0 = gn[DIR], Asq = gn[DIR == 1 ? 4 : (DIR == 2 ? 7 : 9)], Bsq = gn[0], AB = Acon_0;
-        const double rw = 1. / w, reta = 1. / eta;
+        const double rw = d_rcp(w), reta = d_rcp(eta);
         const double cs2 = gam * (gam - 1.) * u * rw;
         const double va2 = bsq * reta;
         double cms2 = cs2 + va2 - cs2 * va2;
@@ -348,7 +348,7 @@ __device__ void state_vjp_from(const double *pr, const Geo<double> &gm, double g
         const bool dfree = !(discr < 0.);
         if (!dfree) discr = 0.;
         const double sq = d_sqrt(discr);
-        const double rA = 1. / A, r2A = 0.5 * rA;
+        const double rA = d_rcp(A), r2A = 0.5 * rA;
         const double vp = -(-B + sq) * r2A, vm = -(-B - sq) * r2A;
         const double vpb = (vp > vm ? cmxb : 0.) + (vp < vm ? cmnb : 0.);
         const double vmb = (vp > vm ? 0. : cmxb) + (vp < vm ? 0. : cmnb);
@@ -356,7 +356,7 @@ __device__ void state_vjp_from(const double *pr, const Geo<double> &gm, double g
         const double sb = (vmb - vpb) * r2A;
         double Ab = -(vpb * vp + vmb * vm) * rA, Cb = 0.;
         if (dfree && sq > 0.) {
-            const double Db = 0.5 * sb / sq;
+            const double Db = 0.5 * sb * d_rcp(sq);
             Bb += 2. * B * Db;
             Ab -= 4. * C * Db;
             Cb = -4. * A * Db;
@@ -488,7 +488,7 @@ __device__ __forceinline__ void adj_flux_face(const Dims &d, const Geom &m, cons
             const double cmin = on < 0. ? -on : on;
             // (the cotangents need no bit-level agreement with a reference:
             // one reciprocal of the HLL denominator for all 45 quotients)
-            const double rD = 1. / (cmax + cmin + SMALL_D);
+            const double rD = d_rcp(cmax + cmin + SMALL_D);
             // this side's flux and conserved-variable cotangents, and the
             // speeds' (which need both sides' fluxes)
             double tfb[NPR], tub[NPR], cmaxb = 0., cminb = 0.;
@@ -537,11 +537,12 @@ __device__ __forceinline__ void adj_flux_face(const Dims &d, const Geom &m, cons
 // two reverses, which only meet in atomics, fill the GPU together
 // build options: minimum resident blocks of 128 threads per SM for the
 // reverse kernels, which cap their registers: the 2-D torus gradient is
-// latency bound at low occupancy, and spilling beats it (face reverse at 5
-// blocks: 102 registers with spills against 230 without, 25 % on the whole
-// gradient; the state kernels another 1-2 %)
+// latency bound at low occupancy, and some spilling beats it (face reverse at
+// 3 blocks, with one reciprocal for the quotients that share a divisor: the
+// 256 x 256 gradient of 20 steps 9.6 -> 8.95 ms against 5 blocks; uncapped, 230
+// registers, was 25 % slower than 5; the state kernels another 1-2 %)
 #ifndef HAMR_ADJ_FLUX_MINB
-#define HAMR_ADJ_FLUX_MINB 5
+#define HAMR_ADJ_FLUX_MINB 3
 #endif
 #ifndef HAMR_ADJ_ZONE_MINB
 #define HAMR_ADJ_ZONE_MINB 4
@@ -574,13 +575,13 @@ __device__ __forceinline__ void adj_divergence_face(const Dims &d, const double 
     const int i = i0 + (int)(t / nj);
     const long c = cix(d, i, j, 0), ks = d.ks;
     const long stride = idel ? (long)d.G2 * d.G3 : (long)d.G3;
-    const double dx = DIR == 1 ? d.dx1 : d.dx2;
+    const double rdx = DIR == 1 ? d.rdx1 : d.rdx2;
     const bool ac = active_zone(d, i, j), am = active_zone(d, i - idel, j - jdel);
     for (int k = 0; k < NPR; k++) {
         if (k == B1 || k == B2) continue;
         double v = 0.;
-        if (ac) v += Dt * aW[k * ks + c] / dx;
-        if (am) v -= Dt * aW[k * ks + c - stride] / dx;
+        if (ac) v += Dt * aW[k * ks + c] * rdx;
+        if (am) v -= Dt * aW[k * ks + c - stride] * rdx;
         aF[k * ks + c] += v;
     }
     if (DIR == 1 && i == ih && j >= d.ng2 && j < d.ng2 + d.n2) aF[RHO * ks + c] += mdot_coef;
@@ -1255,11 +1256,26 @@ int fwd_step(hamr_adjoint *a, double dt) {
     });
 }
 
-// recorded step on the second stream; next_p/next_ps: where its output goes
-int rec_step(hamr_adjoint *a, double dt, double *slot, double *next_p, double *next_ps) {
-    return graph_run(a, a->rec_graph, {dt, slot, next_p}, a->s2, [&]() -> int {
+// recorded step on stream `run`; next_p/next_ps: where its output goes
+int rec_step(hamr_adjoint *a, cudaStream_t run, double dt, double *slot, double *next_p, double *next_ps) {
+    return graph_run(a, a->rec_graph, {dt, slot, next_p}, run, [&]() -> int {
         return record_step(a, dt, slot_of(slot, a->ctx->d.ks), next_p, next_ps);
     });
+}
+
+// what a recorded step that belongs to the forward sweep leaves in the context:
+// its two sub-steps' failure counts added, its last flags
+__global__ void k_adj_take_flags(const Dims d, const int *__restrict__ fih, const int *__restrict__ fif,
+                                 const int *__restrict__ flf, int *__restrict__ failimage, int *__restrict__ pflag) {
+    const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= (long)d.n1 * d.n2) return;
+    const int j = d.ng2 + (int)((unsigned)t % (unsigned)d.n2), i = d.ng1 + (int)((unsigned)t / (unsigned)d.n2);
+    const long c = cix(d, i, j, 0), ks = d.ks;
+    for (int q = 0; q < 4; q++) {
+        const int n = fih[q * ks + c] + fif[q * ks + c];
+        if (n) failimage[q * ks + c] += n;
+    }
+    pflag[c] = flf[c];
 }
 
 // reversed step from slot's record; next_p/next_ps: the step's output state
@@ -1382,11 +1398,14 @@ int hamr_mdot_forward(hamr_adjoint *a, int nsteps, const double *dt, double *J) 
 // Gradient of J = sum_n dt[n] Mdot_n over nsteps fixed-size steps with
 // respect to the initial state (active primitives and face field, before
 // the ghost fill) and the adiabatic index. Checkpoints the state every
-// `every` steps on the forward sweep, and reverses segment by segment: each
-// segment is recomputed from its checkpoint, recording every step's
-// intermediates, then its steps are reversed from those records (no forward
-// work in the reverse). Two banks of records let segment sg-1 be recomputed
-// on a second stream while segment sg is reversed on the context's stream.
+// `every` steps on the forward sweep, whose last segment records every step's
+// intermediates as it goes, and reverses segment by segment: each earlier
+// segment is recomputed from its checkpoint with records, and its steps are
+// reversed from those (no forward work in the reverse). Two banks of records
+// let segment sg-1 be recomputed on a second stream while segment sg is
+// reversed on the context's stream. (The last segment used to be swept and then
+// recomputed like the others, with nothing to overlap the recompute: on 256 x
+// 256 zones, 20 steps in one segment, 12.1 -> 9.6 ms.)
 // grad_p (9 planes) / grad_ps (3 planes) are host arrays in the context's
 // layout (NULL: not copied). The context's state is restored to its initial
 // value on return.
@@ -1438,9 +1457,24 @@ int hamr_adjoint_run(hamr_adjoint *a, int nsteps, const double *dt, int every, d
     // forward sweep with checkpoints
     ACK(cudaMemsetAsync(a->J, 0, sizeof(double), s));
     int rc = bound_ctx(ctx);
+    // segment sg uses bank sg % 2: record k of the segment is slot k of the
+    // bank, and its last step ends in the bank's `ends` state
+    auto slot = [&](int b, int k) { return a->slots[(size_t)b * a->bank_len + k]; };
+    const int nlast = (nseg - 1) * every, blast = (nseg - 1) & 1;
     for (int n = 0; n < nsteps && rc == HAMR_OK; n++) {
         if (n % every == 0) save(a->store[n / every]);
-        rc = fwd_step(a, dt[n]);
+        if (n < nlast) {
+            rc = fwd_step(a, dt[n]);
+            continue;
+        }
+        const int k = n - nlast;
+        if (k == 0) save(slot(blast, 0));   // a record begins with its step's input state, as `save` lays it out
+        double *nx = n + 1 < nsteps ? slot(blast, k + 1) : a->ends[blast];
+        if ((rc = rec_step(a, s, dt[n], slot(blast, k), nx, nx + NPR * d.ks))) break;
+        const Slot r = slot_of(slot(blast, k), d.ks);
+        k_mdot_accum<<<1, BLK, 0, s>>>(d, r.F1f, a->ih, dt[n], a->J);
+        k_adj_take_flags<<<nb((long)d.n1 * d.n2), BLK, 0, s>>>(d, r.fih, r.fif, r.flf, ctx->failimage, ctx->pflag);
+        ACK(cudaGetLastError());
     }
     if (rc) return rc;
     double Jval = 0.;
@@ -1448,9 +1482,6 @@ int hamr_adjoint_run(hamr_adjoint *a, int nsteps, const double *dt, int every, d
     ACK(cudaEventRecord(a->ev_sweep, s));
     ACK(cudaStreamWaitEvent(a->s2, a->ev_sweep, 0));
     if ((rc = hamr_adjoint_zero(a))) return rc;
-    // segment sg uses bank sg % 2: record k of the segment is slot k of the
-    // bank, and its last step ends in the bank's `ends` state
-    auto slot = [&](int b, int k) { return a->slots[(size_t)b * a->bank_len + k]; };
     auto recompute = [&](int sg) -> int {
         const int b = sg & 1, n0 = sg * every, n1 = n0 + every < nsteps ? n0 + every : nsteps;
         ACK(cudaStreamWaitEvent(a->s2, a->ev_rev[b], 0));   // the bank's previous segment is reversed
@@ -1459,7 +1490,7 @@ int hamr_adjoint_run(hamr_adjoint *a, int nsteps, const double *dt, int every, d
         for (int n = n0; n < n1; n++) {
             const int k = n - n0;
             double *nx = n + 1 < n1 ? slot(b, k + 1) : a->ends[b];
-            const int r = rec_step(a, dt[n], slot(b, k), nx, nx + NPR * d.ks);
+            const int r = rec_step(a, a->s2, dt[n], slot(b, k), nx, nx + NPR * d.ks);
             if (r) return r;
         }
         ACK(cudaEventRecord(a->ev_rec[b], a->s2));
@@ -1467,7 +1498,7 @@ int hamr_adjoint_run(hamr_adjoint *a, int nsteps, const double *dt, int every, d
     };
     auto reverse = [&](int sg) -> int {
         const int b = sg & 1, n0 = sg * every, n1 = n0 + every < nsteps ? n0 + every : nsteps;
-        ACK(cudaStreamWaitEvent(s, a->ev_rec[b], 0));
+        if (sg < nseg - 1) ACK(cudaStreamWaitEvent(s, a->ev_rec[b], 0));   // the last: recorded on this stream
         for (int n = n1 - 1; n >= n0; n--) {
             const int k = n - n0;
             const double *nx = n + 1 < n1 ? slot(b, k + 1) : a->ends[b];
@@ -1477,7 +1508,6 @@ int hamr_adjoint_run(hamr_adjoint *a, int nsteps, const double *dt, int every, d
         ACK(cudaEventRecord(a->ev_rev[b], s));
         return HAMR_OK;
     };
-    rc = recompute(nseg - 1);
     for (int sg = nseg - 1; sg >= 0 && rc == HAMR_OK; sg--) {
         if (sg >= 1 && (rc = recompute(sg - 1))) break;
         rc = reverse(sg);
