@@ -264,17 +264,6 @@ __device__ __forceinline__ void gamma_calc(const T *pr, const Geo<G> &gm, T *gam
     *gamma = d_sqrt(T(1.) + qsq);
 }
 
-template <typename T, typename G>
-__device__ __forceinline__ void ucon_calc(const T *pr, const Geo<G> &gm, T *ucon) {
-    const G alpha = gm.lapse;   // 1/sqrt(-g^tt), from the Geo (tabulated or geo_lapse)
-    G beta[4];
-    T gamma;
-    gamma_calc(pr, gm, &gamma);
-    if constexpr (std::is_same<T, double>::value && std::is_same<T, G>::value && !STRICT) {
-        ucon_hll(pr, gm, ucon);   // with the lapse and its reciprocal
-        return;
-    }
-#pragma unroll
 // u_mu, dot product, u^mu and b^mu of the HLL sides and the centre EMFs in both
 // precisions: fused sums, u~^i u~_i nested, one reciprocal and no division
 // (beta^j / alpha = alpha g^tj). The float face-frame solvers, whose star states
@@ -312,6 +301,17 @@ __device__ __forceinline__ void bcon_hll(const T *pr, const T *ucon, const T *uc
     for (int j = 1; j < 4; j++) bcon[j] = mul(mad(bcon[0], ucon[j], pr[B1 - 1 + j]), ru);
 }
 
+template <typename T, typename G>
+__device__ __forceinline__ void ucon_calc(const T *pr, const Geo<G> &gm, T *ucon) {
+    const G alpha = gm.lapse;   // 1/sqrt(-g^tt), from the Geo (tabulated or geo_lapse)
+    G beta[4];
+    T gamma;
+    gamma_calc(pr, gm, &gamma);
+    if constexpr (std::is_same<T, double>::value && std::is_same<T, G>::value && !STRICT) {
+        ucon_hll(pr, gm, ucon);   // with the lapse and its reciprocal
+        return;
+    }
+#pragma unroll
     for (int j = 1; j < 4; j++) beta[j] = gm.gcon[j] * alpha * alpha;
     if constexpr (std::is_same<T, G>::value) {
         const Divisor<T> da(alpha, gm.rlapse);   // four quotients by the lapse
