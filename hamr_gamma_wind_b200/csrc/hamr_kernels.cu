@@ -2,14 +2,19 @@
 // (include/hamr_b200.h) that drives them.
 //
 // One sub-step (the work of advance_GPU, step_ch.c:997-1335, for one block):
-//   k_flux<3>, k_flux<2>, k_flux<1>   PPM + HLL face fluxes and the directional
-//                                      CFL minimum (fluxcalcprep + fluxcalc2D2)
+//   k_flux_x3, k_flux_rows<2>, <1>     PPM + HLL face fluxes and the directional
+//                                      CFL minimum (fluxcalcprep + fluxcalc2D2);
+//                                      k_flux<2>, <1> on blocks too small for rows
 //   k_fix_flux                         reflective-pole flux rules (2-D)
 //   k_emf_centre, k_emf_edge           cell-centre and edge EMFs (consttransport1/2)
 //   k_pole_average                     phi-averaged polar EMF (E_average, 3-D)
 //   k_face_update                      staggered B update (consttransport3)
-//   k_cons, k_invert                   conserved update + source, inversion (fixup)
+//   k_cons_tma                         conserved update + source and primary inversion
+//                                      (fixup), k_invert_fallback for the failed zones;
+//                                      k_cons, k_invert_primary without bulk copies
 //   k_bound_x1/x3/x2                   ghost fill of the written state
+// and on small or 2-D blocks k_flux_2d, k_ct_2d and k_cons_inv, each for several
+// of these.
 // All arrays use the reference's structure-of-arrays layout; cell index
 // (i*G2 + j)*G3 + z puts phi (or x3) innermost, so consecutive threads touch
 // consecutive addresses.
