@@ -504,19 +504,21 @@ __device__ __forceinline__ bool is_pos(float x) { return x > 0.f; }
 //               three times), min(2|a|, 2|b|, |a + b|/2) with the sign of the
 //               centred difference, zero at an extremum. The doublings of the
 //               reference's form are folded into one exact scaling at the end
-//               (powers of two), which gives the same value bit for bit;
+//               (powers of two), which gives the same value bit for bit, NaNs
+//               included (tests/test_gpu_nan_reconstruction.py; in double a
+//               product of the differences below 2^-1042 counts as zero);
 //   ppm_face    the interpolated value between two zones, the upper edge of
 //               one and the lower edge of the next;
 //   ppm_limit   the monotonised edges of a zone from its value and the two.
 template <typename T>
 __device__ __forceinline__ T ppm_slope(T y0, T y1, T y2) {
     const T a = y1 - y0, b = y2 - y1, c = y2 - y0;
-    const T m = T(4.) * d_min(d_fabs(a), d_fabs(b));
-    const T v = T(0.5) * d_min(d_fabs(c), m);
+    const T m = d_min(d_fabs(c), T(4.) * d_min(d_fabs(a), d_fabs(b)));
     // the product's sign; in float scaled as the reference's, so that it
     // underflows no earlier
     const T s = sizeof(T) == 4 ? (T(4.) * a) * b : a * b;
-    return is_pos(s) ? (is_pos(c) ? v : -v) : T(0.);
+    // a product at an extremum too, whose factor is zero there: a NaN stays one
+    return (is_pos(c) ? m : -m) * (is_pos(s) ? T(0.5) : T(0.));
 }
 template <typename T>
 __device__ __forceinline__ T ppm_face(T y1, T y2, T dq1, T dq2) {
