@@ -300,7 +300,7 @@ __device__ __forceinline__ double flux_face(const Dims &d, const Geom &m, const 
             T x[6];
 #pragma unroll
             for (int s = 0; s < 6; s++) x[s] = (T)__ldg(pk + (s - 3) * stride);
-            para_face(x, pl[k], pr[k]);   // upper edge of zone c-1, lower edge of zone c
+            para_face<(REC & 2) != 0>(x, pl[k], pr[k]);   // upper edge of zone c-1, lower edge of zone c
         }
     }
     if constexpr (!FIX) {
@@ -458,7 +458,7 @@ __device__ __forceinline__ void zone_edges(const Dims &d, const double *__restri
             T x[5];
 #pragma unroll
             for (int s = 0; s < 5; s++) x[s] = (T)__ldg(pk + (s - 2) * stride);
-            para(x, lo[k], hi[k]);
+            para<(REC & 2) != 0>(x, lo[k], hi[k]);
         }
     }
 }
@@ -513,26 +513,32 @@ __host__ __device__ __forceinline__ long n_x3_slots(const Dims &d) {
 #endif
 
 // cell-centre EMF, -gdet (u x b), of a zone with primitives pb (velocities and
-// field) in column (i, j): e[0..2] = E1, E2, E3 (E1, E2 only in 3-D)
-template <typename T>
+// field) in column (i, j): e[0..2] = E1, E2, E3 (E1, E2 only in 3-D). FT: the
+// step of a face-frame solver.
+template <typename T, bool FT>
 __device__ __forceinline__ void emf_centre_of(const Dims &d, const Geom &m, const T *pb, int i, int j, T *e) {
     Geo<T> gm;
     load_geo_t(d, m, i, j, CENT, gm);
     T ucon[4], ucov[4], bcon[4];
-    if constexpr (std::is_same<T, double>::value && STRICT) {
+    if constexpr (plain_forms<T, FT>) {
         ucon_calc(pb, gm, ucon);
         lower4(ucon, gm.gcov, ucov);
         bcon_calc(pb, ucon, ucov, bcon);
+        if (d.ng3 > 0) {
+            e[0] = -gm.g * (ucon[2] * bcon[3] - ucon[3] * bcon[2]);
+            e[1] = -gm.g * (ucon[3] * bcon[1] - ucon[1] * bcon[3]);
+        }
+        e[2] = -gm.g * (ucon[1] * bcon[2] - ucon[2] * bcon[1]);
     } else {
         ucon_hll(pb, gm, ucon);
         lower_hll(ucon, gm.gcov, ucov);
         bcon_hll(pb, ucon, ucov, bcon);
+        if (d.ng3 > 0) {
+            e[0] = -gm.g * mad(ucon[2], bcon[3], -mul(ucon[3], bcon[2]));
+            e[1] = -gm.g * mad(ucon[3], bcon[1], -mul(ucon[1], bcon[3]));
+        }
+        e[2] = -gm.g * mad(ucon[1], bcon[2], -mul(ucon[2], bcon[1]));
     }
-    if (d.ng3 > 0) {
-        e[0] = -gm.g * mad(ucon[2], bcon[3], -mul(ucon[3], bcon[2]));
-        e[1] = -gm.g * mad(ucon[3], bcon[1], -mul(ucon[1], bcon[3]));
-    }
-    e[2] = -gm.g * mad(ucon[1], bcon[2], -mul(ucon[2], bcon[1]));
 }
 template <typename T>
 __device__ __forceinline__ void emf_centre_eval(const Dims &d, const Geom &m, const double *__restrict__ pv, int i,
@@ -549,6 +555,7 @@ __device__ __forceinline__ double flux_x3_slots(const Dims &d, const Geom &m, co
                                                 const double *__restrict__ ps, T *__restrict__ F,
                                                 T *__restrict__ Ec, long blk) {
     constexpr int H = X3Slots<REC>::H, STEP = X3Slots<REC>::STEP;
+    constexpr bool FT = (REC & 2) != 0;
     constexpr int NK = NPR - 1;            // B3 is not reconstructed
     __shared__ T sa[NK][BLK], sb[NK][BLK]; // PPM: slopes, then lower edges | face values; MC: lower edges
     const int l = threadIdx.x;
@@ -587,14 +594,14 @@ __device__ __forceinline__ double flux_x3_slots(const Dims &d, const Geom &m, co
         __syncthreads();
         if (l < BLK - 1 && sl + 1 < nslot)
 #pragma unroll
-            for (int q = 0; q < NK; q++) sb[q][l] = ppm_face(y0[q], y1[q], sa[q][l], sa[q][l + 1]);
+            for (int q = 0; q < NK; q++) sb[q][l] = ppm_face<FT>(y0[q], y1[q], sa[q][l], sa[q][l + 1]);
         __syncthreads();
         if (l > 0 && l < BLK - 1 && sl + 1 < nslot)
 #pragma unroll
             for (int k = 0, q = 0; k < NPR; k++) {
                 if (k == B3) continue;
                 T lo;
-                ppm_limit(y0[q], sb[q][l - 1], sb[q][l], lo, hi[k]);
+                ppm_limit<FT>(y0[q], sb[q][l - 1], sb[q][l], lo, hi[k]);
                 sa[q++][l] = lo;
             }
     }
@@ -608,7 +615,7 @@ __device__ __forceinline__ double flux_x3_slots(const Dims &d, const Geom &m, co
             T pb[NPR];
 #pragma unroll
             for (int k = 0, q = 0; k < NPR; k++) pb[k] = k == B3 ? (T)__ldg(pv + (long)k * d.ks + c) : y0[q++];
-            emf_centre_of(d, m, pb, i, j, e);
+            emf_centre_of<T, FT>(d, m, pb, i, j, e);
         }
         Ec[1 * d.ks + c] = e[0];
         Ec[2 * d.ks + c] = e[1];
@@ -711,7 +718,7 @@ struct RowWindow {
                 at(0, kk) = y0;
                 at(1, kk) = yp;
                 at(2, kk) = dq;
-                at(3, kk) = ppm_face(ym, y0, ppm_slope(yl, ym, y0), dq);
+                at(3, kk) = ppm_face<(REC & 2) != 0>(ym, y0, ppm_slope(yl, ym, y0), dq);
             }
             kk++;
         }
@@ -735,8 +742,8 @@ struct RowWindow {
             } else {
                 const T y0 = at(par, kk), yp = at(1 - par, kk);
                 const T dq = ppm_slope(y0, yp, yn);
-                const T f = ppm_face(y0, yp, at(2, kk), dq);
-                ppm_limit(y0, at(3, kk), f, lo[k], hi[k]);
+                const T f = ppm_face<(REC & 2) != 0>(y0, yp, at(2, kk), dq);
+                ppm_limit<(REC & 2) != 0>(y0, at(3, kk), f, lo[k], hi[k]);
                 at(par, kk) = yn;
                 at(2, kk) = dq;
                 at(3, kk) = f;
@@ -870,7 +877,8 @@ __device__ __forceinline__ void emf_centre_eval(const Dims &d, const Geom &m, co
     T pb[NPR];
 #pragma unroll
     for (int k = U1; k <= B3; k++) pb[k] = (T)__ldg(&pv[k * d.ks + c]);
-    emf_centre_of(d, m, pb, i, j, e);
+    if (sizeof(T) == sizeof(float) && d.riemann != HAMR_RIEMANN_HLL) emf_centre_of<T, true>(d, m, pb, i, j, e);
+    else emf_centre_of<T, false>(d, m, pb, i, j, e);
 }
 
 // on the active zones plus one ghost layer
@@ -2831,14 +2839,16 @@ void launch_flux_2d(cudaStream_t s, const Dims &d, const Geom &m, const double *
     auto run = [&](auto plain, auto fixed) {
         (fix ? fixed : plain)<<<nb, BLK, 0, s>>>(d, m, pin, psin, F1, F2, Ec, dtbits, cd, nb1, nb2);
     };
-    switch (rec_key(d)) {
-    case 1: run(k_flux_2d<T, 1, false>, k_flux_2d<T, 1, true>); break;
-    case 2: run(k_flux_2d<T, 2, false>, k_flux_2d<T, 2, true>); break;
-    case 3: run(k_flux_2d<T, 3, false>, k_flux_2d<T, 3, true>); break;
-    case 6: run(k_flux_2d<T, 6, false>, k_flux_2d<T, 6, true>); break;
-    case 7: run(k_flux_2d<T, 7, false>, k_flux_2d<T, 7, true>); break;
-    default: run(k_flux_2d<T, 0, false>, k_flux_2d<T, 0, true>); break;
+    if constexpr (sizeof(T) == sizeof(double)) {   // the float face-frame solvers run their own kernels (launch_stage_t)
+        switch (rec_key(d)) {
+        case 2: run(k_flux_2d<T, 2, false>, k_flux_2d<T, 2, true>); return;
+        case 3: run(k_flux_2d<T, 3, false>, k_flux_2d<T, 3, true>); return;
+        case 6: run(k_flux_2d<T, 6, false>, k_flux_2d<T, 6, true>); return;
+        case 7: run(k_flux_2d<T, 7, false>, k_flux_2d<T, 7, true>); return;
+        }
     }
+    if (d.recon == HAMR_RECON_MC) run(k_flux_2d<T, 1, false>, k_flux_2d<T, 1, true>);
+    else run(k_flux_2d<T, 0, false>, k_flux_2d<T, 0, true>);
 }
 
 // the bulk copies of k_cons_tma need 16-byte aligned flux planes
@@ -2871,8 +2881,10 @@ int launch_stage_t(hamr_ctx *ctx, int full, StepSize st, bool calc_dt, Prof *pf,
     const bool ec_x3 = d.d3 && !ctx->ct_fused && ctx->emf_in_x3;
     // a 2-D block whose faces do not fill the device: one launch for both
     // directions' fluxes, their polar and radial rules and the centre EMFs, one
-    // for the edge EMF and the face update
-    const bool flat = !d.d3 && !conc && n_flux_rows<1>(d) < ctx->rows_min && n_flux_rows<2>(d) < ctx->rows_min;
+    // for the edge EMF and the face update. Not in the float step of the face-frame
+    // solvers: the compiler contracts them otherwise there (plain_forms)
+    const bool plain_2d = sizeof(T) == sizeof(float) && d.riemann != HAMR_RIEMANN_HLL;
+    const bool flat = !d.d3 && !plain_2d && !conc && n_flux_rows<1>(d) < ctx->rows_min && n_flux_rows<2>(d) < ctx->rows_min;
     if (conc) {
         CK(cudaEventRecord(ctx->ev[0], s));
         CK(cudaStreamWaitEvent(s2, ctx->ev[0], 0));

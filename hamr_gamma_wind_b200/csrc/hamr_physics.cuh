@@ -56,6 +56,16 @@ __device__ __forceinline__ float mad(float a, float b, float c) { return STRICT 
 __device__ __forceinline__ double mul(double a, double b) { return STRICT ? a * b : __dmul_rn(a, b); }
 __device__ __forceinline__ float mul(float a, float b) { return STRICT ? a * b : __fmul_rn(a, b); }
 
+// Which of two forms a formula takes. The plain one, the reference's text with
+// whatever the compiler contracts in it: the strict build (which contracts
+// nothing), and the float step of the face-frame solvers (FT: HLLC, HLLD), whose
+// contact speed is the cancelling root of a quadratic: there a changed last bit
+// of an edge value or of an EMF moves u^2 by up to 1e-3 of its norm in a step, so
+// their float arithmetic stays as it is, bit for bit (tests/test_gpu_mixed_face_frame.py).
+// Everything else takes the shorter form, its fused operations spelled out.
+template <typename T, bool FT>
+constexpr bool plain_forms = STRICT || (FT && sizeof(T) == sizeof(float));
+
 template <typename T>
 struct Geo {
     T gcov[10], gcon[10], g;
@@ -520,41 +530,86 @@ __device__ __forceinline__ T ppm_slope(T y0, T y1, T y2) {
     // a product at an extremum too, whose factor is zero there: a NaN stays one
     return (is_pos(c) ? m : -m) * (is_pos(s) ? T(0.5) : T(0.));
 }
-template <typename T>
+template <bool FT, typename T>
 __device__ __forceinline__ T ppm_face(T y1, T y2, T dq1, T dq2) {
-    return mad(T(0.5), y2 + y1, -div6(dq2 - dq1));
+    if constexpr (plain_forms<T, FT>) return T(0.5) * (y2 + y1) - div6(dq2 - dq1);
+    else return mad(T(0.5), y2 + y1, -div6(dq2 - dq1));
 }
-template <typename T>
+template <bool FT, typename T>
 __device__ __forceinline__ void ppm_limit(T y, T l, T r, T &lout, T &rout) {
     const T qa = (r - y) * (y - l);
     const T qd = (r - l);
-    const T qe = mul(T(6.0), mad(T(-0.5), l + r, y));
-    if (qa <= T(0.)) { l = y; r = y; }
-    if (is_neg(qd * (qd - qe))) l = mad(T(3.0), y, T(-2.0) * r);
-    else if (is_neg(qd * (qd + qe))) r = mad(T(3.0), y, T(-2.0) * l);
+    if constexpr (plain_forms<T, FT>) {
+        const T qe = T(6.0) * (y - T(0.5) * (l + r));
+        if (qa <= T(0.)) { l = y; r = y; }
+        if (qd * (qd - qe) < T(0.0)) l = T(3.0) * y - T(2.0) * r;
+        else if (qd * (qd + qe) < T(0.0)) r = T(3.0) * y - T(2.0) * l;
+    } else {
+        const T qe = mul(T(6.0), mad(T(-0.5), l + r, y));
+        if (qa <= T(0.)) { l = y; r = y; }
+        if (is_neg(qd * (qd - qe))) l = mad(T(3.0), y, T(-2.0) * r);
+        else if (is_neg(qd * (qd + qe))) r = mad(T(3.0), y, T(-2.0) * l);
+    }
     lout = l;
     rout = r;
 }
 
-// PPM face values of the middle of five zones: l = lower edge, r = upper edge
+// the plain form of a whole zone: the same values as the three parts, but
+// sharing no part with another zone. How the compiler contracts the solver that
+// follows depends on the code before it, and this is the text that goes with
+// the bits above.
 template <typename T>
+__device__ __forceinline__ void para_plain(const T *y, T &lout, T &rout) {
+    T dq[5];
+#pragma unroll
+    for (int i = 1; i < 4; i++) {
+        T Dqm = T(2.) * (y[i] - y[i - 1]);
+        T Dqp = T(2.) * (y[i + 1] - y[i]);
+        T Dqc = T(0.5) * (y[i + 1] - y[i - 1]);
+        T aDqm = d_fabs(Dqm), aDqp = d_fabs(Dqp), aDqc = d_fabs(Dqc);
+        T s = Dqm * Dqp;
+        Dqm = d_min(aDqm, aDqp);
+        if (aDqc < Dqm) {
+            if (Dqc > T(0.)) dq[i] = (aDqc) * (T)(s > T(0.));
+            else dq[i] = (-aDqc) * (T)(s > T(0.));
+        } else {
+            if (Dqc > T(0.)) dq[i] = (Dqm) * (T)(s > T(0.));
+            else dq[i] = (-Dqm) * (T)(s > T(0.));
+        }
+    }
+    const T l = T(0.5) * (y[2] + y[1]) - div6(dq[2] - dq[1]);
+    const T r = T(0.5) * (y[3] + y[2]) - div6(dq[3] - dq[2]);
+    ppm_limit<true>(y[2], l, r, lout, rout);
+}
+
+// PPM face values of the middle of five zones: l = lower edge, r = upper edge
+template <bool FT = false, typename T>
 __device__ __forceinline__ void para(const T *y, T &lout, T &rout) {
-    const T d1 = ppm_slope(y[0], y[1], y[2]), d2 = ppm_slope(y[1], y[2], y[3]), d3 = ppm_slope(y[2], y[3], y[4]);
-    ppm_limit(y[2], ppm_face(y[1], y[2], d1, d2), ppm_face(y[2], y[3], d2, d3), lout, rout);
+    if constexpr (plain_forms<T, FT>) {
+        para_plain(y, lout, rout);
+    } else {
+        const T d1 = ppm_slope(y[0], y[1], y[2]), d2 = ppm_slope(y[1], y[2], y[3]), d3 = ppm_slope(y[2], y[3], y[4]);
+        ppm_limit<FT>(y[2], ppm_face<FT>(y[1], y[2], d1, d2), ppm_face<FT>(y[2], y[3], d2, d3), lout, rout);
+    }
 }
 
 // the two states at the face between the third and fourth of six zones: the
 // upper edge of the third (hi2) and the lower edge of the fourth (lo3)
-template <typename T>
+template <bool FT, typename T>
 __device__ __forceinline__ void para_face(const T *y, T &hi2, T &lo3) {
-    T dq[4];
-#pragma unroll
-    for (int k = 0; k < 4; k++) dq[k] = ppm_slope(y[k], y[k + 1], y[k + 2]);
-    const T f1 = ppm_face(y[1], y[2], dq[0], dq[1]), f2 = ppm_face(y[2], y[3], dq[1], dq[2]),
-            f3 = ppm_face(y[3], y[4], dq[2], dq[3]);
     T drop;
-    ppm_limit(y[2], f1, f2, drop, hi2);
-    ppm_limit(y[3], f2, f3, lo3, drop);
+    if constexpr (plain_forms<T, FT>) {
+        para_plain(y, drop, hi2);
+        para_plain(y + 1, lo3, drop);
+    } else {
+        T dq[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) dq[k] = ppm_slope(y[k], y[k + 1], y[k + 2]);
+        const T f1 = ppm_face<FT>(y[1], y[2], dq[0], dq[1]), f2 = ppm_face<FT>(y[2], y[3], dq[1], dq[2]),
+                f3 = ppm_face<FT>(y[3], y[4], dq[2], dq[3]);
+        ppm_limit<FT>(y[2], f1, f2, drop, hi2);
+        ppm_limit<FT>(y[3], f2, f3, lo3, drop);
+    }
 }
 
 // ---------------------------------------------------------------- inversion
