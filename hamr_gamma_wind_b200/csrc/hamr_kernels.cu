@@ -1510,7 +1510,7 @@ __device__ __forceinline__ void cons_update_fx(const Dims &d, const Geom &m, con
     if (!full) {
 #pragma unroll
         for (int k = 0; k < NPR; k++) { pf[k] = 0.0; pf[k] += (1.0 / ((double)1)) * pin[k * ks + c]; }
-        get_state(pf, gm, q);
+        get_state<true>(pf, gm, q);
         double vd;
         primtoflux(d.gam, pf, q, 0, gm, entropy(d.gam, pf), U, &vd, &vd);
 #pragma unroll

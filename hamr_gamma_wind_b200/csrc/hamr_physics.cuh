@@ -229,13 +229,15 @@ struct Divisor {
     }
 };
 
-// the same with IEEE quotients in both builds: HLLD's pressure solve differences
-// a residual over a relative step of 1e-10, so the last bits of its quotients
-// are what its root is good to
+// the same with IEEE quotients in both builds: the conserved variables' u^t
+// (ucon_calc), and HLLD's pressure solve, which differences a residual over a
+// relative step of 1e-10, so that the last bits of its quotients are what its
+// root is good to
 template <typename T>
 struct ExactDivisor {
     T b, rb;
     __device__ __forceinline__ explicit ExactDivisor(T b_) : b(b_), rb(T(1.0) / b_) {}
+    __device__ __forceinline__ ExactDivisor(T b_, T rb_) : b(b_), rb(rb_) {}
     __device__ __forceinline__ T div(T a) const {
         if constexpr (std::is_same<T, double>::value) return div_rcp_inf(a, b, rb);
         else return a / b;
@@ -311,27 +313,32 @@ __device__ __forceinline__ void bcon_hll(const T *pr, const T *ucon, const T *uc
     for (int j = 1; j < 4; j++) bcon[j] = mul(mad(bcon[0], ucon[j], pr[B1 - 1 + j]), ru);
 }
 
-template <typename T, typename G>
+// u^mu of a state. The production build's double form is ucon_hll, save for the
+// conserved variables that the update starts from (CONS), whose quotients by
+// alpha are exact in both builds: the inversion multiplies u^t by alpha again,
+// and a product with the rounded 1/alpha would scale a column's mass by the same
+// last bit every step (tests/test_gpu_column_mass.py).
+template <bool CONS = false, typename T, typename G>
 __device__ __forceinline__ void ucon_calc(const T *pr, const Geo<G> &gm, T *ucon) {
     const G alpha = gm.lapse;   // 1/sqrt(-g^tt), from the Geo (tabulated or geo_lapse)
-    G beta[4];
-    T gamma;
-    gamma_calc(pr, gm, &gamma);
-    if constexpr (std::is_same<T, double>::value && std::is_same<T, G>::value && !STRICT) {
-        ucon_hll(pr, gm, ucon);   // with the lapse and its reciprocal
-        return;
-    }
-#pragma unroll
-    for (int j = 1; j < 4; j++) beta[j] = gm.gcon[j] * alpha * alpha;
-    if constexpr (std::is_same<T, G>::value) {
-        const Divisor<T> da(alpha, gm.rlapse);   // four quotients by the lapse
-        ucon[0] = da.div(gamma);
-#pragma unroll
-        for (int j = 1; j < 4; j++) ucon[j] = pr[U1 + j - 1] - da.div(gamma * beta[j]);
+    if constexpr (std::is_same<T, double>::value && std::is_same<T, G>::value && !STRICT && !CONS) {
+        ucon_hll(pr, gm, ucon);
     } else {
-        ucon[0] = gamma / alpha;
+        G beta[4];
+        T gamma;
+        gamma_calc(pr, gm, &gamma);
 #pragma unroll
-        for (int j = 1; j < 4; j++) ucon[j] = pr[U1 + j - 1] - gamma * beta[j] / alpha;
+        for (int j = 1; j < 4; j++) beta[j] = gm.gcon[j] * alpha * alpha;
+        if constexpr (std::is_same<T, G>::value) {
+            const ExactDivisor<T> da(alpha, gm.rlapse);   // four quotients by the lapse
+            ucon[0] = da.div(gamma);
+#pragma unroll
+            for (int j = 1; j < 4; j++) ucon[j] = pr[U1 + j - 1] - da.div(gamma * beta[j]);
+        } else {
+            ucon[0] = gamma / alpha;
+#pragma unroll
+            for (int j = 1; j < 4; j++) ucon[j] = pr[U1 + j - 1] - gamma * beta[j] / alpha;
+        }
     }
 }
 
@@ -343,9 +350,9 @@ __device__ __forceinline__ void bcon_calc(const T *pr, const T *ucon, const T *u
     for (int j = 1; j < 4; j++) bcon[j] = du.div(pr[B1 - 1 + j] + bcon[0] * ucon[j]);
 }
 
-template <typename T, typename G>
+template <bool CONS = false, typename T, typename G>
 __device__ __forceinline__ void get_state(const T *pr, const Geo<G> &gm, State<T> &q) {
-    ucon_calc(pr, gm, q.ucon);
+    ucon_calc<CONS>(pr, gm, q.ucon);
     lower4(q.ucon, gm.gcov, q.ucov);
     bcon_calc(pr, q.ucon, q.ucov, q.bcon);
     lower4(q.bcon, gm.gcov, q.bcov);
