@@ -2673,13 +2673,14 @@ struct hamr_ctx {
     // zones up to which the update without bulk copies takes the
     // inversion into its kernel (HAMR_CONS_INV_MAX overrides)
     long cons_inv_max = 1L << 17;
-    // the primary inversion inside the TMA-staged update kernel (no floors or
-    // repair; HAMR_FUSE_INV=0 keeps the separate inversion kernel)
+    // the primary inversion inside the TMA-staged update kernel (not with the
+    // reset of failed zones; HAMR_FUSE_INV=0 keeps the separate inversion kernel)
     bool fuse_inv = true;
     cudaStream_t side[2] = {nullptr, nullptr};
     cudaEvent_t ev[5] = {};
     std::string err;
-    // device state
+    // device state: all of it within one allocation
+    char *slab = nullptr;
     double *p = nullptr, *ph = nullptr, *ps = nullptr, *psh = nullptr, *U = nullptr;
     double *F1 = nullptr, *F2 = nullptr, *F3 = nullptr, *Ec = nullptr, *emf = nullptr;
     double *W = nullptr;  // updated conserved variables between k_cons and k_invert
@@ -2811,22 +2812,39 @@ void launch_flux(long n, cudaStream_t s, const Dims &d, const Geom &m, const dou
     }
 }
 
-// the TMA-staged update's shared memory for rows of up to 256 zones (as the
-// launch picks the kernel: short rows and long ones)
+// the TMA-staged update with the primary inversion inside, for rows cut in
+// pieces of lpiece zones
 template <typename T>
-void cons_tma_attributes() {
+using ConsTma = void (*)(const Dims, const Geom, const double *, const double *, double *, const T *, const T *,
+                         const T *, double *, int, StepSize, int *, int *, int, int, const double *, double *, int *,
+                         int *, int *);
+template <typename T>
+ConsTma<T> cons_tma_fused(int inversion, int fix, int lpiece) {
     constexpr int S = cons_tma_minb<T>(1, true), L = cons_tma_minb<T>(1, false);
+    constexpr int I2 = HAMR_INV_2D + 1, IN = HAMR_INV_NM + 1;
+    static const ConsTma<T> table[2][2][2] = {
+        {{k_cons_tma<T, I2, L>, k_cons_tma<T, I2, S>}, {k_cons_tma<T, I2, L, FIX_FLOORS>, k_cons_tma<T, I2, S, FIX_FLOORS>}},
+        {{k_cons_tma<T, IN, L>, k_cons_tma<T, IN, S>}, {k_cons_tma<T, IN, L, FIX_FLOORS>, k_cons_tma<T, IN, S, FIX_FLOORS>}}};
+    return table[inversion == HAMR_INV_NM][fix != 0][lpiece <= CONS_SHORT_ROW];
+}
+
+// pieces of at most 256 zones that the TMA-staged update cuts a row into
+inline int cons_pieces(const Dims &d) { return (d.n3 + 255) / 256; }
+inline int cons_piece_zones(const Dims &d) { return (d.n3 + cons_pieces(d) - 1) / cons_pieces(d); }
+
+// shared memory of the TMA-staged update's kernels that this block may launch,
+// up to the longest piece each takes (the same for every block, so that one's
+// setting does not undercut another's)
+template <typename T>
+cudaError_t cons_tma_attributes(const Dims &d, int fix) {
+    if (!d.d3 || d.n3 < 32) return cudaSuccess;
+    const int lpiece = cons_piece_zones(d);
     const int all = cons_tma_layout<T>(256).total, few = cons_tma_layout<T>(CONS_SHORT_ROW).total;
-    auto set = [](auto *k, int bytes) { cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes); };
-    set(k_cons_tma<T>, all);
-    set(k_cons_tma<T, HAMR_INV_2D + 1, L>, all);
-    set(k_cons_tma<T, HAMR_INV_NM + 1, L>, all);
-    set(k_cons_tma<T, HAMR_INV_2D + 1, L, FIX_FLOORS>, all);
-    set(k_cons_tma<T, HAMR_INV_NM + 1, L, FIX_FLOORS>, all);
-    set(k_cons_tma<T, HAMR_INV_2D + 1, S, FIX_FLOORS>, few);
-    set(k_cons_tma<T, HAMR_INV_NM + 1, S, FIX_FLOORS>, few);
-    set(k_cons_tma<T, HAMR_INV_2D + 1, S>, few);
-    set(k_cons_tma<T, HAMR_INV_NM + 1, S>, few);
+    constexpr auto smem = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    const ConsTma<T> alone = k_cons_tma<T>;
+    const cudaError_t e = cudaFuncSetAttribute(alone, smem, all);
+    if (e != cudaSuccess || (fix & FIX_RESET)) return e;   // the reset keeps the separate inversion
+    return cudaFuncSetAttribute(cons_tma_fused<T>(d.inversion, fix, lpiece), smem, lpiece <= CONS_SHORT_ROW ? few : all);
 }
 
 // fluxes of both directions and centre EMFs of a 2-D block (k_flux_2d)
@@ -2982,22 +3000,14 @@ int launch_stage_t(hamr_ctx *ctx, int full, StepSize st, bool calc_dt, Prof *pf,
         // kernel
         const bool small = !tma && !conc && ctx->fuse_inv && n <= ctx->cons_inv_max;
         if (tma) {   // one row of zones per CTA, flux operands staged by bulk copies
-            const int npiece = (d.n3 + 255) / 256, lpiece = (d.n3 + npiece - 1) / npiece;
+            const int npiece = cons_pieces(d), lpiece = cons_piece_zones(d);
             const dim3 grid(d.n1 * d.n2 * npiece), block((lpiece + 31) / 32 * 32);
             const size_t sm = cons_tma_layout<T>(lpiece).total;
             if (fuse) {
                 CK(cudaMemsetAsync(ctx->nfail, 0, sizeof(int), s));
-                constexpr int S = cons_tma_minb<T>(1, true), L = cons_tma_minb<T>(1, false);
-                auto pick = [&](auto k2d, auto knm) { return nm ? knm : k2d; };
-                constexpr int I2 = HAMR_INV_2D + 1, IN = HAMR_INV_NM + 1;
-                const bool brief = lpiece <= CONS_SHORT_ROW;
-                auto kf = fix ? (brief ? pick(k_cons_tma<T, I2, S, FIX_FLOORS>, k_cons_tma<T, IN, S, FIX_FLOORS>)
-                                       : pick(k_cons_tma<T, I2, L, FIX_FLOORS>, k_cons_tma<T, IN, L, FIX_FLOORS>))
-                              : (brief ? pick(k_cons_tma<T, I2, S>, k_cons_tma<T, IN, S>)
-                                       : pick(k_cons_tma<T, I2, L>, k_cons_tma<T, IN, L>));
-                kf<<<grid, block, sm, s>>>(d, m, ctx->p, pg, ctx->U, F1, F2, F3, ctx->W, full, st, ctx->nfail,
-                                           ctx->kerr, npiece, lpiece, psf, pout, ctx->pflag, ctx->failimage,
-                                           ctx->flist);
+                cons_tma_fused<T>(d.inversion, fix, lpiece)<<<grid, block, sm, s>>>(
+                    d, m, ctx->p, pg, ctx->U, F1, F2, F3, ctx->W, full, st, ctx->nfail, ctx->kerr, npiece, lpiece,
+                    psf, pout, ctx->pflag, ctx->failimage, ctx->flist);
             } else {
                 k_cons_tma<T><<<grid, block, sm, s>>>(d, m, ctx->p, pg, ctx->U, F1, F2, F3, ctx->W, full, st,
                                                       ctx->nfail, ctx->kerr, npiece, lpiece);
@@ -3179,22 +3189,32 @@ int hamr_ctx_create(const hamr_params *prm, hamr_ctx **out) {
         {(void **)&ctx->rcount, prm->repair == 2 ? sizeof(int) : 0},
         {(void **)&ctx->flist, sizeof(int) * d.n1 * d.n2 * d.n3}, {(void **)&ctx->nfail, sizeof(int)}};
     if (prm->repair == 2 && d.ks > 0x7fffffffL) { hamr_ctx_destroy(ctx); return HAMR_E_ARG; }
-    for (auto &a : allocs) {
-        if (a.n == 0) continue;
-        if (cudaMalloc(a.p, a.n) != cudaSuccess) {
-            hamr_ctx_destroy(ctx);
-            return HAMR_E_NOMEM;
-        }
-        cudaMemsetAsync(*a.p, 0, a.n, ctx->stream);
+    // one allocation, each array on a 256-byte boundary of it: creating and
+    // destroying a mixed block of 64^3 zones takes 0.5 and 0.4 ms, 5.8 and 4.9
+    // with an allocation per array
+    auto padded = [](size_t n) { return (n + 255) & ~(size_t)255; };
+    size_t total = 0;
+    for (const auto &a : allocs) total += padded(a.n);
+    if (cudaMalloc((void **)&ctx->slab, total) != cudaSuccess) {
+        ctx->slab = nullptr;
+        hamr_ctx_destroy(ctx);
+        return HAMR_E_NOMEM;
+    }
+    cudaMemsetAsync(ctx->slab, 0, total, ctx->stream);
+    char *at = ctx->slab;
+    for (const auto &a : allocs) {
+        if (a.n) *a.p = at;
+        at += padded(a.n);
     }
     ctx->ndt = &ctx->words->ndt;   // device addresses
     ctx->dt_state = &ctx->words->dt_state;
     ctx->kerr = &ctx->words->kerr;
     ctx->counter = &ctx->words->counter;
     k_dt_reset<<<1, 32, 0, ctx->stream>>>(ctx->dtbits);
-    cons_tma_attributes<double>();
-    cons_tma_attributes<float>();
-    if (cudaStreamSynchronize(ctx->stream) != cudaSuccess) {
+    const int fix = (prm->floors ? FIX_FLOORS : 0) | (prm->repair == 1 ? FIX_RESET : 0);
+    const cudaError_t attr = prm->precision == HAMR_MIXED ? cons_tma_attributes<float>(d, fix)
+                                                          : cons_tma_attributes<double>(d, fix);
+    if (attr != cudaSuccess || cudaStreamSynchronize(ctx->stream) != cudaSuccess) {
         hamr_ctx_destroy(ctx);
         return HAMR_E_CUDA;
     }
@@ -3206,12 +3226,7 @@ int hamr_ctx_destroy(hamr_ctx *ctx) {
     if (!ctx) return HAMR_E_ARG;
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
     if (ctx->graph) cudaGraphExecDestroy(ctx->graph);
-    void *bufs[] = {ctx->p, ctx->ph, ctx->ps, ctx->psh, ctx->U, ctx->F1, ctx->F2, ctx->F3, ctx->Ec, ctx->emf,
-                    ctx->W, ctx->pflag, ctx->failimage, ctx->gcov, ctx->gcon, ctx->gdet, ctx->conn, ctx->itab,
-                    ctx->gtab, ctx->gtabf, ctx->dtbits,
-                    ctx->words, ctx->divb, ctx->rlist, ctx->rcount, ctx->flist, ctx->nfail};
-    for (void *b : bufs)
-        if (b) cudaFree(b);
+    if (ctx->slab) cudaFree(ctx->slab);
     for (auto st : ctx->side)
         if (st) cudaStreamDestroy(st);
     for (auto ev : ctx->ev)
