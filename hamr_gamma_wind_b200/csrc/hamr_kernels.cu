@@ -3067,7 +3067,10 @@ int launch_stage_t(hamr_ctx *ctx, int full, StepSize st, bool calc_dt, Prof *pf,
     prof_mark(pf, PROF_INVERT, s);
     // ghost fill of the written state; a block of a decomposed domain leaves
     // it to the caller (hamr_bound_dim around the halo exchange)
-    if (!d.halo) launch_bound_dim(ctx, full, 0, fin);
+    if (!d.halo) {
+        const int rc = launch_bound_dim(ctx, full, 0, fin);
+        if (rc) return rc;
+    }
     prof_mark(pf, PROF_BOUND, s);
     CK(cudaGetLastError());
     return HAMR_OK;
