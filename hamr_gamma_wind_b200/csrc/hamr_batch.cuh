@@ -1026,7 +1026,7 @@ int hamr_batch_autotune(hamr_batch *b, const double *dt, int reps) {
             };
             const float ms = both();
             if (ms < 0) rc = bfail(b, cudaGetLastError(), "autotune");
-            b->fused = ms < b->tuned_ms[PH_CONS] + b->tuned_ms[PH_INV];
+            b->fused = rc == HAMR_OK && ms < b->tuned_ms[PH_CONS] + b->tuned_ms[PH_INV];
             if (b->fused) {
                 b->tuned_ms[PH_CONS] = ms;   // the inversion phase launches nothing
                 b->tuned_ms[PH_INV] = 0.f;
