@@ -65,32 +65,47 @@ def test_batch_step_matches_single_blocks_bitwise(precision):
     _close(solo + mem)
 
 
-@pytest.mark.parametrize("precision", ["fp64", "mixed"])
-def test_batch_bulk_copy_update_matches_single_blocks_bitwise(precision, monkeypatch):
-    """Members 3-D with 32 or more zones along x3: the batch's conserved update
-    runs the single-block row kernel with its fluxes staged by bulk copies,
-    one CTA per row of each member (forced for FP64, where the tiled update
-    is the default), and its x3 fluxes the single-block slot kernel with the
-    centre EMFs; the members must match the members stepped alone bit for
-    bit, before and after the autotuner has timed the update's forms."""
-    monkeypatch.setenv("HAMR_BATCH_CONS_TMA", "1")
-    pbs, _ = problems.torus_ensemble(3, 32, 40, seed=11)
+# the forms of the batch's update on members with 32 or more zones along x3:
+# bulk copies with the primary inversion inside (the default), bulk copies
+# followed by the inversion phase (what floors and reset take), tiles
+UPDATE_FORMS = {"fused": {}, "bulk": {"HAMR_BATCH_FUSE_INV": "0"}, "tiled": {"HAMR_BATCH_CONS_TMA": "0"}}
+
+
+def _long_rows(form, monkeypatch, planted=False, **kw):
+    """Two sets of three such members, one to step alone and one batched."""
+    for name, value in UPDATE_FORMS[form].items():
+        monkeypatch.setenv(name, value)
+    extra = dict(rho_atm=1e-8, u_atm=1e-10) if planted else {}
+    pbs, _ = problems.torus_ensemble(3, 32, 40, seed=11, **extra)
     assert all(pb.n3 >= 32 for pb in pbs)
+    for k, pb in enumerate(pbs):
+        if planted:
+            assert plant(pb, seed=200 + k)[0] > 0
 
     def blocks():
         out = []
         for pb in pbs:
-            b = Block(**pb.block_kwargs(), precision=precision, strict=True)
+            b = Block(**pb.block_kwargs(), strict=True, **kw)
             b.set_geometry(pb.geo)
             b.upload(pb.p, pb.ps)
             b.bound()
             out.append(b)
         return out
 
-    solo, mem = blocks(), blocks()
+    return pbs, blocks(), blocks()
+
+
+@pytest.mark.parametrize("inversion", ["2d", "nm"])
+@pytest.mark.parametrize("form", list(UPDATE_FORMS))
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_batch_update_forms_match_single_blocks_bitwise(precision, form, inversion, monkeypatch):
+    """Each form of the update (and the x3 slot kernel with the centre EMFs)
+    against the members stepped alone, bit for bit, before and after the
+    autotuner has timed the forms that the environment allows."""
+    pbs, solo, mem = _long_rows(form, monkeypatch, precision=precision, inversion=inversion)
     batch = Batch(mem)
     tun = batch.tuning()
-    assert tun["update"]["tile"] == 0   # the row kernel is in use
+    assert (tun["update"]["tile"] == 0) == (form != "tiled")   # the row kernel is in use
     assert tun["flux3"]["tile"] == 0    # and the x3 slot kernel (with the centre EMFs)
     dts = np.array([0.2 * min(pb.dx[:2]) for pb in pbs])
     for s in range(4):
@@ -106,30 +121,16 @@ def test_batch_bulk_copy_update_matches_single_blocks_bitwise(precision, monkeyp
     _close(solo + mem)
 
 
+@pytest.mark.parametrize("floors,repair", [(False, "none"), (True, "none"), (False, "reset"), (True, "reset")])
+@pytest.mark.parametrize("form", list(UPDATE_FORMS))
 @pytest.mark.parametrize("precision", ["fp64", "mixed"])
-def test_batch_bulk_copy_update_with_failed_zones_bitwise(precision, monkeypatch):
-    """The same members with planted failed and near-vacuum zones and no
-    floors: the batch's bulk-copy update and one-pass inversion phase against
-    the members stepped alone (whose update runs the primary inversion
-    inside and leaves the failed zones to the fallback pass over a list);
-    one step, flags and failure counters included."""
-    monkeypatch.setenv("HAMR_BATCH_CONS_TMA", "1")
-    pbs, _ = problems.torus_ensemble(3, 32, 40, seed=11, rho_atm=1e-8, u_atm=1e-10)
-    for k, pb in enumerate(pbs):
-        nfail, _ = plant(pb, seed=200 + k)
-        assert nfail > 0
-
-    def blocks():
-        out = []
-        for pb in pbs:
-            b = Block(**pb.block_kwargs(), precision=precision, strict=True)
-            b.set_geometry(pb.geo)
-            b.upload(pb.p, pb.ps)
-            b.bound()
-            out.append(b)
-        return out
-
-    solo, mem = blocks(), blocks()
+def test_batch_update_forms_with_failed_zones_bitwise(precision, form, floors, repair, monkeypatch):
+    """The same with planted failed and near-vacuum zones: the fallback pass
+    over each member's list (fused form) and the inversion phase with its
+    floors and reset (the form of batches with either, whatever the
+    environment) against the members stepped alone; one step, flags and
+    failure counters included."""
+    pbs, solo, mem = _long_rows(form, monkeypatch, planted=True, precision=precision, floors=floors, repair=repair)
     batch = Batch(mem)
     dts = np.array([0.2 * min(pb.dx[:2]) for pb in pbs])
     dn_solo = np.array([b.step(dt) for b, dt in zip(solo, dts)])
@@ -137,7 +138,7 @@ def test_batch_bulk_copy_update_with_failed_zones_bitwise(precision, monkeypatch
     for a, b in zip(solo, mem):
         for x, y in zip((*a.download(), *a.download_flags()), (*b.download(), *b.download_flags())):
             assert np.array_equal(x, y, equal_nan=True)
-        assert a.download_flags()[1].any()   # the fallback pass had zones to count
+        assert a.download_flags()[1].any()   # there were failed zones to count
     batch.close()
     _close(solo + mem)
 
