@@ -703,8 +703,11 @@ int batch_setup_cons_tma(hamr_batch *b) {
         sm = std::max(sm, cons_tma_layout<T>(lpiece).total);
     }
     if (rs[b->n] > 0x7fffffffL) return HAMR_OK;   // more CTAs than one launch's grid holds
+    // the same for every batch, so that one of short rows does not undercut
+    // another's launches
+    const int all = cons_tma_layout<T>(256).total;
     for (auto k : {k_batch_cons_tma<T, 0>, k_batch_cons_tma<T, HAMR_INV_2D + 1>, k_batch_cons_tma<T, HAMR_INV_NM + 1>})
-        BCK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
+        BCK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, all));
     BCK(cudaMemcpyAsync(b->rstart, rs.data(), sizeof(long) * (b->n + 1), cudaMemcpyHostToDevice, b->stream));
     BCK(cudaStreamSynchronize(b->stream));   // rs goes out of scope
     b->ncons_ctas = rs[b->n];

@@ -143,6 +143,35 @@ def test_batch_update_forms_with_failed_zones_bitwise(precision, form, floors, r
     _close(solo + mem)
 
 
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_two_batches_of_different_row_lengths(precision):
+    """A batch created after another with longer rows leaves that one's
+    launches, whose staging takes more shared memory, as they were."""
+    def batch(n3):
+        pb = problems.fm_torus(12, 8, n3, rout=40.0)
+        out = []
+        for _ in range(2):
+            b = Block(**pb.block_kwargs(), precision=precision, strict=True)
+            b.set_geometry(pb.geo)
+            b.upload(pb.p, pb.ps)
+            b.bound()
+            out.append(b)
+        return pb, out
+
+    pb, (solo, mem) = batch(256)
+    long_rows = Batch([mem])
+    short_pb, short_blocks = batch(32)
+    short_rows = Batch(short_blocks)
+    dt = 0.2 * min(pb.dx[:2])
+    assert solo.step(dt) == long_rows.step(np.array([dt]))[0]
+    short_rows.step(np.full(2, dt))
+    for x, y in zip(solo.download(), mem.download()):
+        np.testing.assert_array_equal(x, y)
+    long_rows.close()
+    short_rows.close()
+    _close([solo, mem, *short_blocks])
+
+
 def test_batch_production_build_close_to_single_blocks():
     pbs, solo = _members(strict=False)
     _, mem = _members(strict=False)
