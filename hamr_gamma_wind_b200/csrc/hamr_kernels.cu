@@ -1510,7 +1510,9 @@ __device__ __forceinline__ void cons_update_fx(const Dims &d, const Geom &m, con
     if (!full) {
 #pragma unroll
         for (int k = 0; k < NPR; k++) { pf[k] = 0.0; pf[k] += (1.0 / ((double)1)) * pin[k * ks + c]; }
-        get_state<true>(pf, gm, q);
+        // exact quotients by the lapse; not with the face-frame solvers, which
+        // return another last bit as up to 1e-7 of a velocity also in FP64
+        get_state(pf, gm, q, d.riemann == HAMR_RIEMANN_HLL);
         double vd;
         primtoflux(d.gam, pf, q, 0, gm, entropy(d.gam, pf), U, &vd, &vd);
 #pragma unroll

@@ -278,8 +278,7 @@ __device__ __forceinline__ void gamma_calc(const T *pr, const Geo<G> &gm, T *gam
 
 // u_mu, dot product, u^mu and b^mu of the HLL sides and the centre EMFs in both
 // precisions: fused sums, u~^i u~_i nested, one reciprocal and no division
-// (beta^j / alpha = alpha g^tj). The float face-frame solvers, whose star states
-// amplify a changed last bit a thousandfold, keep the forms below.
+// (beta^j / alpha = alpha g^tj). Where plain_forms holds, the forms below.
 template <typename T>
 __device__ __forceinline__ void lower_hll(const T *u, const T *g, T *o) {
     o[0] = mad(g[3], u[3], mad(g[2], u[2], mad(g[1], u[1], mul(g[0], u[0]))));
@@ -313,17 +312,20 @@ __device__ __forceinline__ void bcon_hll(const T *pr, const T *ucon, const T *uc
     for (int j = 1; j < 4; j++) bcon[j] = mul(mad(bcon[0], ucon[j], pr[B1 - 1 + j]), ru);
 }
 
-// u^mu of a state. The production build's double form is ucon_hll, save for the
-// conserved variables that the update starts from (CONS), whose quotients by
-// alpha are exact in both builds: the inversion multiplies u^t by alpha again,
+// u^mu of a state. The production build's double form is ucon_hll, but for exact
+// quotients by alpha where the caller asks for them: the conserved variables
+// that the update starts from, since the inversion multiplies u^t by alpha again
 // and a product with the rounded 1/alpha would scale a column's mass by the same
 // last bit every step (tests/test_gpu_column_mass.py).
-template <bool CONS = false, typename T, typename G>
-__device__ __forceinline__ void ucon_calc(const T *pr, const Geo<G> &gm, T *ucon) {
+template <typename T, typename G>
+__device__ __forceinline__ void ucon_calc(const T *pr, const Geo<G> &gm, T *ucon, bool exact = false) {
     const G alpha = gm.lapse;   // 1/sqrt(-g^tt), from the Geo (tabulated or geo_lapse)
-    if constexpr (std::is_same<T, double>::value && std::is_same<T, G>::value && !STRICT && !CONS) {
-        ucon_hll(pr, gm, ucon);
-    } else {
+    bool shorter = false;
+    if constexpr (std::is_same<T, double>::value && std::is_same<T, G>::value && !STRICT) {
+        shorter = !exact;
+        if (shorter) ucon_hll(pr, gm, ucon);
+    }
+    if (!shorter) {
         G beta[4];
         T gamma;
         gamma_calc(pr, gm, &gamma);
@@ -350,9 +352,9 @@ __device__ __forceinline__ void bcon_calc(const T *pr, const T *ucon, const T *u
     for (int j = 1; j < 4; j++) bcon[j] = du.div(pr[B1 - 1 + j] + bcon[0] * ucon[j]);
 }
 
-template <bool CONS = false, typename T, typename G>
-__device__ __forceinline__ void get_state(const T *pr, const Geo<G> &gm, State<T> &q) {
-    ucon_calc<CONS>(pr, gm, q.ucon);
+template <typename T, typename G>
+__device__ __forceinline__ void get_state(const T *pr, const Geo<G> &gm, State<T> &q, bool exact = false) {
+    ucon_calc(pr, gm, q.ucon, exact);
     lower4(q.ucon, gm.gcov, q.ucov);
     bcon_calc(pr, q.ucon, q.ucov, q.bcon);
     lower4(q.bcon, gm.gcov, q.bcov);
