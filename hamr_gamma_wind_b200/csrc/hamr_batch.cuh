@@ -160,10 +160,11 @@ struct OpInvert {
 // primary inversion inside it, the zones it fails to their block's list
 // (emptied by k_batch_begin_lists) for k_batch_fallback.
 // Resident CTAs (of up to 256 threads) per SM, FP64 / float fluxes, of the
-// update alone: on the 64-torus ensemble (rows of 32-96 zones) the float update
-// took 2.37 ms per sub-step at 3 (80 registers), 2.61 at 4 (64), and at 5 (48
-// registers, 0.7 KB of spills) lost to the tiled update, before the magnetic
-// components left it. With the inversion: the single block's short rows.
+// update alone: on the 64-torus ensemble (rows of 32-96 zones), with nine
+// components staged per face where six are, the float update took 2.37 ms per
+// sub-step at 3 (80 registers), 2.61 at 4 (64), and at 5 (48 registers, 0.7 KB
+// of spills) lost to the tiled update. With the inversion: the single block's
+// short rows.
 #ifndef HAMR_BATCH_CONS_TMA_MINB
 #define HAMR_BATCH_CONS_TMA_MINB HAMR_CONS_TMA_MINB
 #endif
@@ -469,8 +470,8 @@ struct hamr_batch {
     int graph_steps = -1, graph_interval = -1;
     // one persistent launch per sub-step (hamr_batch_set_persistent)
     // conserved update phase with bulk-copy staging (k_batch_cons_tma): every
-    // block allows it (cons_tma_ok) and it is in use (cons_tma: by default in
-    // the mixed step; the autotuner times it against the tiled update)
+    // block allows it (cons_tma_ok) and it is in use (cons_tma: by default; the
+    // autotuner times it against the tiled update)
     bool cons_tma_ok = false, cons_tma = false;
     // the primary inversion inside it (no floors or reset): allowed, and in use
     bool fused_ok = false, fused = false;
@@ -715,9 +716,8 @@ int batch_setup_cons_tma(hamr_batch *b) {
     b->cons_smem = (size_t)sm;
     b->cons_tma_ok = true;
     // measured on the 64-torus ensemble (rows of 32-96 zones), per sub-step:
-    // float fluxes 1.64 ms, FP64 2.06 against 2.3 for the tiled update (whose
-    // FP64 form was the faster one, 2.59 against 3.20 ms, while the staging held
-    // the magnetic components and fewer CTAs fitted an SM)
+    // float fluxes 1.64 ms, FP64 2.06 against 2.3 for the tiled update (with nine
+    // components staged per face, where fewer CTAs fit an SM, 3.20 against 2.59)
     b->cons_tma = true;
     if (const char *e = getenv("HAMR_BATCH_CONS_TMA")) b->cons_tma = atoi(e) != 0;   // 0: off
     b->fused_ok = b->fused = b->cons_tma && b->fix == 0 && b->n <= 65535;

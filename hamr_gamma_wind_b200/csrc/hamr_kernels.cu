@@ -475,7 +475,8 @@ __device__ __forceinline__ void zone_edges(const Dims &d, const double *__restri
 // slope and each face value is evaluated once per zone, where the five-zone
 // stencil by itself takes three and two, and a thread loads three zones
 // instead of five (per step of the 384 x 192 x 192 torus, centre EMFs included:
-// FP64 5.60 -> 4.17 ms, mixed 2.34 -> 1.99). MC: the edges straight from the slot's slope, in one phase.
+// FP64 5.60 -> 4.17 ms, mixed 2.34 -> 1.99). MC: the edges straight from the
+// slot's slope, in one phase.
 // Last, thread l evaluates the face between slots l and l + 1 (left state: its
 // own upper edge, right state: the lower edge of slot l + 1). Same values as
 // k_flux<3> face by face.
@@ -1955,8 +1956,9 @@ __host__ __device__ __forceinline__ ConsTmaLayout cons_tma_layout(int lpiece) {
 // output pout, and only a zone whose primary solver fails writes W and goes to
 // the list for k_invert_fallback (*nfail cleared before the launch). FIX: 0 or
 // FIX_FLOORS, the floors on each zone it solves (the reset of failed zones keeps
-// the separate kernels; the neighbour repair follows either way). The W round trip and the inversion's reload of the guess
-// disappear; same values as the update followed by k_invert_primary.
+// the separate kernels; the neighbour repair follows either way). The W round
+// trip and the inversion's reload of the guess disappear; same values as the
+// update followed by k_invert_primary.
 //
 // Resident CTAs of 256 threads per SM, which cap the registers (4: 64, 3: 80,
 // 2: 128). Per step, update with inversion, 384 x 192 x 192 torus (CTAs of 192
@@ -1964,8 +1966,8 @@ __host__ __device__ __forceinline__ ConsTmaLayout cons_tma_layout(int lpiece) {
 // Rows of at most 128 zones have CTAs small enough that the register file
 // still holds many at looser caps: 192 x 96 x 64 FP64 2 0.305 ms, 3 0.330, 4
 // 0.367; 131 x 77 x 50 float 2 and 3 0.171, 4 0.184. The update alone (FUSE 0):
-// float 3, FP64 4 (before the magnetic components left it: 2.86 ms against 2.88
-// at 4, and 3.67 against 3.86 at 3).
+// float 3, FP64 4 (with nine components staged per face: 2.86 ms against 2.88 at
+// 4, and 3.67 against 3.86 at 3).
 #ifndef HAMR_CONS_TMA_MINB_F
 #define HAMR_CONS_TMA_MINB_F 3
 #endif
