@@ -69,12 +69,14 @@ def algorithmic_bytes_per_cell_update(n3: int) -> float:
 def kernel_bytes(slot: str, d: dict, width: float = 8.0) -> float:
     """Bytes one launch of a kernel group must move (FP64 storage; with width 4
     the fluxes and EMFs are float, as in the mixed-precision step):
-    flux_d   per face: 9 primitives + 1 normal face field read, 9 fluxes written,
-             plus the face metric (21 words) once per (i, j) column;
-    update   (k_cons) per zone: 9 primitives, 9 cached conserved values and 27
-             face fluxes read or written, 7 conserved values written, plus the
-             centre metric and connection (61 words) per column;
-    invert   per zone: 9 primitives (initial guess) + 7 conserved values + 3 face
+    flux_d   per face: 8 primitives (all but the normal field) + 1 normal face
+             field read, 8 fluxes written (all but the normal field's), plus
+             the face metric (21 words) once per (i, j) column;
+    update   (k_cons_tma; 3-D, where the faces set U[B]) per zone: 9 primitives,
+             6 cached conserved values and 18 face fluxes read or written, 6
+             conserved values written, plus the centre metric, lapse and
+             connection (63 words) per column;
+    invert   per zone: 9 primitives (initial guess) + 6 conserved values + 3 face
              fields read, 9 primitives and 1 int flag written, plus the centre
              metric and face volumes (23 words) per column;
     emf_centre per zone (one ghost layer around): 3 velocities and 3 face
@@ -83,7 +85,7 @@ def kernel_bytes(slot: str, d: dict, width: float = 8.0) -> float:
     face_update per face triple: 3 EMFs read, old and new face fields;
     update_invert (k_cons_tma with the primary inversion inside) per zone:
              the update's reads, 3 face fields read, 9 primitives and 1 int
-             flag written, plus the update's metric; the 7 words of W and the
+             flag written, plus the update's metric; the 6 words of W and the
              inversion's guess never travel (the guess is the state the
              update read)."""
     n1, n2, n3 = d["n1"], d["n2"], d["n3"]
@@ -91,13 +93,13 @@ def kernel_bytes(slot: str, d: dict, width: float = 8.0) -> float:
         k = int(slot[-1])
         nf = (n1 + 2 - (k == 1)) * (n2 + 2 - (k == 2)) * (n3 + 2 - (k == 3))
         ncol = (n1 + 2 - (k == 1)) * (n2 + 2 - (k == 2))
-        return (10 * 8.0 + 9 * width) * nf + 21 * 8.0 * ncol
+        return (9 * 8.0 + 8 * width) * nf + 21 * 8.0 * ncol
     if slot == "update":
-        return (25 * 8.0 + 27 * width) * n1 * n2 * n3 + 61 * 8.0 * n1 * n2
+        return (21 * 8.0 + 18 * width) * n1 * n2 * n3 + 63 * 8.0 * n1 * n2
     if slot == "invert":
-        return (28 * 8.0 + 4) * n1 * n2 * n3 + 23 * 8.0 * n1 * n2
+        return (27 * 8.0 + 4) * n1 * n2 * n3 + 23 * 8.0 * n1 * n2
     if slot == "update_invert":
-        return (30 * 8.0 + 27 * width + 4) * n1 * n2 * n3 + 61 * 8.0 * n1 * n2
+        return (27 * 8.0 + 18 * width + 4) * n1 * n2 * n3 + 63 * 8.0 * n1 * n2
     if slot == "emf_centre":
         return (6 * 8.0 + 3 * width) * (n1 + 2) * (n2 + 2) * (n3 + 2)
     if slot == "emf_edge":
@@ -114,14 +116,14 @@ def kernel_bytes(slot: str, d: dict, width: float = 8.0) -> float:
 # zones (plus a per-column metric term under 1 %), so a launch on another block
 # moves these figures times its zones. flux1 and flux2 share the row kernel;
 # flux3 includes the centre EMFs (computed by the x3 kernel on 3-D blocks);
-# invert adds the fallback pass's 2.9 B; update_invert is the update kernel
+# invert adds the fallback pass's 1.3 B; update_invert is the update kernel
 # with the primary inversion inside (the default on 3-D blocks with
-# n3 >= 32 and no floors or repair).
+# n3 >= 32, but with the reset of failed zones).
 NCU_DRAM_BYTES_PER_ZONE = {
-    "fp64": {"flux1": 219.3, "flux2": 219.3, "flux3": 296.5, "update": 457.1, "invert": 223.6,
-             "update_invert": 509.2, "emf_edge": 123.7, "face_update": 54.7},
-    "mixed": {"flux1": 134.2, "flux2": 134.2, "flux3": 136.7, "update": 315.4, "invert": 223.4,
-              "update_invert": 388.6, "emf_edge": 58.6, "face_update": 40.6},
+    "fp64": {"flux1": 146.8, "flux2": 146.8, "flux3": 162.2, "update": 359.4, "invert": 191.5,
+             "update_invert": 395.9, "emf_edge": 124.2, "face_update": 60.6},
+    "mixed": {"flux1": 132.3, "flux2": 132.3, "flux3": 124.9, "update": 245.9, "invert": 190.3,
+              "update_invert": 321.2, "emf_edge": 57.4, "face_update": 44.2},
 }
 
 # what limits each kernel group, read from the same captures
@@ -130,9 +132,9 @@ KERNEL_LIMITER = {
     "flux2": "latency: PPM stencil loads (long scoreboard) and dependent FP chains",
     "flux3": "latency: dependent FP64/FP32 chains of the four flux evaluations per face (and the centre EMFs)",
     "update": "FP64 fixed-latency chains after TMA-staged operand loads",
-    "invert": "FP64 dependent Newton iterations (FP64 pipe 45 % active)",
+    "invert": "FP64 dependent Newton iterations (FP64 pipe 40 % active)",
     "update_invert": "FP64 fixed-latency chains of the update's sums and the Newton iterations "
-                     "(FP64 pipe 35-45 % active)",
+                     "(FP64 pipe 36-44 % active)",
     "emf_centre": "memory latency (long scoreboard)",
     "emf_edge": "memory latency (long scoreboard)",
     "face_update": "memory latency (long scoreboard)",
@@ -143,28 +145,28 @@ KERNEL_LIMITER = {
 # same captures (profiles/: FP64 pipe or issue slots active, % of peak; for
 # the latency-bound ones the long-scoreboard stalls per issued instruction)
 KERNEL_BOUND = {
-    "fp64": {"flux1": ("fp64", "sm__pipe_fp64_cycles_active %", 49.0),
-             "flux2": ("fp64", "sm__pipe_fp64_cycles_active %", 49.0),
-             "flux3": ("fp64", "sm__pipe_fp64_cycles_active %", 44.9),
-             "update": ("latency", "long-scoreboard stalls / issue", 6.13),
-             "invert": ("fp64", "sm__pipe_fp64_cycles_active %", 54.9),
-             "update_invert": ("fp64", "sm__pipe_fp64_cycles_active %", 34.8),
-             "emf_edge": ("latency", "long-scoreboard stalls / issue", 6.74),
-             "face_update": ("latency", "long-scoreboard stalls / issue", 12.0)},
-    "mixed": {"flux1": ("issue", "sm__issue_active %", 59.0),
-              "flux2": ("issue", "sm__issue_active %", 59.0),
-              "flux3": ("issue", "sm__issue_active %", 68.8),
-              "update": ("latency", "long-scoreboard stalls / issue", 3.25),
-              "invert": ("fp64", "sm__pipe_fp64_cycles_active %", 47.9),
-              "update_invert": ("fp64", "sm__pipe_fp64_cycles_active %", 45.3),
-              "emf_edge": ("issue", "sm__issue_active %", 61.1),
-              "face_update": ("latency", "long-scoreboard stalls / issue", 12.7)},
+    "fp64": {"flux1": ("fp64", "sm__pipe_fp64_cycles_active %", 44.4),
+             "flux2": ("fp64", "sm__pipe_fp64_cycles_active %", 44.5),
+             "flux3": ("fp64", "sm__pipe_fp64_cycles_active %", 45.4),
+             "update": ("latency", "long-scoreboard stalls / issue", 9.01),
+             "invert": ("fp64", "sm__pipe_fp64_cycles_active %", 40.8),
+             "update_invert": ("fp64", "sm__pipe_fp64_cycles_active %", 35.5),
+             "emf_edge": ("latency", "long-scoreboard stalls / issue", 6.79),
+             "face_update": ("latency", "long-scoreboard stalls / issue", 8.15)},
+    "mixed": {"flux1": ("issue", "sm__issue_active %", 47.0),
+              "flux2": ("issue", "sm__issue_active %", 47.0),
+              "flux3": ("issue", "sm__issue_active %", 64.5),
+              "update": ("fp64", "sm__pipe_fp64_cycles_active %", 34.8),
+              "invert": ("fp64", "sm__pipe_fp64_cycles_active %", 39.5),
+              "update_invert": ("fp64", "sm__pipe_fp64_cycles_active %", 43.7),
+              "emf_edge": ("issue", "sm__issue_active %", 61.3),
+              "face_update": ("latency", "long-scoreboard stalls / issue", 8.8)},
 }
 
 
 def inversion_fused(slots: dict, d: dict) -> bool:
     """The 3-D update kernel with bulk-copy staging (n3 >= 32) runs the
-    primary inversion itself unless floors or a repair are on; the invert
+    primary inversion itself unless failed zones are reset; the invert
     slot then times only the fallback pass over failed zones, a few % of the
     update's time rather than about as much."""
     return d["n3"] >= 32 and slots.get("invert", 0.0) < 0.25 * slots.get("update", 0.0)
@@ -202,9 +204,10 @@ def kernel_rooflines(slots: dict, d: dict, prec: str, hbm: float) -> dict:
 
 
 def launches_per_step(pb, fused_inv: bool = True) -> int:
-    """Kernels one RK2 step launches (two sub-steps and the step-size
-    finalisation), following the stage sequence of the library; with the
-    inversion inside the update, its primary pass launches nothing."""
+    """Kernels one RK2 step of a 3-D block with n3 >= 32 launches (two
+    sub-steps; the step-size words ride on the last ghost fill), following the
+    stage sequence of the library; with the inversion inside the update, its
+    primary pass launches nothing."""
     dims = [n > 1 for n in (pb.n1, pb.n2, pb.n3)]
     per_stage = sum(dims)                       # face fluxes
     per_stage += pb.bc[1] == "pole_refl"        # polar flux fix
@@ -212,7 +215,17 @@ def launches_per_step(pb, fused_inv: bool = True) -> int:
     per_stage += pb.bc[1] == "pole_trans"       # polar EMF average
     per_stage += 1 + 1 + (1 if fused_inv else 2)   # face update, conserved update, inversion (fallback pass)
     per_stage += sum(dims)                      # ghost fills
-    return 2 * per_stage + 1
+    return 2 * per_stage
+
+
+def batch_launches_per_step(tuning: dict) -> int:
+    """Kernels one step of a tuned batch launches: in both sub-steps the phases
+    with items (the x3 slot kernel makes the centre EMFs: tile 0 there; the
+    fused update leaves the inversion phase no time and brings the emptying of
+    the failed-zone lists and the fallback pass), then the step sizes."""
+    phases = [k for k, v in tuning.items() if v["ms"] > 0 and not (k == "emf_centre" and v["tile"] == 0)]
+    fused = tuning["update"]["tile"] == 0 and not tuning["invert"]["ms"] > 0
+    return 2 * (len(phases) + (2 if fused else 0)) + 1
 
 
 class ClockSampler:
@@ -723,9 +736,7 @@ def run_ensemble(args):
                       "precision": head, "members": [d["n"] for d in draws], "l2": "inputs larger than L2"},
            "precisions": {k: {kk: vv for kk, vv in v.items() if kk != "tuning"} for k, v in runs.items()},
            "tuning": {k: v["tuning"] for k, v in runs.items()},
-           # per step: the phases that launch (tuned time > 0) in both
-           # sub-steps and the step-size finalisation
-           "gpu_launches": args.steps * (2 * sum(1 for v in runs[head]["tuning"].values() if v["ms"] > 0) + 1)}
+           "gpu_launches": args.steps * batch_launches_per_step(runs[head]["tuning"])}
     print(json.dumps(out), flush=True)
 
 

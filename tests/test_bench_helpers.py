@@ -27,14 +27,17 @@ def test_fused_inversion_is_told_from_the_slot_times():
 def test_update_bytes_with_and_without_the_inversion():
     zones = 384 * 192 * 192
     cols = 384 * 192
-    for width, per_zone in ((4.0, 352), (8.0, 460)):
-        assert bench.kernel_bytes("update_invert", C3, width) == per_zone * zones + 488 * cols
-    # fusing drops the seven W words written and read back and the guess's
-    # reload (23 words per zone), and the inversion's own metric columns
+    for width, per_zone in ((4.0, 292), (8.0, 364)):
+        assert bench.kernel_bytes("update_invert", C3, width) == per_zone * zones + 504 * cols
+    # fusing drops the six W words written and read back and the guess's
+    # reload (21 words per zone), and the inversion's own metric columns
     for width in (4.0, 8.0):
         split = bench.kernel_bytes("update", C3, width) + bench.kernel_bytes("invert", C3, width)
         fused = bench.kernel_bytes("update_invert", C3, width)
-        assert split - fused == 23 * 8 * zones + 23 * 8 * cols
+        assert split - fused == 21 * 8 * zones + 23 * 8 * cols
+    # a face reads eight primitives and its normal field and writes eight fluxes
+    faces, fcols = 386 * 194 * 193, 386 * 194
+    assert bench.kernel_bytes("flux3", C3, 4.0) == 104 * faces + 168 * fcols
 
 
 @pytest.mark.parametrize("prec", ["mixed", "fp64"])
@@ -57,6 +60,17 @@ def test_roofline_rows(prec):
 def test_launches_per_step_of_the_torus():
     pb = problems.fm_torus(24, 16, 40, rout=40.0)   # 3-D, transmissive poles
     # per sub-step: 3 flux directions, edge EMFs, polar EMF average, face
-    # update, conserved update, inversion (1 or 2 passes), 3 ghost fills
-    assert bench.launches_per_step(pb, True) == 2 * 11 + 1
-    assert bench.launches_per_step(pb, False) == 2 * 12 + 1
+    # update, conserved update, inversion (1 or 2 passes), 3 ghost fills (the
+    # last with the step-size words)
+    assert bench.launches_per_step(pb, True) == 2 * 11
+    assert bench.launches_per_step(pb, False) == 2 * 12
+
+
+def test_launches_per_step_of_a_batch():
+    ph = dict.fromkeys(["flux3", "flux2", "flux1", "emf_edge", "pole_average", "face_update", "update", "invert",
+                        "bound_x1", "bound_x3", "bound_x2"], {"tile": 128, "ms": 1.0})
+    ph["emf_centre"] = {"tile": 0, "ms": 0.004}   # by the x3 slots
+    ph["fix_flux"] = {"tile": 128, "ms": 0.0}
+    assert bench.batch_launches_per_step(ph) == 2 * 11 + 1
+    fused = dict(ph, update={"tile": 0, "ms": 1.5}, invert={"tile": 128, "ms": 0.0})
+    assert bench.batch_launches_per_step(fused) == 2 * 12 + 1
